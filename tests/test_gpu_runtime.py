@@ -280,3 +280,29 @@ def test_executable_writes_the_reference_format(built, dim):
     rt = 1e-9 if dim == 3 else 1e-5
     np.testing.assert_allclose(vals[:p.Ne, 0], one.ER, rtol=rt, atol=1e-300)
     np.testing.assert_allclose(vals[p.Ne:, 0], one.EBR, rtol=rt, atol=1e-300)
+
+
+@pytest.mark.parametrize("name,cap", [("phantom3d", 1), ("phantom3d", 60), ("phantom3d_fd", 60), ("mixed3d", 9),
+                                      ("square2d", 1), ("square2d", 13)])
+def test_step_limit_of_the_tracking_form(built, name, cap):
+    """Photons at the step limit are lost with the weight they have then: no walk is longer, the
+    ledger closes, and a limit that no walk reaches changes nothing.  One-job and per-job forms."""
+    p = cases()[name][0].copy(Nphoton=4000)
+    free = V.run(p, normalize=False)
+    out = V.run(p, normalize=False, max_steps=cap)
+    assert free.stats["capped"] == 0 and 0 < out.stats["capped"] <= p.Nphoton
+    assert out.stats["steps"] <= cap * p.Nphoton
+    assert out.stats["steps"] >= cap * out.stats["capped"]
+    if p.f == 0.0:
+        lg = out.stats["ledger"]
+        total = lg["absorbed"] + lg["exited"] + lg["roulette_kill"] - lg["roulette_gain"] + lg["lost"]
+        assert abs(total / p.Nphoton - 1.0) < 1e-6  # FP32 weights: w - dep and dep round alike
+    mesh = V.Mesh(p)
+    both, st = V.run_batch([mesh, mesh], [p, p.copy(Nphoton=0)], max_steps=cap, normalize=False)
+    assert st["capped"] == out.stats["capped"] and st["steps"] == out.stats["steps"]
+    if p.f == 0.0:  # the one-job and per-job forms round a modulated source's phase differently
+        for k in ("ER", "EBR"):
+            np.testing.assert_allclose(getattr(both[0], k), getattr(out, k), rtol=1e-9, atol=1e-9)
+    wide, _ = V.run_batch([mesh], [p], max_steps=free.stats["steps"], normalize=False)
+    np.testing.assert_allclose(wide[0].ER, free.ER, rtol=1e-9, atol=1e-9)
+    mesh.close()

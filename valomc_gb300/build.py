@@ -21,6 +21,11 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 CU_UNITS = ["kern3d32.cu", "kern3d64.cu", "kern2d32.cu", "kern2d64.cu", "runtime.cu", "tools.cu", "server.cu",
             "noalloc.cu"]
+# The tetrahedral tracking kernel flushes FP32 subnormals: its reciprocals, roots, logarithms and
+# exponentials then need no scaling around them (5 % fewer instructions a step; 202.2 -> 197.2 ms
+# for 1e7 photons on the 648k-tet phantom).  A walk meets none: lengths are clamped at 0 and the
+# conversion to the FP64 accumulators has always dropped subnormal deposits.
+FLAGS = {"kern3d32.cu": ["-ftz=true"]}
 CPP_UNITS = ["host_setup.cpp"]
 APPS = {"MC3D": "app/mc3d_main.cpp", "MC2D": "app/mc2d_main.cpp", "vmc_textdump": "app/textdump.cpp"}
 
@@ -59,7 +64,7 @@ def build(force=False, verbose=False, jobs=None):
     objs = []
     for u in CU_UNITS:
         o = os.path.join(BUILD, u.replace(".cu", ".o"))
-        cmds.append([nv] + cuflags + ["-c", os.path.join(CSRC, u), "-o", o])
+        cmds.append([nv] + cuflags + FLAGS.get(u, []) + ["-c", os.path.join(CSRC, u), "-o", o])
         objs.append(o)
     for u in CPP_UNITS:
         o = os.path.join(BUILD, u.replace(".cpp", ".o"))

@@ -81,14 +81,20 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
     __syncthreads();
   }
   bool alive = false, done = false;
-  uint32_t n_steps = 0, n_scat = 0, n_done = 0;
+  unsigned long long n_steps = 0;
+  uint32_t n_scat = 0, n_done = 0;
   long long chunk_next = 0, chunk_end = 0;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
   const long long total = lp.total;
+  const int32_t cap = (int32_t)min(lp.max_steps, (int64_t)INT32_MAX);
   for (unsigned it = 0;; ++it) {
     if ((it & 1023u) == 0u) {  // the host's cancel flag (an L2 round trip), every 1024 steps
-      if (*reinterpret_cast<volatile const int32_t *>(&lp.ctl->cancel)) { done = true; alive = false; }
+      if (*reinterpret_cast<volatile const int32_t *>(&lp.ctl->cancel)) {
+        if (alive) n_steps += (unsigned long long)s.nsteps;  // an unfinished walk's steps count in the launch's total
+        done = true;
+        alive = false;
+      }
     }
     // refill and the exit test only when some lane is idle (one vote in the common case)
     if (__any_sync(kFull, !alive)) {
@@ -126,13 +132,16 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
     if (__all_sync(kFull, done)) break;
     }
     if (alive) {
-      const int r = s.step(*J, rng, lp.max_steps);
-      if (r == kScattered) { n_steps++; n_scat++; }
-      else if (r == kAlive) { n_steps++; }
-      else {
-        if (r == kDied) n_steps++;
-        alive = false;
+      if constexpr (W::kCap32) {
+        alive = s.step(*J, rng, cap, n_scat);
+      } else {
+        const int r = s.step(*J, rng, lp.max_steps);
+        n_scat += r == kScattered;
+        alive = r <= kAliveMax;
+      }
+      if (!alive) {
         n_done++;
+        n_steps += (unsigned long long)s.nsteps;
         job_count_add(*J, kJcSteps, (unsigned long long)s.nsteps);
       }
     }

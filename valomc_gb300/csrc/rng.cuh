@@ -83,6 +83,22 @@ struct PhiloxT {
   // together, instead of each lane computing blocks at a different draw.  Words left in
   // the previous block are dropped.
   __device__ __forceinline__ void align() { n = 0; }
+  // The first three words of the block that a scatter event draws from; take(k) draws k of them.
+  __device__ __forceinline__ uint3 peek3() {
+    PhiloxT t = *this;
+    t.block();
+    return make_uint3(t.buf.x, t.buf.y, t.buf.z);
+  }
+  __device__ __forceinline__ void take(int k) { c2++; n = 4 - k; }
+  // Before a draw outside the scatter events (interfaces, roulette): the words left in the
+  // current block again, so that no step carries them in registers.
+  __device__ __forceinline__ void reload() {
+    const int32_t left = n;
+    if (left == 0) return;
+    c2--;
+    block();
+    for (n = 4; n > left; n--) { buf.x = buf.y; buf.y = buf.z; buf.z = buf.w; }
+  }
 };
 using PhiloxRng = PhiloxT<false>;  // per-photon key (batched launches)
 using PhiloxOne = PhiloxT<true>;   // launch-wide key (one job)
@@ -100,6 +116,14 @@ struct TapeRng {
   }
   __device__ __forceinline__ bool exhausted() const { return out; }
   __device__ __forceinline__ void align() {}  // a tape is consumed word by word
+  __device__ __forceinline__ uint3 peek3() const {
+    return make_uint3(p < end ? p[0] : 0x80000000u, end - p > 1 ? p[1] : 0x80000000u, end - p > 2 ? p[2] : 0x80000000u);
+  }
+  __device__ __forceinline__ void take(int k) {
+    out |= end - p < k;
+    p = out ? end : p + k;
+  }
+  __device__ __forceinline__ void reload() {}
 };
 
 // reference mappings (double)
@@ -108,8 +132,11 @@ template <class R> __device__ __forceinline__ double unif_open(R &r) { return ((
 template <class R> __device__ __forceinline__ double unif_halfup(R &r) { return (double)r.next() * (1.0 / 4294967296.0); }
 
 // float mappings
-template <class R> __device__ __forceinline__ float unif_closed_f(R &r) { return (float)(r.next() >> 8) * (1.0f / 16777215.0f); }
-template <class R> __device__ __forceinline__ float unif_open_f(R &r) { return ((float)(r.next() >> 9) + 0.5f) * (1.0f / 8388608.0f); }
-template <class R> __device__ __forceinline__ float unif_halfup_f(R &r) { return (float)(r.next() >> 8) * (1.0f / 16777216.0f); }
+__device__ __forceinline__ float closed_f(uint32_t w) { return (float)(w >> 8) * (1.0f / 16777215.0f); }
+__device__ __forceinline__ float open_f(uint32_t w) { return ((float)(w >> 9) + 0.5f) * (1.0f / 8388608.0f); }
+__device__ __forceinline__ float halfup_f(uint32_t w) { return (float)(w >> 8) * (1.0f / 16777216.0f); }
+template <class R> __device__ __forceinline__ float unif_closed_f(R &r) { return closed_f(r.next()); }
+template <class R> __device__ __forceinline__ float unif_open_f(R &r) { return open_f(r.next()); }
+template <class R> __device__ __forceinline__ float unif_halfup_f(R &r) { return halfup_f(r.next()); }
 
 }  // namespace vmc

@@ -28,6 +28,7 @@ __device__ __forceinline__ bool ray_seg(const double R[2], const double D[2], co
 
 template <bool FD, class R>
 struct Walk2D64 {
+  static constexpr bool kCap32 = false;
   static constexpr int kMinBlocks = 1;
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
@@ -275,6 +276,7 @@ struct Walk2D64 {
 
 template <bool FD, class R>
 struct Walk2D32 {
+  static constexpr bool kCap32 = false;
   static constexpr int kMinBlocks = 4;
   static constexpr bool kStaged = false;
   Stage stage;
@@ -364,7 +366,7 @@ struct Walk2D32 {
   }
 
   __device__ __forceinline__ bool fresnel(R &rng, float nx, float ny, float eta, bool boundary) {
-    float dn = dx * nx + dy * ny;
+    float dn = fmaf(dy, ny, __fmul_rn(dx, nx));
     float ci = fabsf(dn);
     float ct = 0.0f;
     if (fresnel_reflects_f(rng, eta, ci, ct)) {
@@ -373,7 +375,7 @@ struct Walk2D32 {
     }
     if (boundary) return false;
     float m = copysignf(ct, dn) - eta * dn;
-    dx = eta * dx + m * nx; dy = eta * dy + m * ny;
+    dx = fmaf(eta, dx, __fmul_rn(m, nx)); dy = fmaf(eta, dy, __fmul_rn(m, ny));
     return false;
   }
 
@@ -456,9 +458,10 @@ struct Walk2D32 {
       const float s1 = a * sin_small(th);
       float sp, cp;
       __sincosf(phase, &sp, &cp);
-      acc += w * (cp * c1 + sp * s1);
-      accI += w * (cp * s1 - sp * c1);
-      phase = wrap_phase(phase + th);
+      // these roundings, whatever the shape of the code around them (as in the 3D walk)
+      acc = fmaf(w, fmaf(sp, s1, __fmul_rn(cp, c1)), acc);
+      accI = fmaf(w, fmaf(cp, s1, -__fmul_rn(sp, c1)), accI);
+      phase = wrap_phase(__fadd_rn(phase, th));
       w *= a;
     }
     prop -= ds;

@@ -19,7 +19,7 @@
 
 namespace vmc {
 
-enum StepResult { kAlive = 0, kDied = 1, kScattered = 2, kDiedEarly = 3 };
+enum StepResult { kAlive = 0, kScattered = 1, kAliveMax = kScattered, kDied = 2, kDiedEarly = 3 };
 
 // Moller-Trumbore (RayTriangleIntersects, cpp/3d/MC3D.hpp:1825-1869)
 __device__ __forceinline__ bool ray_tri(const double O[3], const double D[3], const double *V0, const double *V1,
@@ -65,16 +65,17 @@ __device__ __forceinline__ bool fresnel_reflects_d(R &rng, double nipnt, double 
 // rp = (ci - eta ct)/(ci + eta ct), R = (rs^2 + rp^2)/2 (same R as the reference's angle form).
 template <class R>
 __device__ __forceinline__ bool fresnel_reflects_f(R &rng, float eta, float ci, float &ct) {
-  float s = 1.0f - eta * eta * (1.0f - ci * ci);
+  // fused multiply-adds written out: one rounding whatever kernel this is inlined into
+  float s = fmaf(-__fmul_rn(eta, eta), fmaf(-ci, ci, 1.0f), 1.0f);
   if (s <= 0.0f) return true;
   ct = sqrtf(s);
   // a launch direction that is not unit length (3D BCLNormal of direction type 'a'/'r' is
   // not normalised, MC3D.hpp:679-683) can give |cos| > 1: acos is then NaN in the
   // reference, R is NaN and the photon is transmitted
   if (!(ci <= 1.0f)) return false;
-  float rs = (eta * ci - ct) / (eta * ci + ct);
-  float rp = (ci - eta * ct) / (ci + eta * ct);
-  float Rf = 0.5f * (rs * rs + rp * rp);
+  float rs = fmaf(eta, ci, -ct) / fmaf(eta, ci, ct);
+  float rp = fmaf(-eta, ct, ci) / fmaf(eta, ct, ci);
+  float Rf = 0.5f * fmaf(rs, rs, __fmul_rn(rp, rp));
   return unif_closed_f(rng) <= Rf;
 }
 
@@ -118,6 +119,7 @@ __device__ __forceinline__ float free_path_f(float u, float mus) {
 // =====================================================================================
 template <bool FD, class R>
 struct Walk3D64 {
+  static constexpr bool kCap32 = false;
   static constexpr int kMinBlocks = 1;  // ~125 registers: 2 CTAs of 256 per SM
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
@@ -387,6 +389,7 @@ struct Walk3D32 {
   // per SM beat 24 (+7% on the 648k-tet phantom); 5 CTAs (48 registers) spill and lose
   static constexpr int kMinBlocks = 4;
   static constexpr bool kStaged = !FD;
+  static constexpr bool kCap32 = true;
   using Tr = typename TraceFor<R>::type;
   float px, py, pz, dx, dy, dz;
   float w, prop, phase;
@@ -456,11 +459,11 @@ struct Walk3D32 {
     acc = accI = 0.0f;
   }
 
-  __device__ __forceinline__ int die(const JobDev &J, int64_t ev) {
+  __device__ __forceinline__ bool die(const JobDev &J, int64_t ev) {
     flush(J);
     tr.put(ev);
     tr.end();
-    return kDied;
+    return false;
   }
 
   // Philox streams: a photon launched out through its own entry face is lost before its
@@ -473,31 +476,34 @@ struct Walk3D32 {
     return true;
   }
 
-  __device__ __forceinline__ void scatter(R &rng) {
-    // Henyey-Greenstein: cos(theta) from the inverse CDF, phi uniform; same rotation as
-    // ScatterPhoton (MC3D.hpp:1316-1332)
-    float xi = unif_closed_f(rng);
-    float ct;
-    if (g != 0.0f) {
-      if (xi > 0.0f && xi < 1.0f) {
-        // (1 + g^2 - q^2) / (2 g) with q = (1 - g^2) / D, D = 1 - g + 2 g xi, over one
-        // division: ((1 + g^2) D^2 - (1 - g^2)^2) / (2 g D^2)
-        const float D = 1.0f - g + 2.0f * g * xi;
-        const float a = 1.0f - g * g;
-        const float D2 = D * D;
-        ct = __fdividef((1.0f + g * g) * D2 - a * a, 2.0f * g * D2);
-      } else {
-        ct = xi > 0.5f ? 1.0f : -1.0f;  // theta = (1 - xi) pi at xi in {0, 1}
-      }
-    } else {
-      ct = 2.0f * xi - 1.0f;
-    }
-    ct = fminf(1.0f, fmaxf(-1.0f, ct));
-    const float s2 = fmaxf(0.0f, 1.0f - ct * ct);
-    const float st = s2 > 0.0f ? s2 * rsqrtf(s2) : 0.0f;
-    float sp, cp;
+  // What a scatter event draws: the polar cosine and sine, the azimuth's, the free path after it.
+  struct Event { float ct, st, cp, sp, path; };
+
+  // Henyey-Greenstein: cos(theta) from the inverse CDF, phi uniform (MC3D.hpp:1297-1315), and
+  // the free path after the event, from the words u.  Selects, no branches.
+  __device__ __forceinline__ Event draw_event(uint3 u) const {
+    Event e;
+    const float xi = closed_f(u.x);
+    // (1 + g^2 - q^2) / (2 g) with q = (1 - g^2) / D, D = 1 - g + 2 g xi, over one
+    // division: ((1 + g^2) D^2 - (1 - g^2)^2) / (2 g D^2)
+    const float D = 1.0f - g + 2.0f * g * xi;
+    const float a = 1.0f - g * g;
+    const float D2 = D * D;
+    float ct = __fdividef((1.0f + g * g) * D2 - a * a, 2.0f * g * D2);
+    ct = xi > 0.0f && xi < 1.0f ? ct : xi > 0.5f ? 1.0f : -1.0f;  // theta = (1 - xi) pi at xi in {0, 1}
+    ct = g != 0.0f ? ct : 2.0f * xi - 1.0f;
+    e.ct = fminf(1.0f, fmaxf(-1.0f, ct));
+    const float s2 = fmaxf(0.0f, 1.0f - e.ct * e.ct);
+    e.st = s2 > 0.0f ? s2 * rsqrtf(s2) : 0.0f;
     // phi uniform on [-pi, pi] (the reference's [0, 2 pi] shifted; same distribution)
-    __sincosf((float)kPi * (2.0f * unif_closed_f(rng) - 1.0f), &sp, &cp);
+    __sincosf((float)kPi * (2.0f * closed_f(u.y) - 1.0f), &e.sp, &e.cp);
+    e.path = free_path_f(open_f(u.z), mus);
+    return e;
+  }
+
+  // the rotation of ScatterPhoton (MC3D.hpp:1316-1332)
+  __device__ __forceinline__ void rotate(const Event &e) {
+    const float ct = e.ct, st = e.st, cp = e.cp, sp = e.sp;
     float nx, ny, nz;
     {
       // the general rotation and the near-pole case (|dz| > 0.999) as selects, no branch
@@ -518,7 +524,7 @@ struct Walk3D32 {
 
   // true if reflected; N is the outward unit normal of the face being crossed
   __device__ __forceinline__ bool fresnel(R &rng, float nx, float ny, float nz, float eta) {
-    float dn = dx * nx + dy * ny + dz * nz;  // > 0: leaving through the face
+    float dn = fmaf(dz, nz, fmaf(dx, nx, __fmul_rn(dy, ny)));  // > 0: leaving through the face
     float ci = fabsf(dn);
     float ct = 0.0f;
     if (fresnel_reflects_f(rng, eta, ci, ct)) {
@@ -527,7 +533,7 @@ struct Walk3D32 {
     }
     // refraction: d' = eta d + (ct - eta ci) s N with s the side the photon moves to
     float m = copysignf(ct, dn) - eta * dn;
-    dx = eta * dx + m * nx; dy = eta * dy + m * ny; dz = eta * dz + m * nz;
+    dx = fmaf(eta, dx, __fmul_rn(m, nx)); dy = fmaf(eta, dy, __fmul_rn(m, ny)); dz = fmaf(eta, dz, __fmul_rn(m, nz));
     return false;
   }
 
@@ -544,17 +550,26 @@ struct Walk3D32 {
     return false;
   }
 
-  __device__ int step(const JobDev &J, R &rng, int64_t max_steps) {
-    if (rng.exhausted()) { job_count(J, kJcTapeEnd); die(J, kEvTapeEnd); return kDiedEarly; }
-    if (nsteps >= (int32_t)min(max_steps, (int64_t)INT32_MAX)) {  // a 32-bit compare (loop invariant bound)
-      job_count(J, kJcCapped); job_ledger(J, kLgLost, f2d_int(w));
-      die(J, kEvCapped);
-      return kDiedEarly;
-    }
-    if (R::kReplay && outward) {  // with Philox streams this is settled at launch
-      job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
-      die(J, kEvLost);
-      return kDiedEarly;
+  // One element step; false when the photon's walk has ended.  The kernel issues an
+  // instruction in 74-78 % of its cycles, so its time follows the instructions of a warp's
+  // step: control flow was a fifth of them.  Two branches are left on the common path, the
+  // scatter and the crossing into a scattering element of the same index above the roulette
+  // threshold; what either needs is drawn or tested at once, with selects, and everything
+  // else branches off behind them (rare()).  Both branches run in nearly every step of a warp,
+  // yet one straight run of instructions for both, with selects throughout, issues 12 % more
+  // and measured slower (1e7 photons on the 648k-tet phantom: 228 ms).  Measured against the
+  // form with a branch per case, both with flushed subnormals: 197.2 -> 194.4 ms there, 34.3 ->
+  // 32.1 ms at 1e6 photons, 41.4 -> 40.2 ms for ten cubes in one launch; 202.2, 35.9 and
+  // 42.7 ms before.
+  // The products named __fmul_rn stay out of the fused multiply-adds that the compiler would
+  // otherwise choose by the shape of the code around them: one photon, one rounding.
+  __device__ __forceinline__ bool step(const JobDev &J, R &rng, int32_t cap, uint32_t &n_scat) {
+    if constexpr (R::kReplay) {
+      if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
+      if (outward) {  // with Philox streams this is settled at launch
+        job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
+        return die(J, kEvLost);
+      }
     }
     const Tet32 *T = geomp(J) + el;
     const float4 *P4 = reinterpret_cast<const float4 *>(T->pl);
@@ -573,21 +588,18 @@ struct Walk3D32 {
       for (int f = 0; f < 4; f++) {
         const float nd = pl[f].x * dx + pl[f].y * dy + pl[f].z * dz;
         const float num = pl[f].w - (pl[f].x * px + pl[f].y * py + pl[f].z * pz);
-        const bool better = nd > 0.0f && num * bnd < bnum * nd;
+        const bool better = f == 0 ? nd > 0.0f : nd > 0.0f && num * bnd < bnum * nd;
         bnum = better ? num : bnum;
         bnd = better ? nd : bnd;
         nf = better ? f : nf;
       }
     }
     const float best = __fdividef(bnum, bnd);
-    if (nf < 0) {
-      job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
-      die(J, kEvLost);
-      return kDiedEarly;
-    }
-    nsteps++;
+    const bool found = nf >= 0;
+    nsteps += found;
     const float dist = fmaxf(best, 0.0f);
-    const float ds = fminf(prop, dist);
+    // a photon without an exit takes a step of length 0, which changes nothing of it
+    const float ds = found ? fminf(prop, dist) : 0.0f;
     // a photon that leaves the element: fetch the next element's optics now, so that the
     // load runs under the deposit arithmetic
     const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nf == 2 ? nb.z : nb.w;
@@ -597,13 +609,9 @@ struct Walk3D32 {
     tr.put(el);
     const float x = mua * ds;
     if (!FD) {
-      if (mua > 0.0f) {
-        float dep = w * one_minus_exp_neg(x);
-        acc += dep;
-        w -= dep;
-      } else {
-        acc += w * ds;
-      }
+      const float dep = w * one_minus_exp_neg(x);
+      acc = mua > 0.0f ? acc + dep : acc + w * ds;
+      w = mua > 0.0f ? w - dep : w;
     } else {
       // w (cos phi - cos(phi + k ds) a) and w (-sin phi + sin(phi + k ds) a), a = exp(-mua ds),
       // written so that neither difference cancels: 1 - a cos(th) = (1 - a) + 2 a sin^2(th/2)
@@ -615,34 +623,81 @@ struct Walk3D32 {
       const float s1 = a * sin_small(th);
       float sp, cp;
       __sincosf(phase, &sp, &cp);
-      acc += w * (cp * c1 + sp * s1);
-      accI += w * (cp * s1 - sp * c1);
-      phase = wrap_phase(phase + th);
+      acc = fmaf(w, fmaf(sp, s1, __fmul_rn(cp, c1)), acc);
+      accI = fmaf(w, fmaf(cp, s1, -__fmul_rn(sp, c1)), accI);
+      // fused in the one-job form only, as each has rounded it all along
+      phase = wrap_phase(R::kOneJob ? fmaf(J.k_scale_f * nidx, ds, phase) : __fadd_rn(phase, th));
       w *= a;
     }
     prop -= ds;
-    if (prop <= 0.0f) {
-      int res = kAlive;
-      rng.align();
-      if (mus > 0.0f) { scatter(rng); res = kScattered; }
-      prop = free_path_f(unif_open_f(rng), mus);
-      return res;
+    const bool going = found && nsteps < cap;  // neither lost nor at the step limit
+    if (going && prop <= 0.0f && mus > 0.0f) {
+      const Event ev = draw_event(rng.peek3());
+      rotate(ev);
+      rng.take(3);
+      prop = ev.path;
+      n_scat++;
+      return true;
     }
-    // the crossed face's plane, only on the (rare) mirror and Fresnel paths
-    auto face = [&]() { return nf == 0 ? p0 : nf == 1 ? p1 : nf == 2 ? p2 : p3; };
+    // the common crossing: interior, scattering medium, weight above the roulette threshold,
+    // no index jump
+    if (going && prop > 0.0f && (unsigned)nextel < (unsigned)ne(J) && mus > 0.0f && w >= (float)kWeight0 && nidx == o2.w) {
+      if (o2.y != mus) prop *= mus / o2.y;
+      flush(J);
+      el = nextel;
+      mua = o2.x; mus = o2.y; g = o2.z;
+      return true;
+    }
+    return rare(J, rng, nf, nextel, o2, cap, n_scat);
+  }
+
+  // The rest of a step that is neither a scatter nor a common crossing: no exit face, the end
+  // of a free path without scattering, the boundary, roulette, an index jump, a vacuum element.
+  // nf: the crossed face, whose plane is read again here (a common step keeps none of them).
+  __device__ __forceinline__ bool rare(const JobDev &J, R &rng, int nf, int nextel, const float4 o2, int32_t cap,
+                                       uint32_t &n_scat) {
+    if (nf < 0) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
+      return die(J, kEvLost);
+    }
+    bool on = true;
+    if (prop <= 0.0f) {
+      if (mus > 0.0f) {  // at the step limit
+        const Event ev = draw_event(rng.peek3());
+        rotate(ev);
+        rng.take(3);
+        prop = ev.path;
+        n_scat++;
+      } else {
+        rng.align();
+        prop = free_path_f(unif_open_f(rng), mus);
+      }
+    } else {
+      rng.reload();
+      on = cross_rare(J, rng, nf, nextel, o2);
+    }
+    if (on && nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
+      job_count(J, kJcCapped); job_ledger(J, kLgLost, f2d_int(w));
+      return die(J, kEvCapped);
+    }
+    return on;
+  }
+
+  // The boundary, roulette, an index jump, a vacuum element.
+  __device__ __forceinline__ bool cross_rare(const JobDev &J, R &rng, int nf, int nextel, const float4 o2) {
+    const float4 pf = __ldg(reinterpret_cast<const float4 *>((geomp(J) + el)->pl) + nf);
+    const float nx = pf.x, ny = pf.y, nz = pf.z;
     if (nextel < 0) {
       const int ib = -1 - nextel;
       const uint8_t bt = __ldg(J.bctype + ib);
       if (is_mirror(bt)) {
-        const float4 pf = face();
-        float dn = dx * pf.x + dy * pf.y + dz * pf.z;
-        dx -= 2.0f * dn * pf.x; dy -= 2.0f * dn * pf.y; dz -= 2.0f * dn * pf.z;
-        return kAlive;
+        const float dn = fmaf(dz, nz, fmaf(dx, nx, __fmul_rn(dy, ny)));
+        dx -= 2.0f * dn * nx; dy -= 2.0f * dn * ny; dz -= 2.0f * dn * nz;
+        return true;
       }
       const float bcn = d2f_int(__ldg(J.bcn + ib));
       if (bcn > 0.0f) {
-        const float4 pf = face();
-        if (fresnel(rng, pf.x, pf.y, pf.z, nidx / bcn)) return kAlive;
+        if (fresnel(rng, nx, ny, nz, nidx / bcn)) return true;
       }
       flush(J);
       if (!FD) add_f<R::kOneJob>(J, J.EBR + ib, w);
@@ -654,16 +709,7 @@ struct Walk3D32 {
       }
       tr.put(-1 - (int64_t)ib);
       tr.end();
-      return kDied;
-    }
-    // the common crossing (interior, scattering medium, weight above the roulette
-    // threshold, no index jump) tested at once
-    if (nextel < ne(J) && mus > 0.0f && w >= (float)kWeight0 && nidx == o2.w) {
-      if (o2.y != mus) prop *= mus / o2.y;
-      flush(J);
-      el = nextel;
-      mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;
-      return kAlive;
+      return false;
     }
     if (nextel >= J.Ne) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
@@ -673,21 +719,19 @@ struct Walk3D32 {
       prop = free_path_f(unif_open_f(rng), o2.y);
       if (roulette(J, rng)) return die(J, kEvRoulette);
       if (nidx != o2.w) {
-        const float4 pf = face();
-        if (fresnel(rng, pf.x, pf.y, pf.z, nidx / o2.w)) return kAlive;
+        if (fresnel(rng, nx, ny, nz, nidx / o2.w)) return true;
       }
     } else {
       if (roulette(J, rng)) return die(J, kEvRoulette);
       if (nidx != o2.w) {
-        const float4 pf = face();
-        if (fresnel(rng, pf.x, pf.y, pf.z, nidx / o2.w)) return kAlive;
+        if (fresnel(rng, nx, ny, nz, nidx / o2.w)) return true;
       }
       if (o2.y != mus) prop *= mus / o2.y;
     }
     flush(J);
     el = nextel;
     mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;
-    return kAlive;
+    return true;
   }
 };
 
