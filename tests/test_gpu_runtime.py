@@ -306,3 +306,32 @@ def test_step_limit_of_the_tracking_form(built, name, cap):
     wide, _ = V.run_batch([mesh], [p], max_steps=free.stats["steps"], normalize=False)
     np.testing.assert_allclose(wide[0].ER, free.ER, rtol=1e-9, atol=1e-9)
     mesh.close()
+
+
+@pytest.mark.parametrize("name,precision", [("phantom3d", V.VMC_FP32), ("phantom3d_fd", V.VMC_FP32),
+                                            ("square2d", V.VMC_FP32), ("mixed2d_fd", V.VMC_FP32),
+                                            ("phantom3d", V.VMC_FP64), ("mixed2d_fd", V.VMC_FP64)])
+@pytest.mark.parametrize("n,block", [(1, 0), (33, 0), (609, 64), (2500, 0), (19457, 128), (160001, 0)])
+def test_photons_dealt_and_moved_between_lanes_walk_alike(built, name, precision, n, block):
+    """n photons in one launch equal the same photons in two launches of other sizes, whose lanes,
+    warps and packing differ: only the order of the FP64 additions does."""
+    if precision == V.VMC_FP64 and n > 20000:
+        pytest.skip("the FP64 forms run the smaller counts")
+    p = cases()[name][0].copy(Nphoton=n, seed=4242)
+    one = V.run(p, precision=precision, normalize=False, block_size=block)
+    assert one.stats["photons_done"] == n
+    cut = n // 3
+    parts = [V.run(p, precision=precision, nphoton=k, seed=4242, normalize=False, photon_offset=o)
+             for k, o in ((cut, 0), (n - cut, cut))]
+    assert one.stats["steps"] == sum(x.stats["steps"] for x in parts)
+    assert one.stats["scatters"] == sum(x.stats["scatters"] for x in parts)
+    for k in ("ER", "EI", "EBR", "EBI", "DEBR", "DEBI"):
+        total = sum(getattr(x, k) for x in parts)
+        np.testing.assert_allclose(getattr(one, k), total, rtol=1e-9, atol=1e-9)
+    mesh = V.Mesh(p, precision=precision)  # per-job form: photons of two jobs in the lanes of a warp
+    both, st = V.run_batch([mesh, mesh], [p.copy(Nphoton=cut), p.copy(Nphoton=n - cut, seed=77)], precision=precision,
+                           normalize=False)
+    assert st["photons_done"] == n
+    if p.f == 0.0 or precision == V.VMC_FP64:  # the FP32 one-job form rounds the phase differently
+        np.testing.assert_allclose(both[0].EBR, parts[0].EBR, rtol=1e-9, atol=1e-9)
+    mesh.close()

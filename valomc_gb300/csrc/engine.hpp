@@ -97,7 +97,7 @@ struct LaunchArena {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaStream_t cap_stream = nullptr;  // graph capture
   cudaGraphExec_t exec = nullptr;
-  int64_t total = 0;
+  int64_t total = 0, next0 = 0;  // photons, and those dealt out before the fetch counter starts
   bool pending = false;
   LaunchArena() = default;
   LaunchArena(const LaunchArena &) = delete;
@@ -122,6 +122,8 @@ const void *kernel_2d32(bool fd, bool tape, bool one, bool tab);
 // tab: the per-job form with the job table copied into each CTA's shared memory
 const void *select_kernel(const LaunchSpec &s, bool one = false, bool tab = false);
 void set_single_job(LaunchParams &lp, const JobDev &job);
+// the photons that the warps of a launch start with (lp.total is set)
+void deal_photons(LaunchParams &lp, int grid, int block, int per_sm, int sms);
 // the L1 / shared-memory split of a pool kernel: reset to the driver's default before the
 // occupancy query, then the smallest split holding per_sm CTAs' shared memory
 void reset_carveout(const void *fn);

@@ -33,6 +33,62 @@ __device__ __forceinline__ int find_job(const int64_t *begin, int njobs, int64_t
   return lo;
 }
 
+// ---- the end of a launch ----
+// Once the photons have been handed out, lanes die and are not replaced, yet a warp costs as
+// much with one live lane as with most of them: on the 648k-tet phantom, whose longest walks
+// take ten times the mean, half of a 1e6-photon launch ran in warps that were mostly empty.
+// So the CTA's warps then meet every kPackEvery steps, and when the photons alive would fit
+// three quarters of the warps that hold them they are moved together through shared memory, a
+// few words of the state at a time.  A photon's arithmetic does not depend on the lane that
+// carries it.  With the photons of small launches dealt to all SMs alike (below): 35.9 ->
+// 29.6 ms for 1e6 photons on the phantom (32.1 without), 20.5 -> 13.4 at 1e5, 13-18 -> 9.6 at
+// 1e4; FP64 571 -> 313 ms at 1e5.  Meeting every 64 to 512 steps measured alike there; every 64
+// cost the 2D square and a 2D frequency-domain mesh, whose walks are short, 2-4 %, and the 2D
+// tracking form does without (kPack).
+constexpr unsigned kPackEvery = 512;
+// the warp of a CTA that comes first, by the CTA's place on its SM
+__device__ __forceinline__ int warp_turn(const LaunchParams &lp, int warps) {
+  return (int)((long long)blockIdx.x * lp.ctas_per_sm / gridDim.x) % warps;
+}
+template <class Slot>  // uint2 or uint4: the words moved between two barriers
+struct Packer {
+  static constexpr int kWords = sizeof(Slot) / 4;
+  Slot *buf;  // one per thread of the CTA
+  int src;    // the thread whose photon this one takes, -1: none
+  // to: the thread that takes this one's photon (-1: none to give)
+  __device__ __forceinline__ Packer(Slot *b, int to) : buf(b) {
+    int32_t *from = reinterpret_cast<int32_t *>(b);
+    __syncthreads();
+    from[threadIdx.x] = -1;
+    __syncthreads();
+    if (to >= 0) from[to] = (int)threadIdx.x;
+    __syncthreads();
+    src = from[threadIdx.x];
+    __syncthreads();
+  }
+  template <class T> __device__ __forceinline__ static void get(const T &x, uint32_t *w) { memcpy(w, &x, sizeof(T)); }
+  template <class T> __device__ __forceinline__ static void set(T &x, const uint32_t *w) { memcpy(&x, w, sizeof(T)); }
+  // moves the values given (each of 4, 8 or 16 bytes)
+  template <class... T> __device__ __forceinline__ void operator()(T &...x) const {
+    constexpr int n = (int)((sizeof(T) + ...) / 4);
+    uint32_t w[(n + kWords - 1) / kWords * kWords] = {};
+    int at = 0;
+    ((get(x, w + at), at += (int)sizeof(T) / 4), ...);
+#pragma unroll
+    for (int i = 0; i < n; i += kWords) {
+      Slot v;
+      memcpy(&v, w + i, sizeof(Slot));
+      buf[threadIdx.x] = v;
+      __syncthreads();
+      if (src >= 0) v = buf[src];
+      __syncthreads();
+      memcpy(w + i, &v, sizeof(Slot));
+    }
+    at = 0;
+    ((set(x, w + at), at += (int)sizeof(T) / 4), ...);
+  }
+};
+
 // R::kOneJob: a launch of one job, whose descriptor (lp.job0) and Philox round keys are read
 // from the kernel parameters (constant bank) rather than from global memory and registers.
 // kTab: a launch of at most kSmemJobs jobs whose CTAs first copy the job table and its
@@ -80,57 +136,120 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
     for (int i = threadIdx.x; i < lp.dense; i += blockDim.x) sm[i] = 0.0;
     __syncthreads();
   }
-  bool alive = false, done = false;
-  unsigned long long n_steps = 0;
-  uint32_t n_scat = 0, n_done = 0;
-  long long chunk_next = 0, chunk_end = 0;
+  bool alive = false;
+  uint32_t n_steps = 0, n_scat = 0, n_done = 0;
   const unsigned lane = threadIdx.x & 31u;
+  long long chunk_next;  // this warp's next photon
+  int chunk_left;        // photons it may still take, -1: every photon has been handed out
+  {
+    // A launch with fewer photons than lanes deals them out, lp.fill to a warp (0 otherwise):
+    // first to the warps that come first in their CTA, one of each, and so on, so that every SM
+    // gets as many; "first" turns with the CTA's place on its SM, so that those warps sit on
+    // different schedulers.  All other photons come from the launch's counter.
+    const int warps = blockDim.x >> 5;
+    const int k = ((int)(threadIdx.x >> 5) + warps - warp_turn(lp, warps)) % warps;
+    chunk_next = min(((long long)k * gridDim.x + blockIdx.x) * lp.fill, (long long)lp.total);
+    chunk_left = (int)min((long long)lp.fill, (long long)lp.total - chunk_next);
+  }
+  __shared__ uint32_t pack_count[2][8];
+  __shared__ volatile int launch_dry;  // a warp of the CTA has found every photon handed out
+  if (W::kPack) {
+    if (threadIdx.x == 0) launch_dry = 0;
+    __syncthreads();
+  }
+  bool dry = false;  // the CTA's warps meet and pack from now on
   const unsigned lt_mask = (1u << lane) - 1u;
-  const long long total = lp.total;
   const int32_t cap = (int32_t)min(lp.max_steps, (int64_t)INT32_MAX);
   for (unsigned it = 0;; ++it) {
-    if ((it & 1023u) == 0u) {  // the host's cancel flag (an L2 round trip), every 1024 steps
-      if (*reinterpret_cast<volatile const int32_t *>(&lp.ctl->cancel)) {
-        if (alive) n_steps += (unsigned long long)s.nsteps;  // an unfinished walk's steps count in the launch's total
-        done = true;
-        alive = false;
-      }
-    }
-    // refill and the exit test only when some lane is idle (one vote in the common case)
-    if (__any_sync(kFull, !alive)) {
-    unsigned need = __ballot_sync(kFull, !alive && !done);
-    // short walks: wait (at most 7 iterations) until enough lanes are idle to launch together
-    if (__popc(need) < lp.refill_min && (it & 7u) != 0u) need = 0u;
-    while (need) {
-      if (chunk_next >= chunk_end) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&lp.ctl->next_photon, (unsigned long long)lp.chunk);
-        base = __shfl_sync(kFull, base, 0);
-        if ((long long)base >= total) {
-          if (!alive) done = true;
-          break;
-        }
-        chunk_next = (long long)base;
-        chunk_end = min(chunk_next + (long long)lp.chunk, total);
-      }
-      const long long avail = chunk_end - chunk_next;
-      const int rank = __popc(need & lt_mask);
-      if (((need >> lane) & 1u) && rank < avail) {
-        const long long p = chunk_next + rank;
-        if constexpr (!kOne) J = jobs + (lp.njobs > 1 ? find_job(job_begin, lp.njobs, p) : 0);
-        const long long q = p - J->pbegin;
-        start_rng(rng, *J, q);
-        s.launch(*J, rng, q);
-        alive = true;
-        if constexpr (W::kLaunchLoss) {
-          if (s.lost_at_launch(*J)) { alive = false; n_done++; }
+    if ((it & 31u) == 0u) {
+      if ((it & 1023u) == 0u) {  // the host's cancel flag (an L2 round trip), every 1024 steps
+        if (*reinterpret_cast<volatile const int32_t *>(&lp.ctl->cancel)) {
+          if (alive) n_steps += (uint32_t)s.nsteps;  // an unfinished walk's steps count in the launch's total
+          alive = false;
+          chunk_left = -1;
+          if (W::kPack) launch_dry = 1;
         }
       }
-      chunk_next += min((long long)__popc(need), avail);
-      need = __ballot_sync(kFull, !alive && !done);
+      if (W::kPack && !dry && __shfl_sync(kFull, launch_dry, 0) != 0) {
+        dry = true;
+        it = 0;
+      }
+      if (W::kPack && dry) {
+        if (it % kPackEvery == 0u) {
+          // every warp of the CTA comes here, the same number of times
+          const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+          uint32_t *count = pack_count[(it / kPackEvery) & 1u];
+          const unsigned live = __ballot_sync(kFull, alive);
+          if (lane == 0) count[warp] = (uint32_t)__popc(live) | (chunk_left > 0 ? 0x10000u : 0u);
+          __syncthreads();
+          int all = 0, before = 0, used = 0;
+          bool pending = false;
+          for (int k = 0; k < warps; k++) {
+            const int c = (int)(count[k] & 0xffffu);
+            pending |= count[k] > 0xffffu;
+            before += k < warp ? c : 0;
+            all += c;
+            used += c > 0;
+          }
+          if (all == 0 && !pending) break;
+          const int want = (all + 31) >> 5;
+          if constexpr (!R::kReplay) {
+            if (!pending && 4 * want <= 3 * used) {
+              const int each = (all + want - 1) / want;
+              const int k = before + __popc(live & lt_mask);
+              const int to = alive ? ((k / each + warp_turn(lp, warps)) % warps) * 32 + k % each : -1;
+              auto slot = rng.take_slot();  // the lanes' stream slots are the buffer
+              const Packer<decltype(slot)> pack(rng.slots(), to);
+              s.move(pack);
+              rng.template move<W::kBuffered>(pack, slot);
+              if constexpr (!kOne) pack(J);
+              rng.put_slot(slot);
+              alive = pack.src >= 0;
+            }
+          }
+        }
+        if (chunk_left <= 0 && !__any_sync(kFull, alive)) {
+          it |= kPackEvery - 1u;  // nothing to do until the next meeting
+          continue;
+        }
+      }
     }
-    if (__all_sync(kFull, done)) break;
+    // refill only when some lane is idle and photons are left (one vote in the common case)
+    if (chunk_left >= 0 && __any_sync(kFull, !alive)) {
+      unsigned need = __ballot_sync(kFull, !alive);
+      // short walks: wait (at most 7 iterations) until enough lanes are idle to launch together
+      if (__popc(need) < lp.refill_min && (it & 7u) != 0u) need = 0u;
+      while (need) {
+        if (chunk_left == 0) {
+          unsigned long long base = 0;
+          if (lane == 0) base = atomicAdd(&lp.ctl->next_photon, (unsigned long long)lp.chunk);
+          chunk_next = (long long)__shfl_sync(kFull, base, 0) + lp.next0;
+          if (chunk_next >= lp.total) {
+            chunk_left = -1;
+            if (W::kPack) launch_dry = 1;
+            break;
+          }
+          chunk_left = (int)min((long long)lp.chunk, (long long)lp.total - chunk_next);
+        }
+        const int rank = __popc(need & lt_mask);
+        if (((need >> lane) & 1u) && rank < chunk_left) {
+          const long long p = chunk_next + rank;
+          if constexpr (!kOne) J = jobs + (lp.njobs > 1 ? find_job(job_begin, lp.njobs, p) : 0);
+          const long long q = p - J->pbegin;
+          start_rng(rng, *J, q);
+          s.launch(*J, rng, q);
+          alive = true;
+          if constexpr (W::kLaunchLoss) {
+            if (s.lost_at_launch(*J)) { alive = false; n_done++; }
+          }
+        }
+        const int taken = min(__popc(need), chunk_left);
+        chunk_next += taken;
+        chunk_left -= taken;
+        need = __ballot_sync(kFull, !alive);
+      }
     }
+    if (!W::kPack && chunk_left < 0 && !__any_sync(kFull, alive)) break;
     if (alive) {
       if constexpr (W::kCap32) {
         alive = s.step(*J, rng, cap, n_scat);
@@ -141,7 +260,7 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
       }
       if (!alive) {
         n_done++;
-        n_steps += (unsigned long long)s.nsteps;
+        n_steps += (uint32_t)s.nsteps;
         job_count_add(*J, kJcSteps, (unsigned long long)s.nsteps);
       }
     }

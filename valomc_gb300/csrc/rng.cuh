@@ -45,6 +45,20 @@ struct PhiloxT {
     c0 = (uint32_t)photon;
     c2 = 0; n = 0;
   }
+  // Moves the stream's state between lanes at the end of a launch; kBuf: with the words left
+  // in the block.  The lanes' slots are taken out before, so that they serve as the buffer of
+  // the move, and put back after it.
+  template <bool kBuf, class F, class S> __device__ __forceinline__ void move(const F &f, S &slot) {
+    if constexpr (kBuf) f(c0, c2, n, slot, buf);
+    else f(c0, c2, n, slot);
+  }
+  __device__ __forceinline__ static auto *slot_ptr() {
+    if constexpr (kLaunchKey) return philox_slot_hi_stream();
+    else return philox_slot();
+  }
+  __device__ __forceinline__ static auto take_slot() { return *slot_ptr(); }
+  template <class S> __device__ __forceinline__ static void put_slot(const S &v) { *slot_ptr() = v; }
+  __device__ __forceinline__ static auto *slots() { return slot_ptr() - threadIdx.x; }
   __device__ __forceinline__ void block() {
     uint4 k;  // (key lo, key hi, photon hi, stream); the one-job form's key is in rk
     if constexpr (kLaunchKey) {

@@ -297,6 +297,13 @@ void set_single_job(LaunchParams &lp, const JobDev &job) {
   }
 }
 
+void deal_photons(LaunchParams &lp, int grid, int block, int per_sm, int sms) {
+  const int64_t warps = (int64_t)grid * (block / 32);
+  lp.fill = lp.total <= warps * 32 ? fill_of(lp.total, sms) : 0;
+  lp.ctas_per_sm = per_sm;
+  lp.next0 = std::min<int64_t>(lp.total, warps * lp.fill);
+}
+
 // ---------------------------------------------------------------------------------------
 // launch
 // ---------------------------------------------------------------------------------------
@@ -365,7 +372,7 @@ namespace {
 struct LaunchPlan {
   const void *fn = nullptr;
   bool one = false, tab = false;
-  int grid = 0, block = 0, stage_slots = 0, dense = 0;
+  int grid = 0, block = 0, per_sm = 0, sms = 0, stage_slots = 0, dense = 0;
   size_t smem = 0;
   int64_t total = 0;
   std::vector<JobDev> jobs;
@@ -430,6 +437,8 @@ int plan_launch(int device, const LaunchSpec &spec, const std::vector<JobDev> &j
     }
   }
   if (spec.blocks_per_sm > 0) per_sm = std::min(per_sm, spec.blocks_per_sm);
+  p.per_sm = per_sm;
+  p.sms = sms;
   p.grid = per_sm * sms;
   fit_carveout(p.fn, device, per_sm, p.smem);
   res.grid = p.grid;
@@ -451,6 +460,7 @@ LaunchParams make_params(const LaunchSpec &spec, const LaunchPlan &p, const JobD
   lp.stage_slots = p.stage_slots;
   lp.dense = p.dense;
   lp.refill_min = spec.refill > 0 ? spec.refill : kDefaultRefill;
+  deal_photons(lp, p.grid, p.block, p.per_sm, p.sms);
   return lp;
 }
 
@@ -558,7 +568,8 @@ int launch_jobs(int device, const LaunchSpec &spec, const std::vector<JobDev> &j
         last = now;
         VMC_CK(cudaMemcpyAsync(h_next, &dctl.p->next_photon, 8, cudaMemcpyDeviceToHost, side.s));
         VMC_CK(cudaStreamSynchronize(side.s));
-        double pct = 100.0 * (double)std::min<unsigned long long>(*h_next, (unsigned long long)total) / (double)total;
+        double pct = 100.0 * (double)std::min<unsigned long long>(*h_next + (unsigned long long)lp.next0,
+                                                                  (unsigned long long)total) / (double)total;
         if (!opt->progress(pct, opt->progress_user)) { stop = true; if (status == VMC_OK) status = VMC_ERR_CANCELLED; }
       }
       if (stop && !cancel_sent) {
@@ -634,6 +645,7 @@ int launch_start(int device, const LaunchSpec &spec, const std::vector<JobDev> &
   VMC_TRY(h2d(a.djobs, a.hjobs, nj, st));
   VMC_TRY(h2d(a.dbegin, a.hbegin, nj + 1, st));
   LaunchParams lp = make_params(spec, plan, a.djobs, a.dbegin, a.dctl);
+  a.next0 = lp.next0;
   void *args[] = {&lp};
   if (!spec.graph) {
     VMC_CK(cudaMemsetAsync(a.dctl, 0, sizeof(Ctl), st));

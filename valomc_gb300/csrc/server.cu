@@ -129,7 +129,7 @@ void wait_until_drain_nears(vmc_server &s, Lane &R, cudaStream_t probe, unsigned
               cudaSuccess ||
           cudaStreamSynchronize(probe) != cudaSuccess)
         break;
-      if ((double)*hnext >= 0.85 * (double)a->total) break;
+      if ((double)*hnext + (double)a->next0 >= 0.85 * (double)a->total) break;
     }
     {
       std::lock_guard<std::mutex> lk(s.mu);

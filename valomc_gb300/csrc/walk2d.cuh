@@ -28,8 +28,10 @@ __device__ __forceinline__ bool ray_seg(const double R[2], const double D[2], co
 
 template <bool FD, class R>
 struct Walk2D64 {
+  static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
+  static constexpr bool kPack = true;
   static constexpr bool kCap32 = false;
-  static constexpr int kMinBlocks = 1;
+  static constexpr int kMinBlocks = 2;
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
   Stage stage;
@@ -41,6 +43,12 @@ struct Walk2D64 {
   int el, curface;
   int64_t nsteps;
   Tr tr;
+
+  // moves the photon's state between lanes (Packer)
+  template <class F> __device__ __forceinline__ void move(const F &f) {
+    if constexpr (FD) f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, acc, phase, cph, sph, accI, el, curface, nsteps);
+    else f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, acc, el, curface, nsteps);
+  }
 
   __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
     const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
@@ -276,6 +284,8 @@ struct Walk2D64 {
 
 template <bool FD, class R>
 struct Walk2D32 {
+  static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
+  static constexpr bool kPack = false;  // its walks are short: packing gains nothing and costs the loop 2 %
   static constexpr bool kCap32 = false;
   static constexpr int kMinBlocks = 4;
   static constexpr bool kStaged = false;
@@ -289,6 +299,12 @@ struct Walk2D32 {
   int32_t nsteps;
   bool outward;  // launched out through its own entry edge
   Tr tr;
+
+  // moves the photon's state between lanes (Packer)
+  template <class F> __device__ __forceinline__ void move(const F &f) {
+    if constexpr (FD) f(px, py, dx, dy, w, prop, mua, mus, g, nidx, acc, phase, accI, el, nsteps);
+    else f(px, py, dx, dy, w, prop, mua, mus, g, nidx, acc, el, nsteps);
+  }
 
   __device__ __forceinline__ float4 optics(const JobDev &J, int e) const {
     return __ldg(reinterpret_cast<const float4 *>(J.optics) + (e & J.opt_mask));
@@ -474,17 +490,40 @@ struct Walk2D32 {
     }
     const float nx = lsel(l0, l1, l2, nf, 0), ny = lsel(l0, l1, l2, nf, 1);
     const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nb.z;
-    if (nextel < 0) {
-      const int ib = -1 - nextel;
-      const uint8_t bt = __ldg(J.bctype + ib);
-      if (is_mirror(bt)) {
-        float dn = dx * nx + dy * ny;
+    const int ib = -1 - nextel;  // the boundary edge when nextel < 0
+    const bool inside = nextel >= 0;
+    if (nextel >= J.Ne) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
+      return die(J, kEvLost);
+    }
+    float4 o2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (inside) {
+      o2 = optics(J, nextel);
+      // the common crossing (scattering medium, weight above the roulette threshold, no index
+      // jump) tested at once
+      if (mus > 0.0f && w >= (float)kWeight0 && nidx == o2.w) {
+        if (o2.y != mus) prop *= mus / o2.y;
+        flush(J);
+        el = nextel;
+        mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;
+        return kAlive;
+      }
+    } else {
+      if (is_mirror(__ldg(J.bctype + ib))) {
+        const float dn = fmaf(dy, ny, __fmul_rn(dx, nx));
         dx -= 2.0f * dn * nx; dy -= 2.0f * dn * ny;
         return kAlive;
       }
-      const float bcn = d2f_int(__ldg(J.bcn + ib));
-      if (bcn > 0.0f && fresnel(rng, nx, ny, nidx / bcn, true)) return kAlive;
-      float dn = dx * nx + dy * ny;
+      o2.w = d2f_int(__ldg(J.bcn + ib));
+    }
+    // one copy of roulette and of the interface for elements and the boundary: each holds a
+    // Philox block per draw, and the kernel waits for instructions as it is
+    const bool vacuum = inside && mus <= 0.0f && o2.y > 0.0f;
+    if (vacuum) prop = free_path_f(unif_open_f(rng), o2.y);
+    if (inside && roulette(J, rng)) return die(J, kEvRoulette);
+    if ((inside ? nidx != o2.w : o2.w > 0.0f) && fresnel(rng, nx, ny, nidx / o2.w, !inside)) return kAlive;
+    if (!inside) {
+      const float dn = fmaf(dy, ny, __fmul_rn(dx, nx));
       flush(J);
       if (!FD) {
         add_f<R::kOneJob>(J, J.EBR + ib, w);
@@ -501,29 +540,7 @@ struct Walk2D32 {
       tr.end();
       return kDied;
     }
-    if (nextel >= J.Ne) {
-      job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
-      return die(J, kEvLost);
-    }
-    const float4 o2 = optics(J, nextel);
-    // the common crossing (scattering medium, weight above the roulette threshold, no index
-    // jump) tested at once
-    if (mus > 0.0f && w >= (float)kWeight0 && nidx == o2.w) {
-      if (o2.y != mus) prop *= mus / o2.y;
-      flush(J);
-      el = nextel;
-      mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;
-      return kAlive;
-    }
-    if (mus <= 0.0f && o2.y > 0.0f) {
-      prop = free_path_f(unif_open_f(rng), o2.y);
-      if (roulette(J, rng)) return die(J, kEvRoulette);
-      if (nidx != o2.w && fresnel(rng, nx, ny, nidx / o2.w, false)) return kAlive;
-    } else {
-      if (roulette(J, rng)) return die(J, kEvRoulette);
-      if (nidx != o2.w && fresnel(rng, nx, ny, nidx / o2.w, false)) return kAlive;
-      if (o2.y != mus) prop *= mus / o2.y;
-    }
+    if (!vacuum && o2.y != mus) prop *= mus / o2.y;
     flush(J);
     el = nextel;
     mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;

@@ -119,8 +119,10 @@ __device__ __forceinline__ float free_path_f(float u, float mus) {
 // =====================================================================================
 template <bool FD, class R>
 struct Walk3D64 {
+  static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
+  static constexpr bool kPack = true;
   static constexpr bool kCap32 = false;
-  static constexpr int kMinBlocks = 1;  // ~125 registers: 2 CTAs of 256 per SM
+  static constexpr int kMinBlocks = 2;  // ~125 registers: 2 CTAs of 256 per SM
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
   Stage stage;
@@ -132,6 +134,12 @@ struct Walk3D64 {
   int el, curface;
   int64_t nsteps;
   Tr tr;
+
+  // moves the photon's state between lanes (Packer)
+  template <class F> __device__ __forceinline__ void move(const F &f) {
+    if constexpr (FD) f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, acc, phase, cph, sph, accI, el, curface, nsteps);
+    else f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, acc, el, curface, nsteps);
+  }
 
   __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
     const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
@@ -389,6 +397,8 @@ struct Walk3D32 {
   // per SM beat 24 (+7% on the 648k-tet phantom); 5 CTAs (48 registers) spill and lose
   static constexpr int kMinBlocks = 4;
   static constexpr bool kStaged = !FD;
+  static constexpr bool kBuffered = false;  // words left in a block are carried from step to step
+  static constexpr bool kPack = true;
   static constexpr bool kCap32 = true;
   using Tr = typename TraceFor<R>::type;
   float px, py, pz, dx, dy, dz;
@@ -408,6 +418,13 @@ struct Walk3D32 {
   const Tet32 *hg;
   const float4 *ho;
   int32_t hm, hne;
+
+  // moves the photon's state between lanes (Packer)
+  template <class F> __device__ __forceinline__ void move(const F &f) {
+    if constexpr (FD) f(px, py, pz, dx, dy, dz, w, prop, mua, mus, g, nidx, acc, phase, accI, el, nsteps);
+    else f(px, py, pz, dx, dy, dz, w, prop, mua, mus, g, nidx, acc, el, nsteps);
+    if constexpr (!R::kOneJob) f(hg, ho, hm, hne);
+  }
 
   __device__ __forceinline__ const Tet32 *geomp(const JobDev &J) const {
     if constexpr (R::kOneJob) return reinterpret_cast<const Tet32 *>(J.geom);

@@ -273,6 +273,7 @@ __device__ __forceinline__ void create_photon_3d_f(const JobDev &J, R &rng, floa
     pos[0] = S.L[0]; pos[1] = S.L[1]; pos[2] = S.L[2];
   } else if ((dt == 'n' && bt == 'i') || (dt != 'n' && (bt == 'i' || bt == 'I'))) {
     float rr0 = n0, rr1 = n1, rr2 = n2;
+#pragma unroll 1
     for (int it = 0; it < kMaxRejections; it++) {
       const float th2 = 2.0f * unif_halfup_f(rng);  // theta / pi
       const float u = 2.0f * unif_closed_f(rng) - 1.0f;
@@ -298,6 +299,7 @@ template <class R>
 __device__ __forceinline__ float gauss_angle_f(R &rng, float sigma, float h) {
   const float xi = unif_open_f(rng);
   float a = -0.5f * (float)kPi, b = 0.5f * (float)kPi, phi = 0.0f;
+#pragma unroll 1
   for (int it = 0; it < 16; it++) {
     phi = 0.5f * (a + b);
     const float cdf = (0.5f + 0.5f * erff(phi / sigma * 0.70710678118654752f) - h) / (1.0f - 2.0f * h);
@@ -328,6 +330,7 @@ __device__ __forceinline__ void create_photon_2d_f(const JobDev &J, R &rng, floa
     dir[0] = S.cphi0 * cp - S.sphi0 * sp;
     dir[1] = S.sphi0 * cp + S.cphi0 * sp;
   } else if (bt == 'c' || bt == 'g') {
+#pragma unroll 1
     for (int it = 0; it < kMaxRejections; it++) {
       float sp, cp;
       if (bt == 'c') {  // phi = asin(s): sin phi = s, cos phi = sqrt(1 - s^2)
