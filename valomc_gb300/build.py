@@ -19,8 +19,8 @@ LIB = os.path.join(BUILD, "libvalomc_gb300.so")
 INCLUDE = os.path.join(ROOT, "include")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-CU_UNITS = ["kern3d32.cu", "kern3d64.cu", "kern2d32.cu", "kern2d64.cu", "runtime.cu", "tools.cu", "server.cu",
-            "noalloc.cu"]
+CU_UNITS = ["kern3d32.cu", "kern3d64.cu", "kern2d32.cu", "kern2d64.cu", "kern3d64l.cu", "kern2d64l.cu", "runtime.cu",
+            "tools.cu", "server.cu", "noalloc.cu", "geometry.cu"]
 # The tetrahedral tracking kernel flushes FP32 subnormals: its reciprocals, roots, logarithms and
 # exponentials then need no scaling around them (5 % fewer instructions a step; 202.2 -> 197.2 ms
 # for 1e7 photons on the 648k-tet phantom).  A walk meets none: lengths are clamped at 0 and the

@@ -37,6 +37,8 @@ struct DeviceMesh {
   const void *geom(int precision) const { return d_geom[precision]; }
 };
 int upload_mesh(DeviceMesh &m, int precision_mask);
+// TetRec / TriRec [Ne] at `geom` from the Tet64 / Tri64 [Ne] behind them
+cudaError_t make_plane_records(int dim, void *geom, int64_t Ne, cudaStream_t st);
 
 // Device state of one job.
 struct JobBuffers {
@@ -70,6 +72,7 @@ int zero_job(JobBuffers &b, cudaStream_t st);
 struct LaunchSpec {
   int dim = 3, precision = VMC_FP32;
   bool fd = false, tape = false;
+  bool literal = false; // FP64: the reference's operation sequence (rough_optics)
   bool graph = false;  // launch through a (reused) CUDA graph
   int stage_slots = 0; // shared-memory staging slots per CTA (0: off)
   int block = 0, blocks_per_sm = 0, chunk = 0;
@@ -115,8 +118,10 @@ int collect_job(const HostJob &j, const DeviceMesh &m, const JobBuffers &b, int6
                 vmc_output *out, vmc_stats *st, cudaStream_t stream);
 
 const void *kernel_3d64(bool fd, bool tape, bool one, bool tab);
+const void *kernel_3d64_literal(bool fd, bool tape, bool one, bool tab);
 const void *kernel_3d32(bool fd, bool tape, bool one, bool tab);
 const void *kernel_2d64(bool fd, bool tape, bool one, bool tab);
+const void *kernel_2d64_literal(bool fd, bool tape, bool one, bool tab);
 const void *kernel_2d32(bool fd, bool tape, bool one, bool tab);
 // one: the single-job form (descriptor and round keys in LaunchParams::job0 / rk);
 // tab: the per-job form with the job table copied into each CTA's shared memory

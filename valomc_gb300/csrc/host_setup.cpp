@@ -355,6 +355,13 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
   double ph0 = in->phase0;
   if (ph0 < 0) ph0 += 2 * kPi * ceil(-ph0 / (2 * kPi));  // MC3D.cpp:141-143, MC3Dmex.cpp:158-160
   j.phase0 = ph0;
+  {  // the same in turns, for the plain form's fixed-point phase
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    j.k_turn = (double)((long double)j.k_scale / two_pi);
+    long double t = (long double)ph0 / two_pi;
+    t -= floorl(t);
+    j.turn0 = t >= 0 && t < 1 ? (uint64_t)ldexpl(t, 64) : 0;
+  }
   j.Nphoton = in->Nphoton;
   // optics rows; a job whose elements all share one row keeps a single row
   bool hom = Ne > 0;
@@ -532,6 +539,23 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
   }
   j.cdf_f[ns - 1] = 1.0f;
   return VMC_OK;
+}
+
+bool rough_optics(const vmc_input *in, const HostMesh &m) {
+  const int64_t Ne = m.Ne;
+  bool same = true;
+  for (int64_t i = 1; i < Ne && same; i++) same = in->mus[i] == in->mus[0] && in->n[i] == in->n[0];
+  if (same) return false;
+  int64_t faces = 0, changes = 0;
+#pragma omp parallel for schedule(static) reduction(+ : faces, changes) if (Ne > 20000)
+  for (int64_t i = 0; i < Ne; i++)
+    for (int f = 0; f <= m.dim; f++) {
+      const int64_t h = m.HN[(size_t)(i + Ne * f)];
+      if (h < 0 || h >= Ne) continue;
+      faces++;
+      changes += in->mus[i] != in->mus[h] || in->n[i] != in->n[h];
+    }
+  return 8 * changes > faces;
 }
 
 // MonteCarlo's normalisation, MC3D.hpp:1792-1818 / MC2D.hpp:1672-1703

@@ -44,10 +44,19 @@ struct HostJob {
   std::vector<SourceRecF> src_f;  // FP32 copies for the tracking form
   std::vector<float> cdf_f;
   double f = 0, omega = 0, k_scale = 0, phase0 = 0;
+  double k_turn = 0;            // k_scale / (2 pi)
+  uint64_t turn0 = 0;           // phase0 in 2^-64 turns
   int64_t Nphoton = 0;
   uint64_t seed = 0;
   std::vector<double> k;        // omega / c0 * n per element (FD normalisation)
 };
+
+// Whether the scattering coefficient or the index changes across more than an eighth of the mesh's
+// interior faces: such jobs run the literal FP64 walk.  A photon's remaining path is multiplied
+// by mus / mus2 at each of these faces, so rounding differences are too: on the 648k-tet phantom
+// with mus drawn per element (every face) walks of some thousand steps end elsewhere after any
+// change of rounding, while with one or two inclusions (2-4 % of the faces) results move by 1e-14.
+bool rough_optics(const vmc_input *in, const HostMesh &m);
 
 // ErrorChecks (same checks, same order, same codes).  Returns VMC_OK or 1 + mcerror.
 int check_input(const vmc_input *in);

@@ -206,6 +206,8 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   d.k_scale = hj.k_scale;
   d.k_scale_f = (float)hj.k_scale;
   d.phase0 = hj.phase0;
+  d.k_turn = hj.k_turn;
+  d.turn0 = hj.turn0;
   d.seed = hj.seed;
   d.stream = o.stream_id;
   d.pbegin = 0;
@@ -228,6 +230,7 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   spec.dim = m->host.dim;
   spec.precision = o.precision;
   spec.fd = hj.omega > 0.0;
+  spec.literal = o.precision == VMC_FP64 && rough_optics(&in, m->host);
   spec.tape = false;
   const void *fn = select_kernel(spec);
   int sms = 0;

@@ -118,17 +118,15 @@ int upload_mesh(DeviceMesh &m, int precision_mask) {
   m.dim = h.dim;
   cudaStream_t st = m.st;
   if ((precision_mask & 1) && !m.d_geom[VMC_FP64]) {
-    if (h.dim == 3) {
-      Tet64 *d;
-      VMC_TRY(dalloc(&d, h.tet64.size(), m.bytes, m.pool, st));
-      m.d_geom[VMC_FP64] = d;
-      VMC_TRY(h2d(d, h.tet64.data(), h.tet64.size(), st));
-    } else {
-      Tri64 *d;
-      VMC_TRY(dalloc(&d, h.tri64.size(), m.bytes, m.pool, st));
-      m.d_geom[VMC_FP64] = d;
-      VMC_TRY(h2d(d, h.tri64.data(), h.tri64.size(), st));
-    }
+    // the face-plane records, made on the device from the vertex records uploaded behind them
+    const size_t ne = (size_t)h.Ne, rec = h.dim == 3 ? sizeof(TetRec) : sizeof(TriRec);
+    const size_t vert = h.dim == 3 ? sizeof(Tet64) : sizeof(Tri64);
+    const void *src = h.dim == 3 ? static_cast<const void *>(h.tet64.data()) : h.tri64.data();
+    unsigned char *d;
+    VMC_TRY(dalloc(&d, ne * (rec + vert), m.bytes, m.pool, st));
+    m.d_geom[VMC_FP64] = d;
+    VMC_TRY(h2d(d + ne * rec, static_cast<const unsigned char *>(src), ne * vert, st));
+    VMC_CK(make_plane_records(h.dim, d, (int64_t)ne, st));
   }
   if ((precision_mask & 2) && !m.d_geom[VMC_FP32]) {
     if (h.dim == 3) {
@@ -237,6 +235,8 @@ JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, const 
   d.k_scale = j.k_scale;
   d.k_scale_f = (float)j.k_scale;
   d.phase0 = j.phase0;
+  d.k_turn = j.k_turn;
+  d.turn0 = j.turn0;
   d.seed = j.seed;
   d.ER = b.d_acc;
   d.EI = b.d_acc + Ne;
@@ -255,9 +255,11 @@ const void *select_kernel(const LaunchSpec &s, bool one, bool tab) {
   // trajectories, same registers), so they keep the descriptor and keys in global memory.
   one = one && !s.tape && s.precision == VMC_FP32;
   tab = tab && !one;
-  if (s.dim == 3)
-    return s.precision == VMC_FP64 ? kernel_3d64(s.fd, s.tape, one, tab) : kernel_3d32(s.fd, s.tape, one, tab);
-  return s.precision == VMC_FP64 ? kernel_2d64(s.fd, s.tape, one, tab) : kernel_2d32(s.fd, s.tape, one, tab);
+  const bool d3 = s.dim == 3;
+  if (s.precision != VMC_FP64) return d3 ? kernel_3d32(s.fd, s.tape, one, tab) : kernel_2d32(s.fd, s.tape, one, tab);
+  if (s.literal)
+    return d3 ? kernel_3d64_literal(s.fd, s.tape, one, tab) : kernel_2d64_literal(s.fd, s.tape, one, tab);
+  return d3 ? kernel_3d64(s.fd, s.tape, one, tab) : kernel_2d64(s.fd, s.tape, one, tab);
 }
 
 // The SM's unified L1 / shared-memory array is split per launch.  Left to itself the driver
@@ -857,6 +859,7 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   spec.dim = in->dim;
   spec.precision = o.precision;
   spec.fd = hj.omega > 0.0;
+  spec.literal = o.precision == VMC_FP64 && rough_optics(in, dm.host);
   spec.tape = o.rng == VMC_RNG_TAPE;
   spec.block = o.block_size;
   spec.blocks_per_sm = o.blocks_per_sm;
@@ -936,7 +939,7 @@ int mesh_precision_mask(const vmc_mesh *m) { return m ? m->precision_mask : 0; }
 }  // namespace vmc
 }
 
-// jobs of one (dim, frequency-domain) class share a launch
+// jobs of one (dim, frequency-domain, FP64 walk) class share a launch
 int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs, const vmc_options *opt_in,
                   vmc_output *outs, vmc_stats *stats, vmc_stats *job_stats) {
   auto t0 = std::chrono::steady_clock::now();
@@ -980,6 +983,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
     sp.dim = meshes[i]->m.host.dim;
     sp.precision = o.precision;
     sp.fd = hj[(size_t)i].omega > 0.0;
+    sp.literal = o.precision == VMC_FP64 && rough_optics(&jobs[i], meshes[i]->m.host);
     sp.block = o.block_size;
     sp.blocks_per_sm = o.blocks_per_sm;
     sp.chunk = o.fetch_chunk;
@@ -987,7 +991,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
     sp.graph = o.use_graph != 0;
     sp.stage_slots = o.stage_slots;
     sp.refill = o.refill_lanes;
-    auto it = std::find_if(groups.begin(), groups.end(), [&](const Group &g) { return g.spec.dim == sp.dim && g.spec.fd == sp.fd; });
+    auto it = std::find_if(groups.begin(), groups.end(), [&](const Group &g) { return g.spec.dim == sp.dim && g.spec.fd == sp.fd && g.spec.literal == sp.literal; });
     if (it == groups.end()) { groups.push_back(Group{sp, {}}); it = groups.end() - 1; }
     it->idx.push_back(i);
   }

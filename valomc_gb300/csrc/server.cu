@@ -48,6 +48,7 @@ struct Request {
   HostJob job;
   int64_t nphoton = 0, issued = 0;
   int64_t footprint = 0;
+  bool literal = false;  // FP64: the walk with the reference's operation sequence
   std::unique_ptr<JobBuffers> buf;
   int state = kQueued;
   int status = VMC_OK;
@@ -234,15 +235,15 @@ void vmc_server::loop() {
       const std::vector<int64_t> sl = epoch_slices(left, epoch, cfg.slicing != VMC_SLICE_EQUAL);
       for (size_t i = 0; i < open.size(); i++) open[i]->slice = sl[i];
     }
-    struct Cls { int dim; bool fd; std::vector<Request *> rs; };
+    struct Cls { int dim; bool fd, literal; std::vector<Request *> rs; };
     std::vector<Cls> classes;
     for (Request *r : open) {
       DeviceMesh *m = mesh_impl(meshes[(size_t)r->mesh_id]);
       bool fd = r->job.omega > 0;
       Cls *c = nullptr;
       for (auto &x : classes)
-        if (x.dim == m->host.dim && x.fd == fd) c = &x;
-      if (!c) { classes.push_back(Cls{m->host.dim, fd, {}}); c = &classes.back(); }
+        if (x.dim == m->host.dim && x.fd == fd && x.literal == r->literal) c = &x;
+      if (!c) { classes.push_back(Cls{m->host.dim, fd, r->literal, {}}); c = &classes.back(); }
       c->rs.push_back(r);
     }
     L.members.assign(classes.size(), {});
@@ -266,6 +267,7 @@ void vmc_server::loop() {
       sp.dim = c.dim;
       sp.precision = cfg.precision;
       sp.fd = c.fd;
+      sp.literal = c.literal;
       sp.block = cfg.block_size;
       sp.blocks_per_sm = cfg.blocks_per_sm;
       sp.graph = cfg.use_graph != 0;
@@ -459,6 +461,7 @@ int vmc_server_submit(vmc_server *s, int32_t mesh_id, const vmc_input *job, int6
   st = build_job(&in, m->host, r->job);
   if (st) return st;
   r->job.seed = in.seed_given ? in.seed : clock_seed();
+  r->literal = s->cfg.precision == VMC_FP64 && rough_optics(&in, m->host);
   r->mesh_id = mesh_id;
   r->nphoton = in.Nphoton;
   r->footprint = job_footprint(r->job, m->host);

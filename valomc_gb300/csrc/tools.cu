@@ -174,6 +174,7 @@ int vmc_autotune(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs, 
   const int nshape = 3 * 3 * 2 + 4;
   LaunchSpec base;
   base.dim = dim; base.precision = prec; base.fd = fd; base.max_steps = opt->max_steps;
+  base.literal = prec == VMC_FP64 && rough_optics(&jobs[0], mesh_impl(meshes[0])->host);
   auto run = [&](const LaunchSpec &sp, double frac, double &rate) -> int {
     std::vector<JobDev> d = descs;
     int64_t n = 0;

@@ -2,10 +2,12 @@
 //
 // Device layout (all arrays element-indexed, 16-byte aligned, one record per element so a
 // step's gather is a few 128-bit loads from consecutive sectors):
-//   Tet64 (112 B)  plain FP64 form: the four vertices of the tetrahedron (the reference's
-//                  r(H(el, v), c), cpp/3d/MC3D.hpp:1015-1018) + its HN row.
+//   TetRec (208 B) plain FP64 form: the face planes about vertex 0, in FP64 and FP32, + its HN row.
+//   Tet64 (112 B)  the four vertices of the tetrahedron (the reference's r(H(el, v), c),
+//                  cpp/3d/MC3D.hpp:1015-1018) + its HN row, behind the TetRecs: read where the
+//                  exit face has to be found by Moller-Trumbore.
 //   Tet32 (80 B)   FP32 tracking form: four outward face planes (unit normal, offset) + HN.
-//   Tri64 (64 B)   plain FP64 triangles: three vertices + HN row.
+//   TriRec (128 B), Tri64 (64 B)  the same for triangles.
 //   Tri32 (64 B)   FP32 triangles: three outward edge lines + HN row.
 // HN entries: neighbour element >= 0, boundary -1 - ib, or kOpenFace for a 3D face the
 // reference leaves at INT_FAST64_MAX (cpp/3d/MC3D.hpp:863).
@@ -33,6 +35,31 @@ struct alignas(16) Tet64 {
   int32_t nbr[4];
 };
 static_assert(sizeof(Tet64) == 112, "Tet64 layout");
+
+// The planes of a tetrahedron for the plain form: a point x lies on face f where n_f . (x - v0) =
+// off_f, off_3 = off, off_0..2 = 0.  n_f is the product of two edges that Moller-Trumbore forms
+// (twice the face's area long, exact on a grid of whole numbers), pointing out.  In FP32 the
+// normals have unit length (off_size: off over n_3's length); they pick the exit face where
+// rounding cannot matter, and are NaN in an element so small that the reference's parallel test
+// (|det| < DBL_EPSILON) could take part, which then never is picked by them.
+struct alignas(16) TetRec {
+  double v0[3], off;
+  float nf[4][3];
+  int32_t nbr[4];
+  double n[4][3];
+  float off_size, pad[3];
+};
+static_assert(sizeof(TetRec) == 208, "TetRec layout");
+
+// The edge lines of a triangle about vertex 0, the same way: off_1 = off, off_0 = off_2 = 0; n_f
+// is as long as its edge.
+struct alignas(16) TriRec {
+  double v0[2], off, pad;
+  float nf[3][2], off_size, padf;
+  int32_t nbr[4];  // 3 used
+  double n[3][2];
+};
+static_assert(sizeof(TriRec) == 128, "TriRec layout");
 
 struct alignas(16) Tet32 {
   float pl[4][4];  // (nx, ny, nz, d): n . x = d on the face, n points out of the element
@@ -118,6 +145,8 @@ struct JobDev {
   float k_scale_f;             // the same in FP32, for the tracking form
   int32_t dense;               // > 0: the launch stages the 2 Ne + 4 Nb accumulators per CTA in shared memory
   double phase0;
+  double k_turn;               // k_scale / (2 pi), and phase0 in 2^-64 turns: the plain form's phase
+  uint64_t turn0;
   uint64_t seed;
   uint32_t stream;
   int32_t trace_on;

@@ -1,7 +1,7 @@
 // walk2d.cuh -- the triangular photon walk (MC2D), one element step per call.
 //
-// Walk2D64 follows PropagatePhoton (cpp/2d/MC2D.hpp:1307-1511) with the reference's FP64
-// arithmetic: RayRayIntersects over the edges (0,1), (1,2), (2,0) skipping the entry edge
+// Walk2D64 follows PropagatePhoton (cpp/2d/MC2D.hpp:1307-1511) with its state in FP64:
+// RayRayIntersects' choice among the edges (0,1), (1,2), (2,0) skipping the entry edge
 // (WhichFace :914-955, :1710-1722), the 2D Henyey-Greenstein ScatterPhoton (:1135-1155),
 // FresnelPhoton whose boundary branch transmits without refraction (:1178-1304), and the
 // direction-weighted exitance DEBR/DEBI (:1410-1437).
@@ -26,8 +26,310 @@ __device__ __forceinline__ bool ray_seg(const double R[2], const double D[2], co
   return true;
 }
 
+// The plain form, on the same lines as the tetrahedral one (walk3d.cuh): FP64 for the state,
+// the exit edge picked in FP32 where that is certain, the samples on the integer pipe.
 template <bool FD, class R>
 struct Walk2D64 {
+  static constexpr bool kBuffered = false;
+  static constexpr bool kPack = true;
+  static constexpr bool kCap32 = true;
+  static constexpr int kMinBlocks = 2;
+  static constexpr bool kStaged = false;
+  static constexpr bool kLaunchLoss = false;
+  Stage stage;
+  using Tr = typename TraceFor<R>::type;
+  double pos[2], dir[2];
+  double w, prop, cph, sph;
+  double mua, mus, g, nidx, imus, kg;  // imus = 1 / mus, kg = (1 - g) / (1 + g)
+  double acc, accI;
+  uint64_t turn;  // phase in 2^-64 turns
+  int el, curface;
+  int32_t nsteps;
+  Tr tr;
+
+  // moves the photon's state between lanes (Packer)
+  template <class F> __device__ __forceinline__ void move(const F &f) {
+    if constexpr (FD) f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, imus, kg, acc, turn, cph, sph, accI, el, curface, nsteps);
+    else f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, imus, kg, acc, el, curface, nsteps);
+  }
+
+  __device__ __forceinline__ static const TriRec *recs(const JobDev &J) { return reinterpret_cast<const TriRec *>(J.geom); }
+  __device__ __forceinline__ static const Tri64 *verts(const JobDev &J) { return reinterpret_cast<const Tri64 *>(recs(J) + J.Ne); }
+
+  __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
+    const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
+    const double2 o0 = __ldg(o), o1 = __ldg(o + 1);
+    a = o0.x; s = o0.y; gg = o1.x; nn = o1.y;
+  }
+
+  // (1 - g) / (1 + g); at |g| = 1 the reference's sqrt((g^2 + 1)^2 - 4 g^2) is 0 and its angle NaN
+  __device__ __forceinline__ static double turn_factor(double g) {
+    return fabs(g) == 1.0 ? __longlong_as_double(0x7ff8000000000000ll) : fast_div(1.0 - g, 1.0 + g);
+  }
+
+  __device__ void launch(const JobDev &J, R &rng, int64_t q) {
+    tr.begin(J, q);
+    create_photon_2d(J, rng, pos, dir, el, curface);
+    w = 1.0;
+    if (FD) {
+      turn = J.turn0;
+      sincos_turn(turn, sph, cph);
+    }
+    optics(J, el, mua, mus, g, nidx);
+    imus = fast_rcp(mus);
+    kg = turn_factor(g);
+    prop = neg_log_open(rng.next()) * imus;
+    acc = accI = 0.0;
+    nsteps = 0;
+  }
+
+  __device__ __forceinline__ void flush(const JobDev &J) {
+    add_d(J, J.ER + el, acc);
+    if (FD) add_d(J, J.EI + el, accI);
+    acc = accI = 0.0;
+  }
+
+  __device__ __forceinline__ bool die(const JobDev &J, int64_t ev) {
+    flush(J);
+    tr.put(ev);
+    tr.end();
+    return false;
+  }
+
+  // ScatterPhoton (MC2D.hpp:1135-1155) turns the direction to atan2(dir) + 2 atan(h), h =
+  // tan(pi xi) (1 - g) / (1 + g).  Here the direction is turned by 2 atan(h): with (s0, c0) the
+  // sine and cosine of pi xi and ks = (1 - g) / (1 + g) s0, its cosine is
+  // (c0^2 - ks^2) / (c0^2 + ks^2) and its sine 2 ks c0 / (c0^2 + ks^2) -- no angle is formed.
+  __device__ __forceinline__ void scatter(uint32_t u) {
+    double c, s;
+    if (g != 0.0) {
+      double s0, c0;
+      sincos_turn((uint64_t)u << 31, s0, c0);
+      const double ks = kg * s0;
+      const double a = c0 * c0, b = ks * ks;
+      const double inv = fast_rcp(a + b) * unit_scale(fma(dir[0], dir[0], dir[1] * dir[1]));
+      c = (a - b) * inv;
+      s = 2.0 * ks * c0 * inv;
+      const double ux = dir[0], uy = dir[1];
+      dir[0] = fma(ux, c, -(uy * s));
+      dir[1] = fma(uy, c, ux * s);
+    } else {
+      sincos_turn((uint64_t)u << 32, s, c);
+      dir[0] = c;
+      dir[1] = s;
+    }
+    curface = -1;
+  }
+
+  __device__ __forceinline__ bool fresnel(R &rng, double n0, double n1, double nipnt, int nf, bool boundary) {
+    const double costhi = -(dir[0] * n0 + dir[1] * n1);
+    double costht = 0.0;
+    if (fresnel_reflects_d(rng, nipnt, costhi, costht)) {
+      const double k = 2.0 * costhi;
+      dir[0] = fma(k, n0, dir[0]);
+      dir[1] = fma(k, n1, dir[1]);
+      curface = nf;
+      return true;
+    }
+    if (boundary) return false;
+    const double m = (costhi > 0.0) ? (nipnt * costhi - costht) : (nipnt * costhi + costht);
+    dir[0] = fma(nipnt, dir[0], m * n0);
+    dir[1] = fma(nipnt, dir[1], m * n1);
+    return false;
+  }
+
+  // WhichFace, MC2D.hpp:914-955: edges (0,1), (1,2), (2,0) in order, skipping curface
+  struct Exit { double dist; int nf; };
+  __device__ __noinline__ static Exit which_face(const Tri64 *T, double px, double py, double dx, double dy, int curface) {
+    const double *v = &T->v[0][0];
+    const double pos[2] = {px, py}, dir[2] = {dx, dy};
+    double dist = 0.0;
+    if (curface != 0 && ray_seg(pos, dir, v, v + 2, dist) && dist > 0.0) return Exit{dist, 0};
+    if (curface != 1 && ray_seg(pos, dir, v + 2, v + 4, dist) && dist > 0.0) return Exit{dist, 1};
+    if (curface != 2 && ray_seg(pos, dir, v + 4, v, dist) && dist > 0.0) return Exit{dist, 2};
+    return Exit{0.0, -1};
+  }
+
+  // the exit edge and the distance to it, as in the tetrahedral walk
+  __device__ __forceinline__ int exit_face(const JobDev &J, double &dist, int4 &nbr) const {
+    const TriRec *T = recs(J) + el;
+    const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
+    const double offd = __ldg(&T->off);
+    const float4 q0 = __ldg(reinterpret_cast<const float4 *>(T->nf));
+    const float4 q1 = __ldg(reinterpret_cast<const float4 *>(T->nf) + 1);
+    nbr = __ldg(reinterpret_cast<const int4 *>(T->nbr));
+    const double rx = pos[0] - a0.x, ry = pos[1] - a0.y;
+    const float fx = f32_of(rx), fy = f32_of(ry), off = q1.z;
+    const float dx = f32_of(dir[0]), dy = f32_of(dir[1]);
+    const float n[3][2] = {{q0.x, q0.y}, {q0.z, q0.w}, {q1.x, q1.y}};
+    const float rs = fabsf(fx) + fabsf(fy) + fabsf(off), ds = fabsf(dx) + fabsf(dy);
+    const float en = 1e-6f * rs, ed = 8e-6f * ds, margin = 4e-6f * rs * ds;
+    float num[3], nd[3], bnum = 1.0f, bnd = 0.0f;
+    int nf = -1;
+#pragma unroll
+    for (int f = 0; f < 3; f++) {
+      num[f] = (f == 1 ? off : 0.0f) - (n[f][0] * fx + n[f][1] * fy);
+      nd[f] = n[f][0] * dx + n[f][1] * dy;
+      const bool better = f != curface && nd[f] > ed && num[f] * bnd < bnum * nd[f];
+      bnum = better ? num[f] : bnum;
+      bnd = better ? nd[f] : bnd;
+      nf = better ? f : nf;
+    }
+    bool sure = nf >= 0 && bnum > en;
+#pragma unroll
+    for (int f = 0; f < 3; f++)
+      sure = sure && (f == nf || (num[f] * bnd - bnum * nd[f] > margin && (f == curface || num[f] > en)));
+    if (sure) {
+      const double *m = T->n[nf];
+      const double m0 = __ldg(m), m1 = __ldg(m + 1);
+      dist = fast_div((nf == 1 ? offd : 0.0) - fma(m1, ry, m0 * rx), fma(m1, dir[1], m0 * dir[0]));
+      return nf;
+    }
+    const Exit e = which_face(verts(J) + el, pos[0], pos[1], dir[0], dir[1], curface);
+    dist = e.dist;
+    return e.nf;
+  }
+
+  __device__ __forceinline__ bool step(const JobDev &J, R &rng, int32_t cap, uint32_t &n_scat) {
+    if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
+    double dist;
+    int4 nb;
+    const int nf = exit_face(J, dist, nb);
+    if (nf < 0) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
+      return die(J, kEvLost);
+    }
+    nsteps++;
+    // both lengths are positive, so their bits compare as they do (a NaN path never ends here)
+    const bool ends = __double_as_longlong(prop) <= __double_as_longlong(dist);
+    const double ds = ends ? prop : dist;
+    pos[0] = fma(dir[0], ds, pos[0]);
+    pos[1] = fma(dir[1], ds, pos[1]);
+    tr.put(el);
+    if (!FD) {
+      if (mua > 0.0) {
+        const double dep = absorbed_part(mua, ds) * w;
+        acc += dep;
+        w -= dep;
+      } else {
+        acc = fma(w, ds, acc);
+        if (mua != 0.0) w *= exp(-mua * ds);
+      }
+    } else {
+      const double att = mua > 0.0 ? 1.0 - absorbed_part(mua, ds) : exp(-mua * ds);
+      turn += fixed_of_double(J.k_turn * nidx * ds);
+      double sn, cn;
+      sincos_turn(turn, sn, cn);
+      acc = fma(w, fma(-cn, att, cph), acc);
+      accI = fma(w, fma(sn, att, -sph), accI);
+      cph = cn; sph = sn;
+      w *= att;
+    }
+    bool on = true;
+    if (ends) {
+      if (mus > 0.0) {
+        const uint3 u = rng.peek3();
+        scatter(u.x);
+        rng.take(2);
+        prop = neg_log_open(u.y) * imus;
+        n_scat++;
+      } else {
+        rng.align();
+        prop = neg_log_open(rng.next()) * imus;
+      }
+    } else {
+      prop -= dist;
+      const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nb.z;
+      on = cross(J, rng, nf, nextel);
+    }
+    if (on && nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
+      job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
+      return die(J, kEvCapped);
+    }
+    return on;
+  }
+
+  // the boundary, or the next element, behind edge nf
+  __device__ __forceinline__ bool cross(const JobDev &J, R &rng, int nf, int nextel) {
+    if (nextel >= J.Ne) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
+      return die(J, kEvLost);
+    }
+    const bool inside = nextel >= 0;
+    const int ib = -1 - nextel;
+    double mua2 = 0.0, mus2 = 0.0, g2 = 0.0, n2;
+    if (inside) {
+      optics(J, nextel, mua2, mus2, g2, n2);
+    } else {
+      if (is_mirror(__ldg(J.bctype + ib))) {
+        const double *bn = J.bnorm + 4 * (int64_t)ib;
+        const double cdot = bn[0] * dir[0] + bn[1] * dir[1];
+        dir[0] -= 2.0 * cdot * bn[0];
+        dir[1] -= 2.0 * cdot * bn[1];
+        curface = nf;
+        return true;
+      }
+      n2 = __ldg(J.bcn + ib);
+    }
+    const bool vacuum = inside && mus <= 0.0 && mus2 > 0.0;
+    const bool jump = inside ? nidx != n2 : n2 > 0.0;
+    if (!inside || vacuum || jump || w < kWeight0) {
+      const double *m = (recs(J) + el)->n[nf];
+      double n0 = __ldg(m), n1 = __ldg(m + 1);  // outward
+      double len, inv;
+      fast_sqrt(fma(n0, n0, n1 * n1), len, inv);
+      n0 *= inv; n1 *= inv;
+      rng.reload();
+      if (vacuum) prop = neg_log_open(rng.next()) / mus2;
+      if (inside && w < kWeight0) {
+        if (unif_closed(rng) > kChance) {
+          job_count(J, kJcRoulette); job_ledger(J, kLgRouletteKill, w);
+          return die(J, kEvRoulette);
+        }
+        job_ledger(J, kLgRouletteGain, w / kChance - w);
+        w /= kChance;
+      }
+      if (jump && fresnel(rng, n0, n1, fast_div(nidx, n2), nf, !inside)) return true;
+      if (!inside) {
+        const double idn = fast_rcp(dir[0] * n0 + dir[1] * n1);  // DEBR, MC2D.hpp:1410-1437
+        flush(J);
+        if (!FD) {
+          add_d(J, J.EBR + ib, w);
+          add_d(J, J.DEBR + ib, w * idn);
+        } else {
+          const double re = w * cph, im = -(w * sph);
+          add_d(J, J.EBR + ib, re);
+          add_d(J, J.EBI + ib, im);
+          add_d(J, J.DEBR + ib, re * idn);
+          add_d(J, J.DEBI + ib, im * idn);
+        }
+        tr.put(-1 - (int64_t)ib);
+        tr.end();
+        return false;
+      }
+    }
+    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((recs(J) + nextel)->nbr));
+    const int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : -1;
+    if (mus2 != mus) {
+      if (!vacuum) prop *= mus / mus2;  // x (mus / mus) == x
+      imus = fast_rcp(mus2);
+    }
+    if (f2 < 0) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
+      return die(J, kEvLost);
+    }
+    if (g2 != g) kg = turn_factor(g2);
+    flush(J);
+    curface = f2;
+    el = nextel;
+    mua = mua2; mus = mus2; g = g2; nidx = n2;
+    return true;
+  }
+};
+
+// the reference's operation sequence, for the jobs that need it (as Walk3D64L)
+template <bool FD, class R>
+struct Walk2D64L {
   static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = false;
@@ -50,6 +352,9 @@ struct Walk2D64 {
     else f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, acc, el, curface, nsteps);
   }
 
+  __device__ __forceinline__ static const Tri64 *tris(const JobDev &J) {
+    return reinterpret_cast<const Tri64 *>(reinterpret_cast<const TriRec *>(J.geom) + J.Ne);
+  }
   __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
     const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
     const double2 o0 = __ldg(o), o1 = __ldg(o + 1);
@@ -112,7 +417,7 @@ struct Walk2D64 {
   __device__ bool fresnel(R &rng, const double nor[2], double nipnt, int nf, bool boundary) {
     double costhi = -(dir[0] * nor[0] + dir[1] * nor[1]);
     double costht = 0.0;
-    if (fresnel_reflects_d(rng, nipnt, costhi, costht)) {
+    if (fresnel_reflects_angles(rng, nipnt, costhi, costht)) {
       dir[0] += 2.0 * costhi * nor[0];
       dir[1] += 2.0 * costhi * nor[1];
       curface = nf;
@@ -162,7 +467,7 @@ struct Walk2D64 {
       die(J, kEvCapped);
       return kDiedEarly;
     }
-    const Tri64 *T = reinterpret_cast<const Tri64 *>(J.geom) + el;
+    const Tri64 *T = tris(J) + el;
     double V[3][2];
     {
       const double2 *src = reinterpret_cast<const double2 *>(T->v);
@@ -268,7 +573,7 @@ struct Walk2D64 {
       }
       if (mus2 != mus) prop *= mus / mus2;  // x (mus / mus) == x: skip the division
     }
-    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((reinterpret_cast<const Tri64 *>(J.geom) + nextel)->nbr));
+    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((tris(J) + nextel)->nbr));
     int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : -1;
     if (f2 < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);

@@ -1,12 +1,11 @@
 // walk3d.cuh -- the tetrahedral photon walk, one element step per call.
 //
-// Walk3D64: plain form.  Follows PropagatePhoton (cpp/3d/MC3D.hpp:1450-1638) with the
-//   reference's FP64 arithmetic: Moller-Trumbore exit test over the faces in order,
-//   skipping the entry face (WhichFace :1006-1057), Henyey-Greenstein ScatterPhoton
-//   (:1297-1340; the polar cosine used as drawn, without acos / cos), FresnelPhoton with
-//   the face normal from the vertices (:1365-1447),
-//   MirrorPhoton (:1343-1351), roulette and the reverse-face lookup (:1573-1631).  Draw
-//   order is the reference's, so a tape replay visits the same elements.
+// Walk3D64: plain form.  Follows PropagatePhoton (cpp/3d/MC3D.hpp:1450-1638) with the state
+//   in FP64: the exit face that the reference's Moller-Trumbore test over the faces in order,
+//   skipping the entry face, finds (WhichFace :1006-1057), Henyey-Greenstein ScatterPhoton
+//   (:1297-1340; the polar cosine used as drawn, without acos / cos), FresnelPhoton
+//   (:1365-1447), MirrorPhoton (:1343-1351), roulette and the reverse-face lookup
+//   (:1573-1631).  Draw order is the reference's, so a tape replay visits the same elements.
 // Walk3D32: tracking form.  Position, direction and weight in FP32; the exit face is the
 //   nearest of the faces the direction points out of, from precomputed outward planes
 //   (the barycentric coordinate of the opposite vertex reaching zero), with the distance
@@ -41,9 +40,28 @@ __device__ __forceinline__ bool ray_tri(const double O[3], const double D[3], co
 }
 
 // Fresnel reflect-or-transmit decision in FP64 (cpp/3d/MC3D.hpp:1397-1430).  Returns true
-// when reflected.  costht is the transmitted cosine when false is returned.
+// when reflected.  costht is the transmitted cosine when false is returned.  R from the closed
+// forms rs = (eta ci - ct) / (eta ci + ct), rp = (ci - eta ct) / (ci + eta ct) over one division:
+// the reference's R = (sin^2(thi - tht) / sin^2(thi + tht) + tan^2 / tan^2) / 2 to a few ulps,
+// without its seven angles and their functions.
 template <class R>
 __device__ __forceinline__ bool fresnel_reflects_d(R &rng, double nipnt, double costhi, double &costht) {
+  const double s = 1.0 - nipnt * nipnt * (1.0 - costhi * costhi);
+  if (s <= 0.0) return true;
+  costht = fast_sqrt(s);
+  const double ci = fabs(costhi);
+  const double u = unif_closed(rng);
+  if (!(ci <= 1.0)) return false;  // acos is NaN there in the reference, and so is R
+  const double a = fma(nipnt, ci, -costht), b = fma(nipnt, ci, costht);
+  const double c = fma(-nipnt, costht, ci), d = fma(nipnt, costht, ci);
+  const double q = b * d, rs = a * d, rp = c * b;
+  return u <= 0.5 * fast_div(fma(rs, rs, rp * rp), q * q);
+}
+
+// The same in the reference's angles, for the literal walks (cpp/3d/MC3D.hpp:1397-1430).  Returns true
+// when reflected.  costht is the transmitted cosine when false is returned.
+template <class R>
+__device__ __forceinline__ bool fresnel_reflects_angles(R &rng, double nipnt, double costhi, double &costht) {
   double s = 1.0 - nipnt * nipnt * (1.0 - costhi * costhi);
   if (s <= 0.0) return true;
   costht = sqrt(s);
@@ -117,8 +135,335 @@ __device__ __forceinline__ float free_path_f(float u, float mus) {
 // =====================================================================================
 // plain FP64 form
 // =====================================================================================
+// Bound by the FP64 pipe, which starts one warp instruction in about 19 cycles of the SM; with
+// the reference's operation sequence taken literally a warp's step needed about 450 of them
+// (Moller-Trumbore face by face, the library's exp, log, sin, cos, sqrt and divisions).  Here
+// FP64 is spent where the state is: about 25 operations for the step and 45 for a scatter.
+//   exit face  picked in FP32 from planes about vertex 0, when it is certain by margins above
+//              every FP32 rounding; else (2e-4 of the steps) by Moller-Trumbore, face by face as
+//              in the reference.  Its distance is one FP64 quotient n . (v - p) / n . d, with no
+//              more rounding than Moller-Trumbore's.
+//   samples    log, sine, cosine and the deposit's factor on the integer pipe (fixed64.hpp).
+//   quotients and roots from FP32 first values.
+// 1e5 photons on the phantom 313 -> 102 ms (571 before lanes were packed as well), 1e6 on the 2D
+// square 38.7 -> 9.0 ms, a 2304-tet frequency-domain box 19.5 -> 7.7 ms.  The square keeps the FP64
+// pipe 74 % busy; the phantom's run ends in walks of 12 000 steps, 4 us each.
 template <bool FD, class R>
 struct Walk3D64 {
+  static constexpr bool kBuffered = false;  // words left in a block are carried from step to step
+  static constexpr bool kPack = true;
+  static constexpr bool kCap32 = true;
+  static constexpr int kMinBlocks = 2;
+  static constexpr bool kStaged = false;
+  static constexpr bool kLaunchLoss = false;
+  Stage stage;
+  using Tr = typename TraceFor<R>::type;
+  double pos[3], dir[3];
+  double w, prop, cph, sph;
+  double mua, mus, g, nidx, imus, ig;  // imus = 1 / mus, ig = 1 / (2 g)
+  double acc, accI;
+  uint64_t turn;  // phase in 2^-64 turns
+  int el, curface;
+  int32_t nsteps;
+  Tr tr;
+
+  // moves the photon's state between lanes (Packer)
+  template <class F> __device__ __forceinline__ void move(const F &f) {
+    if constexpr (FD) f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, imus, ig, acc, turn, cph, sph, accI, el, curface, nsteps);
+    else f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, imus, ig, acc, el, curface, nsteps);
+  }
+
+  __device__ __forceinline__ static const TetRec *recs(const JobDev &J) { return reinterpret_cast<const TetRec *>(J.geom); }
+  __device__ __forceinline__ static const Tet64 *verts(const JobDev &J) { return reinterpret_cast<const Tet64 *>(recs(J) + J.Ne); }
+
+  __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
+    const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
+    const double2 o0 = __ldg(o), o1 = __ldg(o + 1);
+    a = o0.x; s = o0.y; gg = o1.x; nn = o1.y;
+  }
+
+  __device__ void launch(const JobDev &J, R &rng, int64_t q) {
+    tr.begin(J, q);
+    create_photon_3d(J, rng, pos, dir, el, curface);
+    w = 1.0;
+    if (FD) {
+      turn = J.turn0;
+      sincos_turn(turn, sph, cph);
+    }
+    optics(J, el, mua, mus, g, nidx);
+    imus = fast_rcp(mus);
+    ig = 0.5 * fast_rcp(g);
+    prop = neg_log_open(rng.next()) * imus;  // the outer loop's first draw, MC3D.hpp:1458
+    acc = accI = 0.0;
+    nsteps = 0;
+  }
+
+  __device__ __forceinline__ void flush(const JobDev &J) {
+    add_d(J, J.ER + el, acc);
+    if (FD) add_d(J, J.EI + el, accI);
+    acc = accI = 0.0;
+  }
+
+  __device__ __forceinline__ bool die(const JobDev &J, int64_t ev) {
+    flush(J);
+    tr.put(ev);
+    tr.end();
+    return false;
+  }
+
+  // ScatterPhoton, MC3D.hpp:1297-1340, from the words u, without the round trip through the
+  // angle: the reference draws theta = acos(c) from the HG inverse CDF c and takes sin and cos
+  // of it; here cos theta is c itself and sin theta = sqrt(1 - c^2) (|c| > 1 from rounding at
+  // the CDF's ends gives a NaN sine, as acos gives a NaN angle).
+  __device__ __forceinline__ void scatter(uint2 u) {
+    const double xi = word_d(u.x) * (1.0 / 4294967295.0);
+    double ct = fma(2.0, xi, -1.0);  // isotropic
+    if (g != 0.0) {
+      const double D = fma(g, ct, 1.0);  // 1 - g (1 - 2 xi)
+      const double q = fast_div(fma(-g, g, 1.0), D);
+      ct = fma(-q, q, fma(g, g, 1.0)) * ig;
+      if (u.x == 0u || u.x == 0xffffffffu) ct = u.x ? 1.0 : -1.0;  // theta = (1 - xi) pi at xi in {0, 1}
+    }
+    const double s2 = fma(-ct, ct, 1.0);
+    const double st = s2 > 0.0 ? fast_sqrt(s2) : sqrt(s2);
+    // the azimuth 2 pi u / (2^32 - 1): u 2^32 + u in 2^-64 turns, to one of them
+    double sp, cp;
+    sincos_turn(((uint64_t)u.y << 32) | u.y, sp, cp);
+    const double dx = dir[0], dy = dir[1], dz = dir[2];
+    double nx, ny, nz;
+    if (fabsf(f32_of(dz)) > 0.9989f && fabs(dz) > 0.999) {
+      nx = st * cp;
+      ny = st * sp;
+      nz = dz > 0.0 ? ct : -ct;
+    } else {
+      double sq, isq;
+      fast_sqrt(fma(-dz, dz, 1.0), sq, isq);
+      const double a = st * isq, zc = dz * cp;
+      nx = fma(a, fma(dx, zc, -(dy * sp)), dx * ct);
+      ny = fma(a, fma(dy, zc, dx * sp), dy * ct);
+      nz = fma(-st * cp, sq, dz * ct);
+    }
+    const double s = unit_scale(fma(nx, nx, fma(ny, ny, nz * nz)));
+    dir[0] = nx * s; dir[1] = ny * s; dir[2] = nz * s;
+    curface = -1;
+  }
+
+  // FresnelPhoton at a face with normal nor, of either orientation and any length
+  // (MC3D.hpp:1365-1447); true if reflected
+  __device__ __forceinline__ bool fresnel(R &rng, const double *nor, double nipnt, int nf) {
+    double n0 = __ldg(nor), n1 = __ldg(nor + 1), n2 = __ldg(nor + 2);
+    double len, inv;
+    fast_sqrt(fma(n0, n0, fma(n1, n1, n2 * n2)), len, inv);
+    n0 *= inv; n1 *= inv; n2 *= inv;
+    const double costhi = -(dir[0] * n0 + dir[1] * n1 + dir[2] * n2);
+    double costht = 0.0;
+    if (fresnel_reflects_d(rng, nipnt, costhi, costht)) {
+      const double k = 2.0 * costhi;
+      dir[0] = fma(k, n0, dir[0]); dir[1] = fma(k, n1, dir[1]); dir[2] = fma(k, n2, dir[2]);
+      curface = nf;
+      return true;
+    }
+    const double m = (costhi > 0.0) ? (nipnt * costhi - costht) : (nipnt * costhi + costht);
+    dir[0] = fma(nipnt, dir[0], m * n0); dir[1] = fma(nipnt, dir[1], m * n1); dir[2] = fma(nipnt, dir[2], m * n2);
+    return false;
+  }
+
+  // WhichFace, MC3D.hpp:1006-1057: faces (0,1,2), (0,1,3), (0,2,3), (1,2,3) in order, skipping curface
+  struct Exit { double dist; int nf; };
+  __device__ __noinline__ static Exit which_face(const Tet64 *T, double px, double py, double pz, double dx, double dy,
+                                                 double dz, int curface) {
+    const double *v = &T->v[0][0];
+    const double pos[3] = {px, py, pz}, dir[3] = {dx, dy, dz};
+    double dist = 0.0;
+    if (curface != 0 && ray_tri(pos, dir, v, v + 3, v + 6, dist) && dist > 0.0) return Exit{dist, 0};
+    if (curface != 1 && ray_tri(pos, dir, v, v + 3, v + 9, dist) && dist > 0.0) return Exit{dist, 1};
+    if (curface != 2 && ray_tri(pos, dir, v, v + 6, v + 9, dist) && dist > 0.0) return Exit{dist, 2};
+    if (curface != 3 && ray_tri(pos, dir, v + 3, v + 6, v + 9, dist) && dist > 0.0) return Exit{dist, 3};
+    return Exit{0.0, -1};
+  }
+
+  // The exit face and the distance to it; nbr: the record's neighbours.
+  //
+  // With r = p - v0 in FP64, FP32 has num_f = off_f - n_f . r (the distance to plane f) within
+  // en = 1e-6 |r|_1 (5e-7 from the roundings of n, r and the sum) and nd_f = n_f . d within
+  // ed = 1e-6 |d|_1.  The face that the ray leaves through is certain when num > en and
+  // nd > 8 ed there, every other face's plane is met later by a margin, num_g nd - num nd_g >
+  // 4e-6 |r|_1 |d|_1, and the ray starts clearly inside every other plane but the one it
+  // entered by (which the reference does not test): then Moller-Trumbore finds u and v well
+  // inside that face, and well outside the others or behind the photon.
+  __device__ __forceinline__ int exit_face(const JobDev &J, double &dist, int4 &nbr) const {
+    const TetRec *T = recs(J) + el;
+    const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
+    const double2 a1 = __ldg(reinterpret_cast<const double2 *>(T->v0) + 1);
+    const float4 q0 = __ldg(reinterpret_cast<const float4 *>(T->nf)), q1 = __ldg(reinterpret_cast<const float4 *>(T->nf) + 1),
+                 q2 = __ldg(reinterpret_cast<const float4 *>(T->nf) + 2);
+    nbr = __ldg(reinterpret_cast<const int4 *>(T->nbr));
+    const double rx = pos[0] - a0.x, ry = pos[1] - a0.y, rz = pos[2] - a1.x;
+    const float fx = f32_of(rx), fy = f32_of(ry), fz = f32_of(rz), off = __ldg(&T->off_size);
+    const float dx = f32_of(dir[0]), dy = f32_of(dir[1]), dz = f32_of(dir[2]);
+    const float n[4][3] = {{q0.x, q0.y, q0.z}, {q0.w, q1.x, q1.y}, {q1.z, q1.w, q2.x}, {q2.y, q2.z, q2.w}};
+    const float rs = fabsf(fx) + fabsf(fy) + fabsf(fz) + fabsf(off), ds = fabsf(dx) + fabsf(dy) + fabsf(dz);
+    const float en = 1e-6f * rs, ed = 8e-6f * ds, margin = 4e-6f * rs * ds;
+    float num[4], nd[4], bnum = 1.0f, bnd = 0.0f;
+    int nf = -1;
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      num[f] = (f == 3 ? off : 0.0f) - (n[f][0] * fx + n[f][1] * fy + n[f][2] * fz);
+      nd[f] = n[f][0] * dx + n[f][1] * dy + n[f][2] * dz;
+      const bool better = f != curface && nd[f] > ed && num[f] * bnd < bnum * nd[f];
+      bnum = better ? num[f] : bnum;
+      bnd = better ? nd[f] : bnd;
+      nf = better ? f : nf;
+    }
+    bool sure = nf >= 0 && bnum > en;
+#pragma unroll
+    for (int f = 0; f < 4; f++)
+      sure = sure && (f == nf || (num[f] * bnd - bnum * nd[f] > margin && (f == curface || num[f] > en)));
+    if (sure) {
+      const double *m = T->n[nf];
+      const double m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2);
+      const double dn = fma(m2, dir[2], fma(m1, dir[1], m0 * dir[0]));
+      const double nr = fma(m2, rz, fma(m1, ry, m0 * rx));
+      dist = fast_div((nf == 3 ? a1.y : 0.0) - nr, dn);
+      return nf;
+    }
+    const Exit e = which_face(verts(J) + el, pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], curface);
+    dist = e.dist;
+    return e.nf;
+  }
+
+  __device__ __forceinline__ bool step(const JobDev &J, R &rng, int32_t cap, uint32_t &n_scat) {
+    if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
+    double dist;
+    int4 nb;
+    const int nf = exit_face(J, dist, nb);
+    if (nf < 0) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
+      return die(J, kEvLost);
+    }
+    nsteps++;
+    // both lengths are positive, so their bits compare as they do (a NaN path never ends here)
+    const bool ends = __double_as_longlong(prop) <= __double_as_longlong(dist);
+    const double ds = ends ? prop : dist;
+#pragma unroll
+    for (int c = 0; c < 3; c++) pos[c] = fma(dir[c], ds, pos[c]);
+    tr.put(el);
+    // element fluence, MC3D.hpp:1479-1526
+    if (!FD) {
+      if (mua > 0.0) {
+        const double dep = absorbed_part(mua, ds) * w;
+        acc += dep;
+        w -= dep;
+      } else {
+        acc = fma(w, ds, acc);
+        if (mua != 0.0) w *= exp(-mua * ds);
+      }
+    } else {
+      const double att = mua > 0.0 ? 1.0 - absorbed_part(mua, ds) : exp(-mua * ds);
+      turn += fixed_of_double(J.k_turn * nidx * ds);
+      double sn, cn;
+      sincos_turn(turn, sn, cn);
+      acc = fma(w, fma(-cn, att, cph), acc);
+      accI = fma(w, fma(sn, att, -sph), accI);
+      cph = cn; sph = sn;
+      w *= att;
+    }
+    bool on = true;
+    if (ends) {
+      if (mus > 0.0) {
+        const uint3 u = rng.peek3();
+        scatter(make_uint2(u.x, u.y));
+        rng.take(3);
+        prop = neg_log_open(u.z) * imus;
+        n_scat++;
+      } else {
+        rng.align();
+        prop = neg_log_open(rng.next()) * imus;
+      }
+    } else {
+      prop -= dist;
+      const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nf == 2 ? nb.z : nb.w;
+      on = cross(J, rng, nf, nextel);
+    }
+    if (on && nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
+      job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
+      return die(J, kEvCapped);
+    }
+    return on;
+  }
+
+  // the boundary, or the next element, behind face nf
+  __device__ __forceinline__ bool cross(const JobDev &J, R &rng, int nf, int nextel) {
+    const double *nor = (recs(J) + el)->n[nf];
+    if (nextel >= J.Ne) {  // open face: the reference would index past its arrays here
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
+      return die(J, kEvLost);
+    }
+    const bool inside = nextel >= 0;
+    const int ib = -1 - nextel;
+    double mua2 = 0.0, mus2 = 0.0, g2 = 0.0, n2;
+    if (inside) {
+      optics(J, nextel, mua2, mus2, g2, n2);
+    } else {
+      if (is_mirror(__ldg(J.bctype + ib))) {  // MirrorPhoton(ib) with Normal(ib)
+        const double *bn = J.bnorm + 4 * (int64_t)ib;
+        const double cdot = bn[0] * dir[0] + bn[1] * dir[1] + bn[2] * dir[2];
+#pragma unroll
+        for (int c = 0; c < 3; c++) dir[c] -= 2.0 * cdot * bn[c];
+        curface = nf;
+        return true;
+      }
+      n2 = __ldg(J.bcn + ib);
+    }
+    const bool vacuum = inside && mus <= 0.0 && mus2 > 0.0;
+    const bool jump = inside ? nidx != n2 : n2 > 0.0;
+    if (vacuum || jump || (inside && w < kWeight0)) {
+      rng.reload();
+      if (vacuum) prop = neg_log_open(rng.next()) / mus2;
+      if (inside && w < kWeight0) {
+        if (unif_closed(rng) > kChance) {
+          job_count(J, kJcRoulette); job_ledger(J, kLgRouletteKill, w);
+          return die(J, kEvRoulette);
+        }
+        job_ledger(J, kLgRouletteGain, w / kChance - w);
+        w /= kChance;
+      }
+      if (jump && fresnel(rng, nor, nidx / n2, nf)) return true;
+    }
+    if (!inside) {
+      flush(J);
+      if (!FD) add_d(J, J.EBR + ib, w);
+      else { add_d(J, J.EBR + ib, w * cph); add_d(J, J.EBI + ib, -(w * sph)); }
+      tr.put(-1 - (int64_t)ib);
+      tr.end();
+      return false;
+    }
+    // reverse-face lookup, MC3D.hpp:1616-1628
+    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((recs(J) + nextel)->nbr));
+    const int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : nb2.w == el ? 3 : -1;
+    if (mus2 != mus) {
+      if (!vacuum) prop *= mus / mus2;  // x (mus / mus) == x
+      imus = fast_rcp(mus2);
+    }
+    if (f2 < 0) {
+      job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
+      return die(J, kEvLost);
+    }
+    if (g2 != g) ig = 0.5 * fast_rcp(g2);
+    flush(J);
+    curface = f2;
+    el = nextel;
+    mua = mua2; mus = mus2; g = g2; nidx = n2;
+    return true;
+  }
+};
+
+// The plain form with the reference's operation sequence taken literally, for jobs whose
+// scattering or index changes across most faces (rough_optics): there a photon's remaining path
+// is rescaled at nearly every crossing, rounding differences grow from crossing to crossing, and
+// walks of thousands of steps keep the reference's steps only with the reference's operations.
+template <bool FD, class R>
+struct Walk3D64L {
   static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = false;
@@ -141,6 +486,9 @@ struct Walk3D64 {
     else f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, acc, el, curface, nsteps);
   }
 
+  __device__ __forceinline__ static const Tet64 *tets(const JobDev &J) {
+    return reinterpret_cast<const Tet64 *>(reinterpret_cast<const TetRec *>(J.geom) + J.Ne);
+  }
   __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
     const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
     const double2 o0 = __ldg(o), o1 = __ldg(o + 1);
@@ -219,7 +567,7 @@ struct Walk3D64 {
   __device__ bool fresnel(R &rng, const double nor[3], double nipnt, int nf) {
     double costhi = -(dir[0] * nor[0] + dir[1] * nor[1] + dir[2] * nor[2]);
     double costht = 0.0;
-    if (fresnel_reflects_d(rng, nipnt, costhi, costht)) {
+    if (fresnel_reflects_angles(rng, nipnt, costhi, costht)) {
 #pragma unroll
       for (int c = 0; c < 3; c++) dir[c] += 2.0 * costhi * nor[c];
       curface = nf;
@@ -238,7 +586,7 @@ struct Walk3D64 {
       die(J, kEvCapped);
       return kDiedEarly;
     }
-    const Tet64 *T = reinterpret_cast<const Tet64 *>(J.geom) + el;
+    const Tet64 *T = tets(J) + el;
     double V[4][3];
     {
       const double2 *src = reinterpret_cast<const double2 *>(T->v);
@@ -353,7 +701,7 @@ struct Walk3D64 {
       if (mus2 != mus) prop *= mus / mus2;  // x (mus / mus) == x: skip the division
     }
     // reverse-face lookup, MC3D.hpp:1616-1628
-    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((reinterpret_cast<const Tet64 *>(J.geom) + nextel)->nbr));
+    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((tets(J) + nextel)->nbr));
     int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : nb2.w == el ? 3 : -1;
     if (f2 < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);

@@ -5,6 +5,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "fixed64.hpp"
 #include "rng.cuh"
 #include "vmc_types.hpp"
 
@@ -344,6 +345,73 @@ __device__ __forceinline__ void create_photon_2d_f(const JobDev &J, R &rng, floa
       if (dt == 'n' || n0 * dir[0] + n1 * dir[1] > 0.0f || rng.exhausted()) break;
     }
   }
+}
+
+// ---- FP64 arithmetic of the plain forms, around the slow FP64 pipe ----
+
+// x rounded toward zero to FP32 on the integer pipe; 0 below FP32's normal range, NaN above it
+// and for a NaN
+__device__ __forceinline__ float f32_of(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t t = hi & 0x7fffffffu;
+  uint32_t f = __funnelshift_l(lo, t, 3) + 0x40000000u;  // exponent rebased by 1023 - 127 = 896
+  f = t < 0x38100000u ? 0u : t >= 0x47f00000u ? 0x7fc00000u : f;
+  return __uint_as_float(f | (hi & 0x80000000u));
+}
+
+// 1 / b, a / b, sqrt(s) and 1 / sqrt(s) from an FP32 first value and Newton's step of second
+// and third order: 3 to 5 FP64 operations, to an ulp or two.  Outside the range where FP32
+// holds the first value the library's function takes over.
+__device__ __forceinline__ bool f32_safe(float f) { return fabsf(f) > 1e-30f && fabsf(f) < 1e30f; }
+
+__device__ __forceinline__ double fast_rcp(double b) {
+  const float bf = f32_of(b);
+  if (!f32_safe(bf)) return 1.0 / b;
+  const double y = f2d_int(__frcp_rn(bf));
+  const double e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double fast_div(double a, double b) {
+  const float bf = f32_of(b);
+  if (!f32_safe(bf)) return a / b;
+  double y = f2d_int(__frcp_rn(bf));
+  y = fma(y, fma(-b, y, 1.0), y);
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+// sqrt(s) in r, 1 / sqrt(s) in y
+__device__ __forceinline__ void fast_sqrt(double s, double &r, double &y) {
+  const float sf = f32_of(s);
+  if (!(sf > 1e-30f && sf < 1e30f)) {
+    r = sqrt(s);
+    y = 1.0 / r;
+    return;
+  }
+  const double y0 = f2d_int(rsqrtf(sf));
+  const double h = s * y0;
+  const double e = fma(-h, y0, 1.0);
+  const double p = e * fma(e, 0.375, 0.5);
+  r = fma(h, p, h);
+  y = fma(y0, p, y0);
+}
+__device__ __forceinline__ double fast_sqrt(double s) {
+  double r, y;
+  fast_sqrt(s, r, y);
+  return r;
+}
+// 1 / sqrt(n2) of a squared length that is nearly 1 (directions)
+__device__ __forceinline__ double unit_scale(double n2) {
+  const double d = n2 - 1.0;
+  if (fabsf(f32_of(d)) < 9.5e-7f) return fma(d, fma(d, 0.375, -0.5), 1.0);  // d^3 5/16 < 2^-61
+  return 1.0 / sqrt(n2);
+}
+// the word as a double, exactly, with one FP64 operation
+__device__ __forceinline__ double word_d(uint32_t w) { return __hiloint2double(0x43300000, (int)w) - 4503599627370496.0; }
+
+// w (1 - exp(-mua ds)) and the weight left of an absorbing step (mua > 0)
+__device__ __forceinline__ double absorbed_part(double mua, double ds) {
+  const double x = mua * ds;
+  return f32_of(x) < 0.0625f ? x * one_minus_exp_over_x(x) : -expm1(-x);
 }
 
 }  // namespace vmc
