@@ -96,27 +96,41 @@ struct Walk2D64 {
     return false;
   }
 
+  // What a scatter event draws: cosine and sine of the turn, the free path after it.
+  struct Event { double c, s, path; };
+
   // ScatterPhoton (MC2D.hpp:1135-1155) turns the direction to atan2(dir) + 2 atan(h), h =
   // tan(pi xi) (1 - g) / (1 + g).  Here the direction is turned by 2 atan(h): with (s0, c0) the
   // sine and cosine of pi xi and ks = (1 - g) / (1 + g) s0, its cosine is
   // (c0^2 - ks^2) / (c0^2 + ks^2) and its sine 2 ks c0 / (c0^2 + ks^2) -- no angle is formed.
-  __device__ __forceinline__ void scatter(uint32_t u) {
-    double c, s;
-    if (g != 0.0) {
-      double s0, c0;
-      sincos_turn((uint64_t)u << 31, s0, c0);
-      const double ks = kg * s0;
-      const double a = c0 * c0, b = ks * ks;
-      const double inv = fast_rcp(a + b) * unit_scale(fma(dir[0], dir[0], dir[1] * dir[1]));
-      c = (a - b) * inv;
-      s = 2.0 * ks * c0 * inv;
-      const double ux = dir[0], uy = dir[1];
+  // Drawn before the exit edge is looked for, as in the tetrahedral walk.
+  __device__ __forceinline__ Event draw_event(uint3 u) const {
+    Event e;
+    const bool iso = (__double_as_longlong(g) << 1) == 0;  // then the turn is 2 pi xi itself
+    double s0, c0;
+    sincos_turn((uint64_t)u.x << (iso ? 32 : 31), s0, c0);
+    const double ks = kg * s0;
+    const double a = c0 * c0, b = ks * ks;
+    const double den = a + b;
+    const double y0 = f2d_int(__frcp_rn(f32_of(den)));
+    const double r = fma(-den, y0, 1.0);
+    const double inv = fma(y0, fma(r, r, r), y0);
+    const double k2 = ks * c0;
+    e.c = iso ? c0 : (a - b) * inv;
+    e.s = iso ? s0 : (k2 + k2) * inv;
+    e.path = neg_log_open(u.y) * imus;
+    return e;
+  }
+
+  __device__ __forceinline__ void rotate(const Event &e) {
+    if ((__double_as_longlong(g) << 1) == 0) {  // the drawn direction, whatever the old one
+      dir[0] = e.c;
+      dir[1] = e.s;
+    } else {
+      const double k = unit_scale(fma(dir[0], dir[0], dir[1] * dir[1]));
+      const double c = e.c * k, s = e.s * k, ux = dir[0], uy = dir[1];
       dir[0] = fma(ux, c, -(uy * s));
       dir[1] = fma(uy, c, ux * s);
-    } else {
-      sincos_turn((uint64_t)u << 32, s, c);
-      dir[0] = c;
-      dir[1] = s;
     }
     curface = -1;
   }
@@ -151,7 +165,7 @@ struct Walk2D64 {
   }
 
   // the exit edge and the distance to it, as in the tetrahedral walk
-  __device__ __forceinline__ int exit_face(const JobDev &J, double &dist, int4 &nbr) const {
+  __device__ __forceinline__ int exit_face(const JobDev &J, R &rng, double &dist, int4 &nbr, Event &ev) const {
     const TriRec *T = recs(J) + el;
     const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
     const double offd = __ldg(&T->off);
@@ -179,12 +193,13 @@ struct Walk2D64 {
 #pragma unroll
     for (int f = 0; f < 3; f++)
       sure = sure && (f == nf || (num[f] * bnd - bnum * nd[f] > margin && (f == curface || num[f] > en)));
-    if (sure) {
-      const double *m = T->n[nf];
-      const double m0 = __ldg(m), m1 = __ldg(m + 1);
-      dist = fast_div((nf == 1 ? offd : 0.0) - fma(m1, ry, m0 * rx), fma(m1, dir[1], m0 * dir[0]));
-      return nf;
-    }
+    const double *m = T->n[nf < 0 ? 0 : nf];
+    const double m0 = __ldg(m), m1 = __ldg(m + 1);
+    const double dn = fma(m1, dir[1], m0 * dir[0]);
+    const float dnf = f32_of(dn);
+    dist = div_near((nf == 1 ? offd : 0.0) - fma(m1, ry, m0 * rx), dn, dnf);
+    ev = draw_event(rng.peek3());
+    if (sure && f32_safe(dnf)) return nf;
     const Exit e = which_face(verts(J) + el, pos[0], pos[1], dir[0], dir[1], curface);
     dist = e.dist;
     return e.nf;
@@ -194,7 +209,8 @@ struct Walk2D64 {
     if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     double dist;
     int4 nb;
-    const int nf = exit_face(J, dist, nb);
+    Event ev;
+    const int nf = exit_face(J, rng, dist, nb, ev);
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
@@ -207,7 +223,7 @@ struct Walk2D64 {
     pos[1] = fma(dir[1], ds, pos[1]);
     tr.put(el);
     if (!FD) {
-      if (mua > 0.0) {
+      if (positive(mua)) {
         const double dep = absorbed_part(mua, ds) * w;
         acc += dep;
         w -= dep;
@@ -216,7 +232,7 @@ struct Walk2D64 {
         if (mua != 0.0) w *= exp(-mua * ds);
       }
     } else {
-      const double att = mua > 0.0 ? 1.0 - absorbed_part(mua, ds) : exp(-mua * ds);
+      const double att = positive(mua) ? 1.0 - absorbed_part(mua, ds) : exp(-mua * ds);
       turn += fixed_of_double(J.k_turn * nidx * ds);
       double sn, cn;
       sincos_turn(turn, sn, cn);
@@ -227,11 +243,10 @@ struct Walk2D64 {
     }
     bool on = true;
     if (ends) {
-      if (mus > 0.0) {
-        const uint3 u = rng.peek3();
-        scatter(u.x);
+      if (positive(mus)) {
+        rotate(ev);
         rng.take(2);
-        prop = neg_log_open(u.y) * imus;
+        prop = ev.path;
         n_scat++;
       } else {
         rng.align();
@@ -271,9 +286,10 @@ struct Walk2D64 {
       }
       n2 = __ldg(J.bcn + ib);
     }
-    const bool vacuum = inside && mus <= 0.0 && mus2 > 0.0;
-    const bool jump = inside ? nidx != n2 : n2 > 0.0;
-    if (!inside || vacuum || jump || w < kWeight0) {
+    const bool vacuum = inside && !positive(mus) && positive(mus2);
+    const bool jump = inside ? differ(nidx, n2) : positive(n2);
+    const bool light = inside && below(w, kWeight0);
+    if (!inside || vacuum || jump || light) {
       const double *m = (recs(J) + el)->n[nf];
       double n0 = __ldg(m), n1 = __ldg(m + 1);  // outward
       double len, inv;
@@ -281,8 +297,8 @@ struct Walk2D64 {
       n0 *= inv; n1 *= inv;
       rng.reload();
       if (vacuum) prop = neg_log_open(rng.next()) / mus2;
-      if (inside && w < kWeight0) {
-        if (unif_closed(rng) > kChance) {
+      if (light) {
+        if (!closed_at_most(rng, kChance)) {
           job_count(J, kJcRoulette); job_ledger(J, kLgRouletteKill, w);
           return die(J, kEvRoulette);
         }
@@ -310,7 +326,7 @@ struct Walk2D64 {
     }
     const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((recs(J) + nextel)->nbr));
     const int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : -1;
-    if (mus2 != mus) {
+    if (differ(mus2, mus)) {
       if (!vacuum) prop *= mus / mus2;  // x (mus / mus) == x
       imus = fast_rcp(mus2);
     }
@@ -318,7 +334,7 @@ struct Walk2D64 {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
     }
-    if (g2 != g) kg = turn_factor(g2);
+    if (differ(g2, g)) kg = turn_factor(g2);
     flush(J);
     curface = f2;
     el = nextel;

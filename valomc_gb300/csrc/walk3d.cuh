@@ -50,7 +50,7 @@ __device__ __forceinline__ bool fresnel_reflects_d(R &rng, double nipnt, double 
   if (s <= 0.0) return true;
   costht = fast_sqrt(s);
   const double ci = fabs(costhi);
-  const double u = unif_closed(rng);
+  const double u = word_d(rng.next()) * (1.0 / 4294967295.0);  // unif_closed
   if (!(ci <= 1.0)) return false;  // acos is NaN there in the reference, and so is R
   const double a = fma(nipnt, ci, -costht), b = fma(nipnt, ci, costht);
   const double c = fma(-nipnt, costht, ci), d = fma(nipnt, costht, ci);
@@ -211,24 +211,38 @@ struct Walk3D64 {
     return false;
   }
 
-  // ScatterPhoton, MC3D.hpp:1297-1340, from the words u, without the round trip through the
+  // What a scatter event draws: the polar cosine and sine, the azimuth's, the free path after it.
+  struct Event { double ct, st, cp, sp, path; };
+
+  // ScatterPhoton, MC3D.hpp:1297-1315, from the words u, without the round trip through the
   // angle: the reference draws theta = acos(c) from the HG inverse CDF c and takes sin and cos
   // of it; here cos theta is c itself and sin theta = sqrt(1 - c^2) (|c| > 1 from rounding at
-  // the CDF's ends gives a NaN sine, as acos gives a NaN angle).
-  __device__ __forceinline__ void scatter(uint2 u) {
-    const double xi = word_d(u.x) * (1.0 / 4294967295.0);
-    double ct = fma(2.0, xi, -1.0);  // isotropic
-    if (g != 0.0) {
-      const double D = fma(g, ct, 1.0);  // 1 - g (1 - 2 xi)
-      const double q = fast_div(fma(-g, g, 1.0), D);
-      ct = fma(-q, q, fma(g, g, 1.0)) * ig;
-      if (u.x == 0u || u.x == 0xffffffffu) ct = u.x ? 1.0 : -1.0;  // theta = (1 - xi) pi at xi in {0, 1}
-    }
+  // the CDF's ends gives a NaN sine, as acos gives a NaN angle).  Drawn before the exit face is
+  // looked for, whether the step ends in a scatter or not: nearly every step of a warp has one,
+  // and the two chains of FP64 operations, each waiting some 75 cycles a link, overlap.
+  __device__ __forceinline__ Event draw_event(uint3 u) const {
+    Event e;
+    const double c0 = fma(word_d(u.x), 2.0 / 4294967295.0, -1.0);  // 2 xi - 1, the isotropic cosine
+    const double D = fma(g, c0, 1.0);                              // 1 - g (1 - 2 xi)
+    const double q = div_near(fma(-g, g, 1.0), D, f32_of(D));
+    double ct = fma(-q, q, fma(g, g, 1.0)) * ig;
+    ct = u.x == 0u ? -1.0 : u.x == 0xffffffffu ? 1.0 : ct;  // theta = (1 - xi) pi at xi in {0, 1}
+    ct = (__double_as_longlong(g) << 1) == 0 ? c0 : ct;
+    e.ct = ct;
     const double s2 = fma(-ct, ct, 1.0);
-    const double st = s2 > 0.0 ? fast_sqrt(s2) : sqrt(s2);
+    const float s2f = f32_of(s2);
+    double y;
+    sqrt_near(s2, s2f, e.st, y);
+    e.st = s2f > 0.0f ? e.st : s2f == 0.0f ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
     // the azimuth 2 pi u / (2^32 - 1): u 2^32 + u in 2^-64 turns, to one of them
-    double sp, cp;
-    sincos_turn(((uint64_t)u.y << 32) | u.y, sp, cp);
+    sincos_turn(((uint64_t)u.y << 32) | u.y, e.sp, e.cp);
+    e.path = neg_log_open(u.z) * imus;
+    return e;
+  }
+
+  // the rotation of ScatterPhoton, MC3D.hpp:1316-1340
+  __device__ __forceinline__ void rotate(const Event &e) {
+    const double ct = e.ct, st = e.st, cp = e.cp, sp = e.sp;
     const double dx = dir[0], dy = dir[1], dz = dir[2];
     double nx, ny, nz;
     if (fabsf(f32_of(dz)) > 0.9989f && fabs(dz) > 0.999) {
@@ -237,7 +251,8 @@ struct Walk3D64 {
       nz = dz > 0.0 ? ct : -ct;
     } else {
       double sq, isq;
-      fast_sqrt(fma(-dz, dz, 1.0), sq, isq);
+      const double s2 = fma(-dz, dz, 1.0);
+      sqrt_near(s2, f32_of(s2), sq, isq);
       const double a = st * isq, zc = dz * cp;
       nx = fma(a, fma(dx, zc, -(dy * sp)), dx * ct);
       ny = fma(a, fma(dy, zc, dx * sp), dy * ct);
@@ -291,7 +306,7 @@ struct Walk3D64 {
   // 4e-6 |r|_1 |d|_1, and the ray starts clearly inside every other plane but the one it
   // entered by (which the reference does not test): then Moller-Trumbore finds u and v well
   // inside that face, and well outside the others or behind the photon.
-  __device__ __forceinline__ int exit_face(const JobDev &J, double &dist, int4 &nbr) const {
+  __device__ __forceinline__ int exit_face(const JobDev &J, R &rng, double &dist, int4 &nbr, Event &ev) const {
     const TetRec *T = recs(J) + el;
     const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
     const double2 a1 = __ldg(reinterpret_cast<const double2 *>(T->v0) + 1);
@@ -319,14 +334,14 @@ struct Walk3D64 {
 #pragma unroll
     for (int f = 0; f < 4; f++)
       sure = sure && (f == nf || (num[f] * bnd - bnum * nd[f] > margin && (f == curface || num[f] > en)));
-    if (sure) {
-      const double *m = T->n[nf];
-      const double m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2);
-      const double dn = fma(m2, dir[2], fma(m1, dir[1], m0 * dir[0]));
-      const double nr = fma(m2, rz, fma(m1, ry, m0 * rx));
-      dist = fast_div((nf == 3 ? a1.y : 0.0) - nr, dn);
-      return nf;
-    }
+    const double *m = T->n[nf < 0 ? 0 : nf];
+    const double m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2);
+    const double dn = fma(m2, dir[2], fma(m1, dir[1], m0 * dir[0]));
+    const double nr = fma(m2, rz, fma(m1, ry, m0 * rx));
+    const float dnf = f32_of(dn);
+    dist = div_near((nf == 3 ? a1.y : 0.0) - nr, dn, dnf);
+    ev = draw_event(rng.peek3());
+    if (sure && f32_safe(dnf)) return nf;
     const Exit e = which_face(verts(J) + el, pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], curface);
     dist = e.dist;
     return e.nf;
@@ -336,7 +351,8 @@ struct Walk3D64 {
     if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     double dist;
     int4 nb;
-    const int nf = exit_face(J, dist, nb);
+    Event ev;
+    const int nf = exit_face(J, rng, dist, nb, ev);
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
@@ -350,7 +366,7 @@ struct Walk3D64 {
     tr.put(el);
     // element fluence, MC3D.hpp:1479-1526
     if (!FD) {
-      if (mua > 0.0) {
+      if (positive(mua)) {
         const double dep = absorbed_part(mua, ds) * w;
         acc += dep;
         w -= dep;
@@ -359,7 +375,7 @@ struct Walk3D64 {
         if (mua != 0.0) w *= exp(-mua * ds);
       }
     } else {
-      const double att = mua > 0.0 ? 1.0 - absorbed_part(mua, ds) : exp(-mua * ds);
+      const double att = positive(mua) ? 1.0 - absorbed_part(mua, ds) : exp(-mua * ds);
       turn += fixed_of_double(J.k_turn * nidx * ds);
       double sn, cn;
       sincos_turn(turn, sn, cn);
@@ -370,11 +386,10 @@ struct Walk3D64 {
     }
     bool on = true;
     if (ends) {
-      if (mus > 0.0) {
-        const uint3 u = rng.peek3();
-        scatter(make_uint2(u.x, u.y));
+      if (positive(mus)) {
+        rotate(ev);
         rng.take(3);
-        prop = neg_log_open(u.z) * imus;
+        prop = ev.path;
         n_scat++;
       } else {
         rng.align();
@@ -415,13 +430,14 @@ struct Walk3D64 {
       }
       n2 = __ldg(J.bcn + ib);
     }
-    const bool vacuum = inside && mus <= 0.0 && mus2 > 0.0;
-    const bool jump = inside ? nidx != n2 : n2 > 0.0;
-    if (vacuum || jump || (inside && w < kWeight0)) {
+    const bool vacuum = inside && !positive(mus) && positive(mus2);
+    const bool jump = inside ? differ(nidx, n2) : positive(n2);
+    const bool light = inside && below(w, kWeight0);
+    if (vacuum || jump || light) {
       rng.reload();
       if (vacuum) prop = neg_log_open(rng.next()) / mus2;
-      if (inside && w < kWeight0) {
-        if (unif_closed(rng) > kChance) {
+      if (light) {
+        if (!closed_at_most(rng, kChance)) {
           job_count(J, kJcRoulette); job_ledger(J, kLgRouletteKill, w);
           return die(J, kEvRoulette);
         }
@@ -441,7 +457,7 @@ struct Walk3D64 {
     // reverse-face lookup, MC3D.hpp:1616-1628
     const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((recs(J) + nextel)->nbr));
     const int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : nb2.w == el ? 3 : -1;
-    if (mus2 != mus) {
+    if (differ(mus2, mus)) {
       if (!vacuum) prop *= mus / mus2;  // x (mus / mus) == x
       imus = fast_rcp(mus2);
     }
@@ -449,7 +465,7 @@ struct Walk3D64 {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
     }
-    if (g2 != g) ig = 0.5 * fast_rcp(g2);
+    if (differ(g2, g)) ig = 0.5 * fast_rcp(g2);
     flush(J);
     curface = f2;
     el = nextel;

@@ -190,8 +190,10 @@ __device__ __forceinline__ void acc_add(const JobDev &J, double *p, double v) {
   red_global(p, v);
 }
 
+// v != 0 by its bits: a comparison of doubles is an instruction of the FP64 pipe, which the plain
+// forms wait for
 __device__ __forceinline__ void add_d(const JobDev &J, double *p, double v) {
-  if (v != 0.0) acc_add<false>(J, p, v);
+  if ((__double_as_longlong(v) << 1) != 0) acc_add<false>(J, p, v);
 }
 
 // float -> double by bit manipulation on the integer pipe (exact for normal floats; zero
@@ -359,9 +361,22 @@ __device__ __forceinline__ float f32_of(double x) {
   return __uint_as_float(f | (hi & 0x80000000u));
 }
 
+// Comparisons on the integer pipe (one of doubles takes an instruction of the FP64 pipe).
+__device__ __forceinline__ bool positive(double x) {  // x > 0
+  return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool differ(double a, double b) {  // a != b (a, b no NaN)
+  const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
+  return x != y && ((x | y) << 1) != 0ull;
+}
+__device__ __forceinline__ bool below(double x, double limit) {  // x < limit, for x >= 0 and limit > 0
+  return __double_as_longlong(x) < __double_as_longlong(limit);
+}
+
 // 1 / b, a / b, sqrt(s) and 1 / sqrt(s) from an FP32 first value and Newton's step of second
 // and third order: 3 to 5 FP64 operations, to an ulp or two.  Outside the range where FP32
-// holds the first value the library's function takes over.
+// holds the first value (f32_safe) the library's function takes over; the forms named _near
+// leave that test to the caller.
 __device__ __forceinline__ bool f32_safe(float f) { return fabsf(f) > 1e-30f && fabsf(f) < 1e30f; }
 
 __device__ __forceinline__ double fast_rcp(double b) {
@@ -371,28 +386,33 @@ __device__ __forceinline__ double fast_rcp(double b) {
   const double e = fma(-b, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
-__device__ __forceinline__ double fast_div(double a, double b) {
-  const float bf = f32_of(b);
-  if (!f32_safe(bf)) return a / b;
+__device__ __forceinline__ double div_near(double a, double b, float bf) {  // bf = f32_of(b)
   double y = f2d_int(__frcp_rn(bf));
   y = fma(y, fma(-b, y, 1.0), y);
   const double q = a * y;
   return fma(fma(-b, q, a), y, q);
 }
+__device__ __forceinline__ double fast_div(double a, double b) {
+  const float bf = f32_of(b);
+  return f32_safe(bf) ? div_near(a, b, bf) : a / b;
+}
 // sqrt(s) in r, 1 / sqrt(s) in y
-__device__ __forceinline__ void fast_sqrt(double s, double &r, double &y) {
-  const float sf = f32_of(s);
-  if (!(sf > 1e-30f && sf < 1e30f)) {
-    r = sqrt(s);
-    y = 1.0 / r;
-    return;
-  }
+__device__ __forceinline__ void sqrt_near(double s, float sf, double &r, double &y) {  // sf = f32_of(s)
   const double y0 = f2d_int(rsqrtf(sf));
   const double h = s * y0;
   const double e = fma(-h, y0, 1.0);
   const double p = e * fma(e, 0.375, 0.5);
   r = fma(h, p, h);
   y = fma(y0, p, y0);
+}
+__device__ __forceinline__ void fast_sqrt(double s, double &r, double &y) {
+  const float sf = f32_of(s);
+  if (sf > 1e-30f && sf < 1e30f) {
+    sqrt_near(s, sf, r, y);
+  } else {
+    r = sqrt(s);
+    y = 1.0 / r;
+  }
 }
 __device__ __forceinline__ double fast_sqrt(double s) {
   double r, y;
@@ -407,11 +427,17 @@ __device__ __forceinline__ double unit_scale(double n2) {
 }
 // the word as a double, exactly, with one FP64 operation
 __device__ __forceinline__ double word_d(uint32_t w) { return __hiloint2double(0x43300000, (int)w) - 4503599627370496.0; }
+// unif_closed(rng) <= p, by that mapping (word / (2^32 - 1))
+template <class R> __device__ __forceinline__ bool closed_at_most(R &rng, double p) {
+  return word_d(rng.next()) * (1.0 / 4294967295.0) <= p;
+}
 
-// w (1 - exp(-mua ds)) and the weight left of an absorbing step (mua > 0)
+// 1 - exp(-mua ds) of an absorbing step (mua > 0)
 __device__ __forceinline__ double absorbed_part(double mua, double ds) {
   const double x = mua * ds;
-  return f32_of(x) < 0.0625f ? x * one_minus_exp_over_x(x) : -expm1(-x);
+  double part = x * one_minus_exp_over_x(x);
+  if (!(f32_of(x) < 0.0625f)) part = -expm1(-x);
+  return part;
 }
 
 }  // namespace vmc
