@@ -161,11 +161,12 @@ def lib(build_if_missing=True):
 
 
 def _ptr(a, t=C.c_double):
-    return None if a is None else a.ctypes.data_as(C.POINTER(t))
+    return None if a is None else C.cast(a.__array_interface__["data"][0], C.POINTER(t))
 
 
 def colmajor(a, dtype):
-    return np.asfortranarray(np.asarray(a, dtype=dtype)).ravel(order="F").copy()
+    a = np.asarray(a, dtype=dtype)
+    return a.T.ravel() if a.flags.c_contiguous and a.ndim == 2 and min(a.shape) > 1 else a.ravel(order="F").copy()
 
 
 class _Marshal:

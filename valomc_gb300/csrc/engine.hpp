@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -40,17 +41,29 @@ int upload_mesh(DeviceMesh &m, int precision_mask);
 // TetRec / TriRec [Ne] at `geom` from the Tet64 / Tri64 [Ne] behind them
 cudaError_t make_plane_records(int dim, void *geom, int64_t Ne, cudaStream_t st);
 
-// Device state of one job.
+// Memory of calls and launches: a pool of this library's per device, so that a call's buffers
+// are not mapped and unmapped each time.  It keeps at most kPoolKeep bytes between calls (what is
+// freed beyond that goes back at the next synchronisation), and all of it when an allocation fails.
+constexpr uint64_t kPoolKeep = 256ull << 20;
+int call_pool(int device, cudaMemPool_t *pool);
+// cudaMallocFromPoolAsync; gives the kept memory back and tries again when there is none
+cudaError_t pool_alloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st);
+
+// Device state of one job, in one allocation: what is uploaded, then what the kernel adds to.
 struct JobBuffers {
+  void *d_block = nullptr;
+  Raw<unsigned char> staged;  // host image of the uploaded part (alive while its copy may run)
   void *d_optics = nullptr;
   uint8_t *d_bctype = nullptr;
   double *d_bcn = nullptr, *d_cdf = nullptr;
   SourceRec *d_src = nullptr;
   float *d_cdf_f = nullptr;
   SourceRecF *d_src_f = nullptr;
-  double *d_acc = nullptr;  // ER, EI [Ne]; EBR, EBI, DEBR, DEBI [Nb]
+  // counters, ledger and accumulators lie back to back: cleared and read back at once
   unsigned long long *d_jc = nullptr;
   double *d_ledger = nullptr;
+  double *d_acc = nullptr;  // ER, EI [Ne]; EBR, EBI, DEBR, DEBI [Nb]
+  size_t result_bytes() const { return sizeof(double) * (size_t)(kSlots * (kJcN + kLgN) + 2 * Ne + 4 * Nb); }
   uint32_t *d_tape = nullptr;
   int64_t *d_tape_off = nullptr, *d_trace = nullptr, *d_trace_len = nullptr;
   int64_t bytes = 0;
@@ -85,9 +98,10 @@ struct LaunchResult {
   int grid = 0, block = 0;
 };
 // Runs the pool kernel over jobs (device descriptors are uploaded here) and waits,
-// polling progress / cancel / timeout from opt (may be null).  Stream-ordered.
+// polling progress / cancel / timeout from opt (may be null).  Stream-ordered.  meanwhile: host
+// work to do while the kernel runs.
 int launch_jobs(int device, const LaunchSpec &spec, const std::vector<JobDev> &jobs, const vmc_options *opt,
-                cudaStream_t st, LaunchResult &res);
+                cudaStream_t st, LaunchResult &res, const std::function<void()> &meanwhile = nullptr);
 
 // Device and pinned buffers of one launch at a time, reused across launches: the job
 // table, its photon prefix, the control block, the timing events and a graph.  Lets a
@@ -113,9 +127,13 @@ int launch_start(int device, const LaunchSpec &spec, const std::vector<JobDev> &
 // Waits for the arena's launch and reads its counters (no-op when nothing is in flight).
 int launch_finish(LaunchArena &a, cudaStream_t st, LaunchResult &res);
 
-// Copies a job's accumulators and counters back and fills out/stats.
+// Copies a job's accumulators and counters back (into `back`, kept by the caller for the next)
+// and fills out/stats.
 int collect_job(const HostJob &j, const DeviceMesh &m, const JobBuffers &b, int64_t nphoton, bool normalize,
-                vmc_output *out, vmc_stats *st, cudaStream_t stream);
+                vmc_output *out, vmc_stats *st, cudaStream_t stream, Raw<double> &back);
+// Touches the pages that collect_job will fill, so that they are mapped while the kernel runs and
+// not by the copy (10 MB into fresh pages took 2 to 10 ms, into mapped ones 0.07).
+void touch_results(const HostMesh &m, const JobBuffers &b, const vmc_output *out, Raw<double> &back);
 
 const void *kernel_3d64(bool fd, bool tape, bool one, bool tab);
 const void *kernel_3d64_literal(bool fd, bool tape, bool one, bool tab);

@@ -131,7 +131,20 @@ const char *mcerror_string(int s) {
 }
 
 // ErrorChecks, MC3D.hpp:460-571 / MC2D.hpp:390-513
-int check_input(const vmc_input *in) {
+bool nodes_in_range(const int64_t *idx, int64_t n, int64_t Nr) {
+  int64_t bad = 0;
+#pragma omp parallel for schedule(static) reduction(+ : bad) if (n > 200000)
+  for (int64_t i = 0; i < n; i++) bad += (uint64_t)idx[i] >= (uint64_t)Nr;
+  return bad == 0;
+}
+
+void use_mesh(vmc_input &in, const HostMesh &m) {
+  in.dim = m.dim; in.Ne = m.Ne; in.Nb = m.Nb; in.Nr = m.Nr;
+  in.H = m.H; in.BH = m.BH; in.r = m.r;
+  in.HN = nullptr; in.n_HN = 0;
+}
+
+int check_input(const vmc_input *in, bool indices) {
   if (!in || (in->dim != 2 && in->dim != 3)) return VMC_ERR_INVALID_ARGUMENT;
   if (in->Ne < 0 || in->Nb < 0 || in->Nr < 0) return VMC_ERR_INVALID_ARGUMENT;
   if (in->n_g != in->Ne) return E_SIZE_MISMATCH_G;
@@ -151,11 +164,9 @@ int check_input(const vmc_input *in) {
   if (in->n_BCLNormal && in->n_BCLNormal != in->Nb) return E_SIZE_MISMATCH_LIGHT_DIRECTION;
   if (in->n_BCLightDirectionType && in->n_BCLightDirectionType != in->Nb) return E_SIZE_MISMATCH_LIGHT_DIRECTION_TYPE;
   if ((in->Ne && !in->H) || (in->Nb && !in->BH) || (in->Nr && !in->r)) return VMC_ERR_INVALID_ARGUMENT;
-  const int64_t nh = in->Ne * (in->dim + 1), nb = in->Nb * in->dim;
-  for (int64_t i = 0; i < nh; i++)
-    if (in->H[i] < 0 || in->H[i] >= in->Nr) return E_INCONSISTENT_H;
-  for (int64_t i = 0; i < nb; i++)
-    if (in->BH[i] < 0 || in->BH[i] >= in->Nr) return E_INCONSISTENT_BH;
+  if (!indices) return VMC_OK;
+  if (!nodes_in_range(in->H, in->Ne * (in->dim + 1), in->Nr)) return E_INCONSISTENT_H;
+  if (!nodes_in_range(in->BH, in->Nb * in->dim, in->Nr)) return E_INCONSISTENT_BH;
   return VMC_OK;
 }
 
@@ -168,22 +179,26 @@ int check_input(const vmc_input *in) {
 // reference's sequential loop.
 int build_neighbours(int dim, int64_t Ne, int64_t Nb, int64_t Nr, const int64_t *H, const int64_t *BH, int64_t *HN) {
   const int NF = dim + 1;
+  // incidence lists, filled by all threads: the order within a list does not matter below
   std::vector<int64_t> off((size_t)Nr + 1, 0);
-  for (int64_t i = 0; i < Ne; i++)
-    for (int c = 0; c < NF; c++) off[(size_t)H[i + Ne * c] + 1]++;
-  for (int64_t i = 0; i < Nb; i++)
-    for (int c = 0; c < dim; c++) off[(size_t)BH[i + Nb * c] + 1]++;
+  auto each_incidence = [&](auto &&take) {
+#pragma omp parallel for schedule(static) if (Ne > 20000)
+    for (int64_t i = 0; i < Ne; i++)
+      for (int c = 0; c < NF; c++) take((size_t)H[i + Ne * c], i);
+    for (int64_t i = 0; i < Nb; i++)
+      for (int c = 0; c < dim; c++) take((size_t)BH[i + Nb * c], -1 - i);
+  };
+  each_incidence([&](size_t v, int64_t) { __atomic_fetch_add(&off[v + 1], 1, __ATOMIC_RELAXED); });
   for (int64_t v = 0; v < Nr; v++) off[(size_t)v + 1] += off[(size_t)v];
-  std::vector<int64_t> fill(off.begin(), off.end() - 1), lst((size_t)off[(size_t)Nr]);
-  for (int64_t i = 0; i < Ne; i++)
-    for (int c = 0; c < NF; c++) lst[(size_t)fill[(size_t)H[i + Ne * c]]++] = i;
-  for (int64_t i = 0; i < Nb; i++)
-    for (int c = 0; c < dim; c++) lst[(size_t)fill[(size_t)BH[i + Nb * c]]++] = -1 - i;
+  std::vector<int64_t> fill(off.begin(), off.end() - 1);
+  Raw<int64_t> lst;
+  lst.resize((size_t)off[(size_t)Nr]);
+  each_incidence([&](size_t v, int64_t i) { lst[(size_t)__atomic_fetch_add(&fill[v], 1, __ATOMIC_RELAXED)] = i; });
 
   const int dup_err = dim == 3 ? E_INCONSISTENT_MESH_DUPLICATE_NEIGHBORS : E_INCONSISTENT_MESH;
   int64_t worst_el = std::numeric_limits<int64_t>::max();
   int worst_code = 0;
-#pragma omp parallel
+#pragma omp parallel if (Ne > 2000)
   {
     int64_t my_el = std::numeric_limits<int64_t>::max();
     int my_code = 0;
@@ -232,26 +247,59 @@ int build_neighbours(int dim, int64_t Ne, int64_t Nb, int64_t Nr, const int64_t 
   return worst_code;
 }
 
-int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m) {
+template <class T>
+static void copy_of(Raw<T> &to, const T *from, size_t n) {
+  to.resize(n);
+#pragma omp parallel for schedule(static) if (n > 100000)
+  for (size_t i = 0; i < n; i++) to[i] = from[i];
+}
+
+int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own) {
   const int D = in->dim, NF = D + 1;
   m.dim = D; m.Ne = in->Ne; m.Nb = in->Nb; m.Nr = in->Nr;
   if (m.Ne >= (int64_t)kOpenFace || m.Nb >= (int64_t)kOpenFace) return VMC_ERR_SIZE_LIMIT;
-  m.H.assign(in->H, in->H + m.Ne * NF);
-  m.BH.assign(in->BH, in->BH + m.Nb * D);
-  m.r.assign(in->r, in->r + m.Nr * D);
-  m.HN.assign((size_t)(m.Ne * NF), 0);
+  m.H = in->H; m.BH = in->BH; m.r = in->r;
+  if (own) {
+    copy_of(m.own_H, in->H, (size_t)(m.Ne * NF));
+    copy_of(m.own_BH, in->BH, (size_t)(m.Nb * D));
+    copy_of(m.own_r, in->r, (size_t)(m.Nr * D));
+    m.H = m.own_H.data(); m.BH = m.own_BH.data(); m.r = m.own_r.data();
+  }
   if (in->HN && in->n_HN == in->Ne) {  // MC3D.hpp:839: a neighbourhood of the right size is used as given
-    m.HN.assign(in->HN, in->HN + m.Ne * NF);
+    copy_of(m.HN, in->HN, (size_t)(m.Ne * NF));
   } else {
-    int s = build_neighbours(D, m.Ne, m.Nb, m.Nr, m.H.data(), m.BH.data(), m.HN.data());
+    m.HN.resize((size_t)(m.Ne * NF));
+    int s = build_neighbours(D, m.Ne, m.Nb, m.Nr, m.H, m.BH, m.HN.data());
     if (s) return s;
   }
-  Geo G{m.H.data(), m.BH.data(), m.r.data(), m.Ne, m.Nb, m.Nr};
+  // the faces on the boundary, for the light sources of every job on the mesh
+  m.faces.clear();
+  m.faces.reserve((size_t)m.Nb);
+#pragma omp parallel if (m.Ne > 20000)
+  {
+    std::vector<BoundaryFace> mine;
+#pragma omp for schedule(static) nowait
+    for (int64_t el = 0; el < m.Ne; el++)
+      for (int f = 0; f < NF; f++) {
+        const int64_t h = m.HN[(size_t)(el + m.Ne * f)];
+        if (h > -1 || h < -m.Nb) continue;
+        int first = f;
+        for (int ff = f - 1; ff >= 0; ff--)
+          if (m.HN[(size_t)(el + m.Ne * ff)] == h) first = ff;
+        mine.push_back(BoundaryFace{(int32_t)el, (int32_t)(-1 - h), (int8_t)f, (int8_t)first});
+      }
+#pragma omp critical
+    m.faces.insert(m.faces.end(), mine.begin(), mine.end());
+  }
+  std::sort(m.faces.begin(), m.faces.end(),
+            [](const BoundaryFace &a, const BoundaryFace &b) { return a.el != b.el ? a.el < b.el : a.f < b.f; });
+  Geo G{m.H, m.BH, m.r, m.Ne, m.Nb, m.Nr};
   m.volume.resize((size_t)m.Ne);
   m.area.resize((size_t)m.Nb);
   m.bnorm.assign((size_t)m.Nb * 4, 0.0);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (m.Ne > 20000)
   for (int64_t i = 0; i < m.Ne; i++) m.volume[(size_t)i] = D == 3 ? volume3(G, i) : area2(G, i);
+#pragma omp parallel for schedule(static) if (m.Nb > 10000)
   for (int64_t i = 0; i < m.Nb; i++) {
     m.area[(size_t)i] = D == 3 ? area3(G, i) : length2(G, i);
     if (D == 3) normal_b3(G, i, &m.bnorm[(size_t)i * 4]);
@@ -265,7 +313,7 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m) {
   if (D == 3) {
     if (precision_mask & 1) {
       m.tet64.resize((size_t)m.Ne);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (m.Ne > 20000)
       for (int64_t el = 0; el < m.Ne; el++) {
         Tet64 &T = m.tet64[(size_t)el];
         for (int v = 0; v < 4; v++)
@@ -275,7 +323,7 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m) {
     }
     if (precision_mask & 2) {
       m.tet32.resize((size_t)m.Ne);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (m.Ne > 20000)
       for (int64_t el = 0; el < m.Ne; el++) {
         Tet32 &T = m.tet32[(size_t)el];
         for (int f = 0; f < 4; f++) {
@@ -306,6 +354,7 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m) {
   } else {
     if (precision_mask & 1) {
       m.tri64.resize((size_t)m.Ne);
+#pragma omp parallel for schedule(static) if (m.Ne > 20000)
       for (int64_t el = 0; el < m.Ne; el++) {
         Tri64 &T = m.tri64[(size_t)el];
         for (int v = 0; v < 3; v++)
@@ -316,6 +365,7 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m) {
     }
     if (precision_mask & 2) {
       m.tri32.resize((size_t)m.Ne);
+#pragma omp parallel for schedule(static) if (m.Ne > 20000)
       for (int64_t el = 0; el < m.Ne; el++) {
         Tri32 &T = m.tri32[(size_t)el];
         for (int f = 0; f < 3; f++) {
@@ -341,13 +391,47 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m) {
   return VMC_OK;
 }
 
+// all of x equal its first value
+static bool uniform(const double *x, int64_t n) {
+  for (int64_t i = 1; i < n && i < 4096; i++)
+    if (x[i] != x[0]) return false;
+  int64_t other = 0;
+#pragma omp parallel for schedule(static) reduction(+ : other) if (n > 100000)
+  for (int64_t i = 4096; i < n; i++) other += x[i] != x[0];
+  return other == 0;
+}
+
+double HostJob::k_of(int64_t i) const { return omega / kC0 * n[homogeneous ? 0 : i]; }
+
+void HostJob::keep() {
+  const size_t c = rows();
+  own.resize(4 * c);
+  const double *from[4] = {mua, mus, g, n};
+  for (int q = 0; q < 4; q++) memcpy(own.data() + q * c, from[q], c * sizeof(double));
+  mua = own.data(); mus = mua + c; g = mua + 2 * c; n = mua + 3 * c;
+}
+
+template <class T>
+static void rows_of(const HostJob &j, T *out) {
+  const int64_t c = (int64_t)j.rows();
+#pragma omp parallel for schedule(static) if (c > 50000)
+  for (int64_t i = 0; i < c; i++) {
+    out[4 * i] = (T)j.mua[i];
+    out[4 * i + 1] = (T)j.mus[i];
+    out[4 * i + 2] = (T)j.g[i];
+    out[4 * i + 3] = (T)j.n[i];
+  }
+}
+void HostJob::optics_rows(float *out) const { rows_of(*this, out); }
+void HostJob::optics_rows(double *out) const { rows_of(*this, out); }
+
 // Init's light sources and BCLNormal handling (MC3D.hpp:611-735, :941-1002;
 // MC2D.hpp:553-640, :851-911) and the per-face launch quantities of CreatePhoton.
 int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
-  const int D = m.dim, NF = D + 1;
+  const int D = m.dim;
   const int64_t Ne = m.Ne, Nb = m.Nb;
   if (in->dim != D || in->Ne != Ne || in->Nb != Nb) return VMC_ERR_INVALID_ARGUMENT;
-  Geo G{m.H.data(), m.BH.data(), m.r.data(), m.Ne, m.Nb, m.Nr};
+  Geo G{m.H, m.BH, m.r, m.Ne, m.Nb, m.Nr};
   j.dim = D; j.Ne = Ne; j.Nb = Nb;
   j.f = in->f;
   j.omega = 2.0 * kPi * in->f;
@@ -364,21 +448,8 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
   }
   j.Nphoton = in->Nphoton;
   // optics rows; a job whose elements all share one row keeps a single row
-  bool hom = Ne > 0;
-  for (int64_t i = 1; i < Ne && hom; i++)
-    hom = in->mua[i] == in->mua[0] && in->mus[i] == in->mus[0] && in->g[i] == in->g[0] && in->n[i] == in->n[0];
-  j.homogeneous = hom;
-  const int64_t rows = hom ? 1 : Ne;
-  j.optics.resize((size_t)rows * 4);
-  for (int64_t i = 0; i < rows; i++) {
-    j.optics[(size_t)i * 4 + 0] = in->mua[i];
-    j.optics[(size_t)i * 4 + 1] = in->mus[i];
-    j.optics[(size_t)i * 4 + 2] = in->g[i];
-    j.optics[(size_t)i * 4 + 3] = in->n[i];
-  }
-  j.mua.assign(in->mua, in->mua + Ne);
-  j.k.resize((size_t)Ne);
-  for (int64_t i = 0; i < Ne; i++) j.k[(size_t)i] = j.omega / kC0 * in->n[i];  // MC3D.hpp:660-662
+  j.homogeneous = Ne > 0 && uniform(in->mua, Ne) && uniform(in->mus, Ne) && uniform(in->g, Ne) && uniform(in->n, Ne);
+  j.mua = in->mua; j.mus = in->mus; j.g = in->g; j.n = in->n;
   j.bctype.assign(reinterpret_cast<const uint8_t *>(in->BCType), reinterpret_cast<const uint8_t *>(in->BCType) + Nb);
   j.bcn.assign(in->BCn, in->BCn + Nb);
   // BCLightDirectionType defaults to 'n' (MC3D.hpp:646-654), BCLNormal is normalised
@@ -435,11 +506,9 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
   // BuildLightSource: emitting faces in (element, face) order; CDF of area x intensity
   j.src.clear();
   std::vector<double> w;
-  for (int64_t el = 0; el < Ne; el++) {
-    for (int f = 0; f < NF; f++) {
-      const int64_t h = m.HN[(size_t)(el + Ne * f)];
-      if (h > -1) continue;
-      const int64_t ib = -1 - h;
+  {
+    for (const BoundaryFace &bf : m.faces) {
+      const int64_t el = bf.el, ib = bf.ib;
       const char bt = in->BCType[ib];
       if (!is_source(D, bt)) continue;
       SourceRec S;
@@ -448,9 +517,7 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
       S.ib = (int32_t)ib;
       S.type = bt;
       S.dirtype = dtype[(size_t)ib];
-      S.curface = -1;
-      for (int ff = 0; ff < NF; ff++)
-        if (-1 - m.HN[(size_t)(el + Ne * ff)] == ib) { S.curface = ff; break; }
+      S.curface = bf.first;
       if (D == 3) {
         for (int c = 0; c < 3; c++) {
           S.v0[c] = G.x(G.bh(ib, 0), c);
@@ -543,9 +610,7 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
 
 bool rough_optics(const vmc_input *in, const HostMesh &m) {
   const int64_t Ne = m.Ne;
-  bool same = true;
-  for (int64_t i = 1; i < Ne && same; i++) same = in->mus[i] == in->mus[0] && in->n[i] == in->n[0];
-  if (same) return false;
+  if (uniform(in->mus, Ne) && uniform(in->n, Ne)) return false;
   int64_t faces = 0, changes = 0;
 #pragma omp parallel for schedule(static) reduction(+ : faces, changes) if (Ne > 20000)
   for (int64_t i = 0; i < Ne; i++)
@@ -570,11 +635,11 @@ void normalise(const HostMesh &m, const HostJob &j, int64_t nphoton, const doubl
     double a = ER[i], b = EI[i], er, ei;
     if (!apply) { er = a; ei = b; }
     else if (cw) {
-      const double mu = j.mua[(size_t)i], V = m.volume[(size_t)i];
+      const double mu = j.mua_of(i), V = m.volume[(size_t)i];
       er = mu > 0.0 ? a / (mu * V * Nd) : a / (V * Nd);
       ei = b;
     } else {
-      const double k = j.k[(size_t)i], mu = j.mua[(size_t)i], V = m.volume[(size_t)i];
+      const double k = j.k_of(i), mu = j.mua_of(i), V = m.volume[(size_t)i];
       er = (b * k + a * mu) / (sq(k) + sq(mu)) / Nd / V;
       ei = -(a * k - b * mu) / (sq(k) + sq(mu)) / Nd / V;
     }

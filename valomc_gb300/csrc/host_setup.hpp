@@ -5,6 +5,9 @@
 #pragma once
 #include <stdint.h>
 
+#include <cstddef>
+#include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -13,21 +16,53 @@
 
 namespace vmc {
 
+// An array of plain values that starts uninitialised: its pages are first touched by the threads
+// that fill it, not by a zeroing constructor.
+template <class T>
+class Raw {
+ public:
+  void resize(size_t n) {
+    if (n != n_) p_.reset(n ? new T[n] : nullptr);
+    n_ = n;
+  }
+  void clear() { resize(0); }
+  T *data() { return p_.get(); }
+  const T *data() const { return p_.get(); }
+  size_t size() const { return n_; }
+  T &operator[](size_t i) { return p_[i]; }
+  const T &operator[](size_t i) const { return p_[i]; }
+
+ private:
+  std::unique_ptr<T[]> p_;
+  size_t n_ = 0;
+};
+
+// A face of element el on the boundary (face f behind boundary element ib); first: the lowest
+// face of el on ib.
+struct BoundaryFace {
+  int32_t el, ib;
+  int8_t f, first;
+};
+
 // Geometry shared by every job on a mesh.
 struct HostMesh {
   int dim = 3;
   int64_t Ne = 0, Nb = 0, Nr = 0;
-  std::vector<int64_t> H, BH;   // column-major copies
-  std::vector<double> r;
-  std::vector<int64_t> HN;      // column-major [Ne x (dim+1)]
-  std::vector<double> volume;   // ElementVolume / ElementArea(el)
-  std::vector<double> area;     // ElementArea(ib) / ElementLength(ib)
+  // column-major; the caller's arrays for a mesh that lives for one call, else copies
+  const int64_t *H = nullptr, *BH = nullptr;
+  const double *r = nullptr;
+  Raw<int64_t> own_H, own_BH;
+  Raw<double> own_r;
+  Raw<int64_t> HN;              // column-major [Ne x (dim+1)]
+  std::vector<BoundaryFace> faces;  // in (element, face) order
+  Raw<double> volume;           // ElementVolume / ElementArea(el)
+  Raw<double> area;             // ElementArea(ib) / ElementLength(ib)
   std::vector<double> bnorm;    // [Nb x 4] Normal(ib)
-  // device records
-  std::vector<Tet64> tet64;
-  std::vector<Tet32> tet32;
-  std::vector<Tri64> tri64;
-  std::vector<Tri32> tri32;
+  // device records, until they are uploaded
+  Raw<Tet64> tet64;
+  Raw<Tet32> tet32;
+  Raw<Tri64> tri64;
+  Raw<Tri32> tri32;
 };
 
 // One problem on a mesh: optics, boundary conditions, sources, scalars.
@@ -35,8 +70,17 @@ struct HostJob {
   int dim = 3;
   int64_t Ne = 0, Nb = 0;
   bool homogeneous = false;
-  std::vector<double> optics;   // rows of (mua, mus, g, n); one row when homogeneous
-  std::vector<double> mua;      // for the normalisation
+  // optics of the elements (a single one each when homogeneous): the caller's arrays, or the
+  // job's own after keep()
+  const double *mua = nullptr, *mus = nullptr, *g = nullptr, *n = nullptr;
+  Raw<double> own;
+  size_t rows() const { return homogeneous ? 1 : (size_t)Ne; }
+  double mua_of(int64_t i) const { return mua[homogeneous ? 0 : i]; }
+  double k_of(int64_t i) const;  // omega / c0 * n (MC3D.hpp:660-662)
+  void keep();                   // copies the optics out of the caller's arrays
+  // rows of (mua, mus, g, n)
+  void optics_rows(float *out) const;
+  void optics_rows(double *out) const;
   std::vector<uint8_t> bctype;
   std::vector<double> bcn;
   std::vector<SourceRec> src;
@@ -48,7 +92,6 @@ struct HostJob {
   uint64_t turn0 = 0;           // phase0 in 2^-64 turns
   int64_t Nphoton = 0;
   uint64_t seed = 0;
-  std::vector<double> k;        // omega / c0 * n per element (FD normalisation)
 };
 
 // Whether the scattering coefficient or the index changes across more than an eighth of the mesh's
@@ -59,7 +102,11 @@ struct HostJob {
 bool rough_optics(const vmc_input *in, const HostMesh &m);
 
 // ErrorChecks (same checks, same order, same codes).  Returns VMC_OK or 1 + mcerror.
-int check_input(const vmc_input *in);
+// indices: also that H and BH name nodes (done once, when a resident mesh was made).
+int check_input(const vmc_input *in, bool indices = true);
+bool nodes_in_range(const int64_t *idx, int64_t n, int64_t Nr);
+// an input's geometry replaced by a resident mesh's
+void use_mesh(vmc_input &in, const HostMesh &m);
 
 // BuildNeighbourhoods: HN [Ne x (dim+1)] column-major with the reference's semantics
 // (boundary -1 - ib, 3D open faces INT64_MAX, 2D open edges -> MISSING_BOUNDARY,
@@ -67,11 +114,12 @@ int check_input(const vmc_input *in);
 int build_neighbours(int dim, int64_t Ne, int64_t Nb, int64_t Nr, const int64_t *H, const int64_t *BH, int64_t *HN);
 
 // Mesh from the geometry arrays of an input (HN built unless given).  precision_mask:
-// bit 0 builds the FP64 records, bit 1 the FP32 records.
-int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m);
+// bit 0 builds the FP64 records, bit 1 the FP32 records.  own: the mesh outlives the input's
+// arrays and copies them.
+int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own);
 
 // Job from the problem arrays of an input on mesh m (Init's light sources, BCLNormal
-// processing and wave numbers).
+// processing and wave numbers).  The job reads the input's optics arrays until keep().
 int build_job(const vmc_input *in, const HostMesh &m, HostJob &j);
 
 // MonteCarlo's normalisation of raw accumulators into the caller's output arrays.

@@ -137,10 +137,8 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   if (!(mesh_precision_mask(mesh) & (o.precision == VMC_FP64 ? 1 : 2))) return VMC_ERR_INVALID_ARGUMENT;
   // host half: ErrorChecks + Init on the mesh's geometry
   vmc_input in = *job;
-  in.dim = m->host.dim; in.Ne = m->host.Ne; in.Nb = m->host.Nb; in.Nr = m->host.Nr;
-  in.H = m->host.H.data(); in.BH = m->host.BH.data(); in.r = m->host.r.data();
-  in.HN = nullptr; in.n_HN = 0;
-  int s = check_input(&in);
+  use_mesh(in, m->host);
+  int s = check_input(&in, false);
   if (s) return s;
   HostJob hj;
   s = build_job(&in, m->host, hj);
@@ -167,11 +165,14 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   cudaStream_t st = own.s;
   // the job's arrays into the caller's buffers
   std::vector<float> optf;
+  std::vector<double> optd;
   if (o.precision == VMC_FP64) {
-    VMC_CK(cudaMemcpyAsync(dev->optics, hj.optics.data(), rows * 4 * sizeof(double), cudaMemcpyHostToDevice, st));
+    optd.resize(rows * 4);
+    hj.optics_rows(optd.data());
+    VMC_CK(cudaMemcpyAsync(dev->optics, optd.data(), rows * 4 * sizeof(double), cudaMemcpyHostToDevice, st));
   } else {
     optf.resize(rows * 4);
-    for (size_t i = 0; i < rows * 4; i++) optf[i] = (float)hj.optics[i];
+    hj.optics_rows(optf.data());
     VMC_CK(cudaMemcpyAsync(dev->optics, optf.data(), rows * 4 * sizeof(float), cudaMemcpyHostToDevice, st));
   }
   VMC_CK(cudaMemcpyAsync(dev->bctype, hj.bctype.data(), (size_t)Nb, cudaMemcpyHostToDevice, st));

@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cmath>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -71,9 +72,52 @@ template <class T>
 static int dalloc(T **p, size_t count, int64_t &bytes) {
   *p = nullptr;
   if (count == 0) count = 1;
-  VMC_CK(cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T)));
+  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T));
+  if (e == cudaErrorMemoryAllocation) {  // what the call pool keeps may be enough
+    cudaGetLastError();
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    if (cudaGetDevice(&dev) == cudaSuccess && call_pool(dev, &pool) == VMC_OK) {
+      cudaDeviceSynchronize();
+      cudaMemPoolTrimTo(pool, 0);
+      e = cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T));
+    }
+  }
+  VMC_CK(e);
   bytes += (int64_t)(count * sizeof(T));
   return VMC_OK;
+}
+
+int call_pool(int device, cudaMemPool_t *pool) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[128] = {nullptr};
+  if (device < 0 || device >= 128) return VMC_ERR_INVALID_ARGUMENT;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[device]) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t p = nullptr;
+    VMC_CK(cudaMemPoolCreate(&p, &props));
+    uint64_t keep = kPoolKeep;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    pools[device] = p;
+  }
+  *pool = pools[device];
+  return VMC_OK;
+}
+
+cudaError_t pool_alloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaStreamSynchronize(st);
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  }
+  return e;
 }
 
 // from a memory pool, ordered on stream st (pool == nullptr: plain cudaMalloc)
@@ -82,7 +126,7 @@ static int dalloc(T **p, size_t count, int64_t &bytes, cudaMemPool_t pool, cudaS
   if (!pool) return dalloc(p, count, bytes);
   *p = nullptr;
   if (count == 0) count = 1;
-  VMC_CK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), count * sizeof(T), pool, st));
+  VMC_CK(pool_alloc(reinterpret_cast<void **>(p), count * sizeof(T), pool, st));
   bytes += (int64_t)(count * sizeof(T));
   return VMC_OK;
 }
@@ -114,7 +158,7 @@ DeviceMesh::~DeviceMesh() {
 }
 
 int upload_mesh(DeviceMesh &m, int precision_mask) {
-  const HostMesh &h = m.host;
+  HostMesh &h = m.host;
   m.dim = h.dim;
   cudaStream_t st = m.st;
   if ((precision_mask & 1) && !m.d_geom[VMC_FP64]) {
@@ -146,19 +190,20 @@ int upload_mesh(DeviceMesh &m, int precision_mask) {
     VMC_TRY(h2d(m.d_bnorm, h.bnorm.data(), h.bnorm.size(), st));
   }
   VMC_CK(cudaStreamSynchronize(st));
+  h.tet64.clear(); h.tet32.clear(); h.tri64.clear(); h.tri32.clear();  // on the device from here on
   return VMC_OK;
 }
 
 JobBuffers::~JobBuffers() { release(); }
 
 void JobBuffers::release() {
-  void *ps[] = {d_optics, d_bctype, d_bcn, d_cdf, d_src, d_cdf_f, d_src_f, d_acc, d_jc, d_ledger,
-                d_tape, d_tape_off, d_trace, d_trace_len};
+  void *ps[] = {d_block, d_tape, d_tape_off, d_trace, d_trace_len};
   for (void *p : ps)
     if (p) {
       if (pool) cudaFreeAsync(p, free_stream);
       else cudaFree(p);
     }
+  d_block = nullptr;
   d_optics = nullptr; d_bctype = nullptr; d_bcn = d_cdf = nullptr; d_src = nullptr; d_acc = nullptr;
   d_cdf_f = nullptr; d_src_f = nullptr;
   d_jc = nullptr; d_ledger = nullptr; d_tape = nullptr; d_tape_off = d_trace = d_trace_len = nullptr;
@@ -174,43 +219,51 @@ int64_t job_footprint(const HostJob &j, const HostMesh &m) {
 int upload_job(const HostJob &j, const DeviceMesh &m, int precision, JobBuffers &b, cudaStream_t st) {
   const int64_t Ne = m.host.Ne, Nb = m.host.Nb;
   b.Ne = Ne; b.Nb = Nb;
-  const size_t rows = j.homogeneous ? 1 : (size_t)Ne;
-  if (precision == VMC_FP64) {
-    double *d;
-    VMC_TRY(dalloc(&d, rows * 4, b.bytes, b.pool, st));
-    b.d_optics = d;
-    VMC_TRY(h2d(d, j.optics.data(), rows * 4, st));
-  } else {
-    std::vector<float> f(rows * 4);
-    for (size_t i = 0; i < rows * 4; i++) f[i] = (float)j.optics[i];
-    float *d;
-    VMC_TRY(dalloc(&d, rows * 4, b.bytes, b.pool, st));
-    b.d_optics = d;
-    VMC_TRY(h2d(d, f.data(), rows * 4, st));
-    VMC_CK(cudaStreamSynchronize(st));  // f is a temporary
-  }
-  VMC_TRY(dalloc(&b.d_bctype, (size_t)Nb, b.bytes, b.pool, st));
-  VMC_TRY(h2d(b.d_bctype, j.bctype.data(), (size_t)Nb, st));
-  VMC_TRY(dalloc(&b.d_bcn, (size_t)Nb, b.bytes, b.pool, st));
-  VMC_TRY(h2d(b.d_bcn, j.bcn.data(), (size_t)Nb, st));
-  VMC_TRY(dalloc(&b.d_cdf, j.cdf.size(), b.bytes, b.pool, st));
-  VMC_TRY(h2d(b.d_cdf, j.cdf.data(), j.cdf.size(), st));
-  VMC_TRY(dalloc(&b.d_src, j.src.size(), b.bytes, b.pool, st));
-  VMC_TRY(h2d(b.d_src, j.src.data(), j.src.size(), st));
-  VMC_TRY(dalloc(&b.d_cdf_f, j.cdf_f.size(), b.bytes, b.pool, st));
-  VMC_TRY(h2d(b.d_cdf_f, j.cdf_f.data(), j.cdf_f.size(), st));
-  VMC_TRY(dalloc(&b.d_src_f, j.src_f.size(), b.bytes, b.pool, st));
-  VMC_TRY(h2d(b.d_src_f, j.src_f.data(), j.src_f.size(), st));
-  VMC_TRY(dalloc(&b.d_acc, (size_t)(2 * Ne + 4 * Nb), b.bytes, b.pool, st));
-  VMC_TRY(dalloc(&b.d_jc, (size_t)kSlots * kJcN, b.bytes, b.pool, st));
-  VMC_TRY(dalloc(&b.d_ledger, (size_t)kSlots * kLgN, b.bytes, b.pool, st));
+  // one block: optics, boundary and sources, then counters, ledger and accumulators
+  size_t at = 0;
+  auto place = [&](size_t bytes) {
+    const size_t off = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return off;
+  };
+  const size_t row = precision == VMC_FP64 ? 4 * sizeof(double) : 4 * sizeof(float);
+  const size_t o_opt = place(j.rows() * row), o_src = place(j.src.size() * sizeof(SourceRec)),
+               o_srcf = place(j.src_f.size() * sizeof(SourceRecF)), o_cdf = place(j.cdf.size() * sizeof(double)),
+               o_bcn = place((size_t)Nb * sizeof(double)), o_cdff = place(j.cdf_f.size() * sizeof(float)),
+               o_bct = place((size_t)Nb);
+  const size_t up = at, o_res = place(b.result_bytes());
+  unsigned char *d;
+  VMC_TRY(dalloc(&d, at, b.bytes, b.pool, st));
+  b.d_block = d;
+  b.staged.resize(up);
+  unsigned char *h = b.staged.data();
+  if (precision == VMC_FP64) j.optics_rows(reinterpret_cast<double *>(h + o_opt));
+  else j.optics_rows(reinterpret_cast<float *>(h + o_opt));
+  auto put = [&](size_t off, const void *src, size_t bytes) {
+    if (bytes) memcpy(h + off, src, bytes);
+  };
+  put(o_src, j.src.data(), j.src.size() * sizeof(SourceRec));
+  put(o_srcf, j.src_f.data(), j.src_f.size() * sizeof(SourceRecF));
+  put(o_cdf, j.cdf.data(), j.cdf.size() * sizeof(double));
+  put(o_bcn, j.bcn.data(), (size_t)Nb * sizeof(double));
+  put(o_cdff, j.cdf_f.data(), j.cdf_f.size() * sizeof(float));
+  put(o_bct, j.bctype.data(), (size_t)Nb);
+  VMC_TRY(h2d(d, h, up, st));
+  b.d_optics = d + o_opt;
+  b.d_src = reinterpret_cast<SourceRec *>(d + o_src);
+  b.d_src_f = reinterpret_cast<SourceRecF *>(d + o_srcf);
+  b.d_cdf = reinterpret_cast<double *>(d + o_cdf);
+  b.d_bcn = reinterpret_cast<double *>(d + o_bcn);
+  b.d_cdf_f = reinterpret_cast<float *>(d + o_cdff);
+  b.d_bctype = d + o_bct;
+  b.d_jc = reinterpret_cast<unsigned long long *>(d + o_res);
+  b.d_ledger = reinterpret_cast<double *>(d + o_res) + kSlots * kJcN;
+  b.d_acc = b.d_ledger + kSlots * kLgN;
   return zero_job(b, st);
 }
 
 int zero_job(JobBuffers &b, cudaStream_t st) {
-  VMC_CK(cudaMemsetAsync(b.d_acc, 0, sizeof(double) * (size_t)(2 * b.Ne + 4 * b.Nb), st));
-  VMC_CK(cudaMemsetAsync(b.d_jc, 0, sizeof(unsigned long long) * kSlots * kJcN, st));
-  VMC_CK(cudaMemsetAsync(b.d_ledger, 0, sizeof(double) * kSlots * kLgN, st));
+  VMC_CK(cudaMemsetAsync(b.d_jc, 0, b.result_bytes(), st));
   return VMC_OK;
 }
 
@@ -328,9 +381,11 @@ template <class T>
 struct DevGuard {
   T *p = nullptr;
   cudaStream_t st = nullptr;
-  int alloc(size_t count, cudaStream_t s) {
+  int alloc(int device, size_t count, cudaStream_t s) {
+    cudaMemPool_t pool = nullptr;
+    VMC_TRY(call_pool(device, &pool));
     st = s;
-    VMC_CK(cudaMallocAsync(reinterpret_cast<void **>(&p), (count ? count : 1) * sizeof(T), s));
+    VMC_CK(pool_alloc(reinterpret_cast<void **>(&p), (count ? count : 1) * sizeof(T), pool, s));
     return VMC_OK;
   }
   ~DevGuard() {
@@ -496,7 +551,7 @@ int capture_launch(cudaStream_t cap, const LaunchPlan &p, void **args, Ctl *dctl
 }  // namespace
 
 int launch_jobs(int device, const LaunchSpec &spec, const std::vector<JobDev> &jobs_in, const vmc_options *opt,
-                cudaStream_t st, LaunchResult &res) {
+                cudaStream_t st, LaunchResult &res, const std::function<void()> &meanwhile) {
   LaunchPlan plan;
   VMC_TRY(plan_launch(device, spec, jobs_in, plan, res));
   const std::vector<JobDev> &jobs = plan.jobs;
@@ -505,17 +560,24 @@ int launch_jobs(int device, const LaunchSpec &spec, const std::vector<JobDev> &j
   const void *fn = plan.fn;
   const int grid = plan.grid, block = plan.block;
   const size_t smem = plan.smem;
-  if (total == 0) return VMC_OK;
+  if (total == 0) {
+    if (meanwhile) meanwhile();
+    return VMC_OK;
+  }
 
-  DevGuard<JobDev> djobs;
-  DevGuard<int64_t> dbegin;
-  DevGuard<Ctl> dctl;
-  VMC_TRY(djobs.alloc(jobs.size(), st));
-  VMC_TRY(dbegin.alloc(begin.size(), st));
-  VMC_TRY(dctl.alloc(1, st));
-  VMC_TRY(h2d(djobs.p, jobs.data(), jobs.size(), st));
-  VMC_TRY(h2d(dbegin.p, begin.data(), begin.size(), st));
-  VMC_CK(cudaMemsetAsync(dctl.p, 0, sizeof(Ctl), st));
+  // control block, photon prefix and job table in one copy
+  constexpr size_t kBegin = (sizeof(Ctl) + 15) & ~(size_t)15;
+  const size_t o_jobs = (kBegin + begin.size() * sizeof(int64_t) + 15) & ~(size_t)15;
+  const size_t table_bytes = o_jobs + jobs.size() * sizeof(JobDev);
+  std::vector<unsigned char> table(table_bytes, 0);
+  memcpy(table.data() + kBegin, begin.data(), begin.size() * sizeof(int64_t));
+  memcpy(table.data() + o_jobs, jobs.data(), jobs.size() * sizeof(JobDev));
+  DevGuard<unsigned char> dtable;
+  VMC_TRY(dtable.alloc(device, table_bytes, st));
+  VMC_TRY(h2d(dtable.p, table.data(), table_bytes, st));
+  struct { Ctl *p; } dctl{reinterpret_cast<Ctl *>(dtable.p)};
+  struct { const int64_t *p; } dbegin{reinterpret_cast<const int64_t *>(dtable.p + kBegin)};
+  struct { const JobDev *p; } djobs{reinterpret_cast<const JobDev *>(dtable.p + o_jobs)};
   LaunchParams lp = make_params(spec, plan, djobs.p, dbegin.p, dctl.p);
   EventGuard e0, e1;
   VMC_CK(cudaEventCreate(&e0.e));
@@ -541,6 +603,7 @@ int launch_jobs(int device, const LaunchSpec &spec, const std::vector<JobDev> &j
     VMC_CK(cudaStreamWaitEvent(st, e1.e, 0));
   }
 
+  if (meanwhile) meanwhile();
   const bool poll = opt && (opt->progress || opt->cancel || opt->timeout_s > 0);
   int status = VMC_OK;
   if (poll) {
@@ -683,18 +746,33 @@ int launch_finish(LaunchArena &a, cudaStream_t st, LaunchResult &res) {
   return VMC_OK;
 }
 
+void touch_results(const HostMesh &m, const JobBuffers &b, const vmc_output *out, Raw<double> &back) {
+  if (back.size() < b.result_bytes() / sizeof(double)) back.resize(b.result_bytes() / sizeof(double));
+  struct Span { double *p; int64_t n; };
+  const Span spans[] = {{back.data(), (int64_t)back.size()}, {out->ER, m.Ne}, {out->EI, m.Ne}, {out->EBR, m.Nb},
+                        {out->EBI, m.Nb}, {out->DEBR, m.Nb}, {out->DEBI, m.Nb}};
+  constexpr int64_t kStride = 4096 / sizeof(double);
+  for (const Span &s : spans) {
+    if (!s.p) continue;
+    volatile double *p = s.p;  // each page written with what it holds
+#pragma omp parallel for schedule(static) if (s.n > 100000)
+    for (int64_t i = 0; i < s.n; i += kStride) p[i] = p[i];
+    if (s.n > 0) p[s.n - 1] = p[s.n - 1];
+  }
+}
+
 int collect_job(const HostJob &j, const DeviceMesh &m, const JobBuffers &b, int64_t nphoton, bool normalize,
-                vmc_output *out, vmc_stats *st, cudaStream_t stream) {
+                vmc_output *out, vmc_stats *st, cudaStream_t stream, Raw<double> &back) {
   const int64_t Ne = m.host.Ne, Nb = m.host.Nb;
-  std::vector<double> acc((size_t)(2 * Ne + 4 * Nb));
-  std::vector<unsigned long long> jc((size_t)kSlots * kJcN);
-  std::vector<double> lg((size_t)kSlots * kLgN);
-  VMC_CK(cudaMemcpyAsync(acc.data(), b.d_acc, acc.size() * 8, cudaMemcpyDeviceToHost, stream));
-  VMC_CK(cudaMemcpyAsync(jc.data(), b.d_jc, jc.size() * 8, cudaMemcpyDeviceToHost, stream));
-  VMC_CK(cudaMemcpyAsync(lg.data(), b.d_ledger, lg.size() * 8, cudaMemcpyDeviceToHost, stream));
+  const size_t bytes = b.result_bytes();
+  if (back.size() < bytes / sizeof(double)) back.resize(bytes / sizeof(double));
+  VMC_CK(cudaMemcpyAsync(back.data(), b.d_jc, bytes, cudaMemcpyDeviceToHost, stream));
   VMC_CK(cudaStreamSynchronize(stream));
-  g_d2h_bytes += (int64_t)(acc.size() + jc.size() + lg.size()) * 8;
-  const double *ER = acc.data(), *EI = ER + Ne, *EBR = EI + Ne, *EBI = EBR + Nb, *DEBR = EBI + Nb, *DEBI = DEBR + Nb;
+  g_d2h_bytes += (int64_t)bytes;
+  unsigned long long jc[kSlots * kJcN];
+  memcpy(jc, back.data(), sizeof(jc));
+  const double *lg = back.data() + kSlots * kJcN;
+  const double *ER = lg + kSlots * kLgN, *EI = ER + Ne, *EBR = EI + Ne, *EBI = EBR + Nb, *DEBR = EBI + Nb, *DEBI = DEBR + Nb;
   if (out) normalise(m.host, j, nphoton, ER, EI, EBR, EBI, DEBR, DEBI, out, normalize);
   if (st) {
     unsigned long long c[kJcN] = {0};
@@ -710,8 +788,17 @@ int collect_job(const HostJob &j, const DeviceMesh &m, const JobBuffers &b, int6
     if (c[kJcTapeEnd]) st->status_detail |= kErrTapeEnd;
     double absorbed = 0, exited = 0;
     if (j.omega <= 0.0) {
-      for (int64_t i = 0; i < Ne; i++)
-        if (j.mua[(size_t)i] > 0.0) absorbed += ER[i];
+      // in blocks of fixed size, so that the sum does not depend on the number of threads
+      constexpr int64_t kBlock = 8192;
+      std::vector<double> part((size_t)((Ne + kBlock - 1) / kBlock), 0.0);
+#pragma omp parallel for schedule(static) if (Ne > 100000)
+      for (int64_t q = 0; q < (int64_t)part.size(); q++) {
+        double a = 0;
+        for (int64_t i = q * kBlock; i < std::min(Ne, (q + 1) * kBlock); i++)
+          if (j.mua_of(i) > 0.0) a += ER[i];
+        part[(size_t)q] = a;
+      }
+      for (double a : part) absorbed += a;
       for (int64_t i = 0; i < Nb; i++) exited += EBR[i];
     } else {
       absorbed = exited = NAN;
@@ -804,7 +891,7 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   DeviceMesh dm;
   dm.device = o.device;
   const int mask = o.precision == VMC_FP64 ? 1 : 2;
-  s = build_mesh(in, mask, dm.host);
+  s = build_mesh(in, mask, dm.host, false);
   if (s) return s;
   HostJob hj;
   s = build_job(in, dm.host, hj);
@@ -820,7 +907,7 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   VMC_CK(cudaStreamCreateWithFlags(&call_stream.s, cudaStreamNonBlocking));
   cudaStream_t stream = call_stream.s;
   cudaMemPool_t call_pool = nullptr;
-  VMC_CK(cudaDeviceGetDefaultMemPool(&call_pool, o.device));
+  VMC_TRY(vmc::call_pool(o.device, &call_pool));
   dm.pool = call_pool;
   dm.st = stream;
   s = upload_mesh(dm, mask);
@@ -869,7 +956,9 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   spec.stage_slots = o.stage_slots;
   spec.refill = o.refill_lanes;
   LaunchResult lr;
-  int ls = launch_jobs(o.device, spec, std::vector<JobDev>{d}, &o, stream, lr);
+  Raw<double> back;
+  int ls = launch_jobs(o.device, spec, std::vector<JobDev>{d}, &o, stream, lr,
+                       [&] { touch_results(dm.host, jb, out, back); });
   if (ls != VMC_OK && ls != VMC_ERR_CANCELLED && ls != VMC_ERR_TIMEOUT) return ls;
   st->photons_requested = in->Nphoton;
   st->photons_done = (int64_t)lr.done;
@@ -879,7 +968,7 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   st->seconds_kernel = lr.kernel_ms * 1e-3;
   st->grid_blocks = lr.grid;
   st->block_size = lr.block;
-  s = collect_job(hj, dm, jb, in->Nphoton, o.normalize != 0 || !opt_in, out, st, stream);
+  s = collect_job(hj, dm, jb, in->Nphoton, o.normalize != 0 || !opt_in, out, st, stream, back);
   if (s) return s;
   if (ntr > 0) {
     VMC_CK(cudaMemcpyAsync(o.trace, jb.d_trace, sizeof(int64_t) * (size_t)(ntr * o.trace_stride),
@@ -907,16 +996,14 @@ int vmc_mesh_create(const vmc_input *geometry, int32_t precision, int32_t device
   if ((geometry->Ne && !geometry->H) || (geometry->Nb && !geometry->BH) || (geometry->Nr && !geometry->r))
     return VMC_ERR_INVALID_ARGUMENT;
   const int64_t nh = geometry->Ne * (geometry->dim + 1), nb = geometry->Nb * geometry->dim;
-  for (int64_t i = 0; i < nh; i++)
-    if (geometry->H[i] < 0 || geometry->H[i] >= geometry->Nr) return VMC_INCONSISTENT_H;
-  for (int64_t i = 0; i < nb; i++)
-    if (geometry->BH[i] < 0 || geometry->BH[i] >= geometry->Nr) return VMC_INCONSISTENT_BH;
+  if (!nodes_in_range(geometry->H, nh, geometry->Nr)) return VMC_INCONSISTENT_H;
+  if (!nodes_in_range(geometry->BH, nb, geometry->Nr)) return VMC_INCONSISTENT_BH;
   int s = select_device(device);
   if (s) return s;
   std::unique_ptr<vmc_mesh> m(new vmc_mesh);
   m->m.device = device;
   const int mask = precision == VMC_FP64 ? 1 : 2;
-  s = build_mesh(geometry, mask, m->m.host);
+  s = build_mesh(geometry, mask, m->m.host, true);
   if (s) return s;
   s = upload_mesh(m->m, mask);
   if (s) return s;
@@ -960,10 +1047,8 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
     if (!mm || !(mm->precision_mask & mask)) return VMC_ERR_INVALID_ARGUMENT;
     vmc_input in = jobs[i];
     // geometry comes from the mesh
-    in.dim = mm->m.host.dim; in.Ne = mm->m.host.Ne; in.Nb = mm->m.host.Nb; in.Nr = mm->m.host.Nr;
-    in.H = mm->m.host.H.data(); in.BH = mm->m.host.BH.data(); in.r = mm->m.host.r.data();
-    in.HN = nullptr; in.n_HN = 0;
-    s = check_input(&in);
+    use_mesh(in, mm->m.host);
+    s = check_input(&in, false);
     if (s) return s;
     s = build_job(&in, mm->m.host, hj[(size_t)i]);
     if (s) return s;
@@ -974,7 +1059,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
   VMC_CK(cudaStreamCreateWithFlags(&call_stream.s, cudaStreamNonBlocking));
   cudaStream_t stream = call_stream.s;
   cudaMemPool_t call_pool = nullptr;
-  VMC_CK(cudaDeviceGetDefaultMemPool(&call_pool, o.device));
+  VMC_TRY(vmc::call_pool(o.device, &call_pool));
   // group by launch class
   struct Group { LaunchSpec spec; std::vector<int> idx; };
   std::vector<Group> groups;
@@ -999,6 +1084,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
   memset(&tot, 0, sizeof(tot));
   auto t1 = std::chrono::steady_clock::now();
   double kernel_s = 0;
+  Raw<double> back;
   for (auto &g : groups) {
     std::vector<JobDev> descs;
     for (int i : g.idx) {
@@ -1014,7 +1100,9 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
       descs.push_back(d);
     }
     LaunchResult lr;
-    int ls = launch_jobs(o.device, g.spec, descs, &o, stream, lr);
+    int ls = launch_jobs(o.device, g.spec, descs, &o, stream, lr, [&] {
+      for (int i : g.idx) touch_results(meshes[i]->m.host, *jb[(size_t)i], &outs[i], back);
+    });
     if (ls != VMC_OK) return ls;
     kernel_s += lr.kernel_ms * 1e-3;
     tot.steps += (int64_t)lr.steps;
@@ -1029,7 +1117,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
       js.photons_done = std::max<int64_t>(0, jobs[i].Nphoton);
       js.seed_used = hj[(size_t)i].seed;
       s = collect_job(hj[(size_t)i], meshes[i]->m, *jb[(size_t)i], jobs[i].Nphoton, o.normalize != 0 || !opt_in,
-                      &outs[i], &js, stream);
+                      &outs[i], &js, stream, back);
       if (s) return s;
       tot.photons_requested += jobs[i].Nphoton;
       tot.loss += js.loss;

@@ -57,7 +57,7 @@ struct Request {
   bool retiring = false;
   Clock::time_point t_submit, t_admit, t_finish;
   double kernel_s = 0;
-  std::vector<double> ER, EI, EBR, EBI, DEBR, DEBI;
+  Raw<double> ER, EI, EBR, EBI, DEBR, DEBI;
   vmc_stats stats;
 };
 
@@ -357,6 +357,7 @@ void vmc_server::collect_loop() {
   cudaSetDevice(cfg.device);
   cudaStream_t st = nullptr;
   cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  Raw<double> back;
   for (;;) {
     Request *r = nullptr;
     {
@@ -379,7 +380,7 @@ void vmc_server::collect_loop() {
     r->stats.photons_requested = r->nphoton;
     r->stats.photons_done = r->issued;
     r->stats.seed_used = r->job.seed;
-    r->status = collect_job(r->job, *m, *r->buf, r->nphoton, true, &o, &r->stats, st);
+    r->status = collect_job(r->job, *m, *r->buf, r->nphoton, true, &o, &r->stats, st, back);
     finalize(r);
   }
   cudaStreamDestroy(st);
@@ -453,13 +454,12 @@ int vmc_server_submit(vmc_server *s, int32_t mesh_id, const vmc_input *job, int6
   std::unique_ptr<Request> r(new Request);
   memset(&r->stats, 0, sizeof(r->stats));
   vmc_input in = *job;
-  in.dim = m->host.dim; in.Ne = m->host.Ne; in.Nb = m->host.Nb; in.Nr = m->host.Nr;
-  in.H = m->host.H.data(); in.BH = m->host.BH.data(); in.r = m->host.r.data();
-  in.HN = nullptr; in.n_HN = 0;
-  int st = check_input(&in);
+  use_mesh(in, m->host);
+  int st = check_input(&in, false);
   if (st) return st;
   st = build_job(&in, m->host, r->job);
   if (st) return st;
+  r->job.keep();  // the caller's arrays may go before the request is admitted
   r->job.seed = in.seed_given ? in.seed : clock_seed();
   r->literal = s->cfg.precision == VMC_FP64 && rough_optics(&in, m->host);
   r->mesh_id = mesh_id;
@@ -478,8 +478,8 @@ int vmc_server_submit(vmc_server *s, int32_t mesh_id, const vmc_input *job, int6
 static int take_result(Request *r, vmc_output *out, vmc_stats *stats) {
   if (r->state == kFailed) return -r->status;
   if (out) {
-    auto cp = [](double *dst, const std::vector<double> &v) {
-      if (dst && !v.empty()) memcpy(dst, v.data(), v.size() * sizeof(double));
+    auto cp = [](double *dst, const Raw<double> &v) {
+      if (dst && v.size()) memcpy(dst, v.data(), v.size() * sizeof(double));
     };
     cp(out->ER, r->ER); cp(out->EI, r->EI); cp(out->EBR, r->EBR); cp(out->EBI, r->EBI);
     cp(out->DEBR, r->DEBR); cp(out->DEBI, r->DEBI);

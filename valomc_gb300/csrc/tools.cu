@@ -150,10 +150,8 @@ int vmc_autotune(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs, 
     DeviceMesh *m = mesh_impl(meshes[i]);
     if (!m || !(mesh_precision_mask(meshes[i]) & mask)) return VMC_ERR_INVALID_ARGUMENT;
     vmc_input in = jobs[i];
-    in.dim = m->host.dim; in.Ne = m->host.Ne; in.Nb = m->host.Nb; in.Nr = m->host.Nr;
-    in.H = m->host.H.data(); in.BH = m->host.BH.data(); in.r = m->host.r.data();
-    in.HN = nullptr; in.n_HN = 0;
-    s = check_input(&in);
+    use_mesh(in, m->host);
+    s = check_input(&in, false);
     if (s) return s;
     s = build_job(&in, m->host, hj[(size_t)i]);
     if (s) return s;
