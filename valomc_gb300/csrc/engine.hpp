@@ -13,6 +13,9 @@ namespace vmc {
 
 void set_error(const std::string &msg);
 int cuda_status(cudaError_t e, const char *what);
+// bytes this thread's call has copied to and from the device
+extern thread_local int64_t g_h2d_bytes, g_d2h_bytes;
+
 #define VMC_CK(call)                                      \
   do {                                                    \
     cudaError_t _e = (call);                              \
@@ -38,6 +41,17 @@ struct DeviceMesh {
   const void *geom(int precision) const { return d_geom[precision]; }
 };
 int upload_mesh(DeviceMesh &m, int precision_mask);
+// The same from the input's arrays with neighbours and records made on the device (m.device is
+// current, m.st and m.pool are set).  keep_HN: the host gets HN too.  Out of memory leaves nothing
+// on the device, and the host can build.
+int build_mesh_on_device(const vmc_input *in, int precision_mask, DeviceMesh &m, bool own, bool keep_HN);
+// Whether that pays.  A call with one photon takes on the host / with the device, in ms: 0.33 /
+// 0.35 at 800 triangles in FP64 (0.33 / 0.30 in FP32), 0.40 / 0.37 at 1250 (0.40 / 0.31), 1.45 /
+// 0.64 at 20000; 0.61 / 0.40 at 750 tetrahedra, 11.0 / 2.1 at 162k, 95 / 32 at 1.3M: launches and
+// copies cost 0.1 ms, the host's search some 50 ns a face on its 16 cores and its records 5 more.
+// Above 2^26 elements the scratch of 90 bytes an element could be what a mesh that fits by itself
+// lacks.
+inline bool builds_on_device(int64_t Ne) { return Ne >= 1000 && Ne <= (int64_t)1 << 26; }
 // TetRec / TriRec [Ne] at `geom` from the Tet64 / Tri64 [Ne] behind them
 cudaError_t make_plane_records(int dim, void *geom, int64_t Ne, cudaStream_t st);
 

@@ -254,7 +254,7 @@ static void copy_of(Raw<T> &to, const T *from, size_t n) {
   for (size_t i = 0; i < n; i++) to[i] = from[i];
 }
 
-int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own) {
+int take_geometry(const vmc_input *in, HostMesh &m, bool own) {
   const int D = in->dim, NF = D + 1;
   m.dim = D; m.Ne = in->Ne; m.Nb = in->Nb; m.Nr = in->Nr;
   if (m.Ne >= (int64_t)kOpenFace || m.Nb >= (int64_t)kOpenFace) return VMC_ERR_SIZE_LIMIT;
@@ -265,14 +265,12 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own) {
     copy_of(m.own_r, in->r, (size_t)(m.Nr * D));
     m.H = m.own_H.data(); m.BH = m.own_BH.data(); m.r = m.own_r.data();
   }
-  if (in->HN && in->n_HN == in->Ne) {  // MC3D.hpp:839: a neighbourhood of the right size is used as given
-    copy_of(m.HN, in->HN, (size_t)(m.Ne * NF));
-  } else {
-    m.HN.resize((size_t)(m.Ne * NF));
-    int s = build_neighbours(D, m.Ne, m.Nb, m.Nr, m.H, m.BH, m.HN.data());
-    if (s) return s;
-  }
-  // the faces on the boundary, for the light sources of every job on the mesh
+  return VMC_OK;
+}
+
+// the faces on the boundary, for the light sources of every job on the mesh
+void list_boundary_faces(HostMesh &m) {
+  const int NF = m.dim + 1;
   m.faces.clear();
   m.faces.reserve((size_t)m.Nb);
 #pragma omp parallel if (m.Ne > 20000)
@@ -291,20 +289,49 @@ int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own) {
 #pragma omp critical
     m.faces.insert(m.faces.end(), mine.begin(), mine.end());
   }
+}
+
+void sort_faces(HostMesh &m) {
   std::sort(m.faces.begin(), m.faces.end(),
             [](const BoundaryFace &a, const BoundaryFace &b) { return a.el != b.el ? a.el < b.el : a.f < b.f; });
+}
+
+void measure_boundary(HostMesh &m) {
   Geo G{m.H, m.BH, m.r, m.Ne, m.Nb, m.Nr};
-  m.volume.resize((size_t)m.Ne);
   m.area.resize((size_t)m.Nb);
   m.bnorm.assign((size_t)m.Nb * 4, 0.0);
-#pragma omp parallel for schedule(static) if (m.Ne > 20000)
-  for (int64_t i = 0; i < m.Ne; i++) m.volume[(size_t)i] = D == 3 ? volume3(G, i) : area2(G, i);
 #pragma omp parallel for schedule(static) if (m.Nb > 10000)
   for (int64_t i = 0; i < m.Nb; i++) {
-    m.area[(size_t)i] = D == 3 ? area3(G, i) : length2(G, i);
-    if (D == 3) normal_b3(G, i, &m.bnorm[(size_t)i * 4]);
+    m.area[(size_t)i] = m.dim == 3 ? area3(G, i) : length2(G, i);
+    if (m.dim == 3) normal_b3(G, i, &m.bnorm[(size_t)i * 4]);
     else normal_b2(G, i, &m.bnorm[(size_t)i * 4]);
   }
+}
+
+void measure_elements(HostMesh &m) {
+  if (m.volume.size() == (size_t)m.Ne) return;
+  Geo G{m.H, m.BH, m.r, m.Ne, m.Nb, m.Nr};
+  m.volume.resize((size_t)m.Ne);
+#pragma omp parallel for schedule(static) if (m.Ne > 20000)
+  for (int64_t i = 0; i < m.Ne; i++) m.volume[(size_t)i] = m.dim == 3 ? volume3(G, i) : area2(G, i);
+}
+
+int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own) {
+  const int D = in->dim, NF = D + 1;
+  int s = take_geometry(in, m, own);
+  if (s) return s;
+  if (in->HN && in->n_HN == in->Ne) {  // MC3D.hpp:839: a neighbourhood of the right size is used as given
+    copy_of(m.HN, in->HN, (size_t)(m.Ne * NF));
+  } else {
+    m.HN.resize((size_t)(m.Ne * NF));
+    s = build_neighbours(D, m.Ne, m.Nb, m.Nr, m.H, m.BH, m.HN.data());
+    if (s) return s;
+  }
+  list_boundary_faces(m);
+  sort_faces(m);
+  measure_boundary(m);
+  measure_elements(m);
+  Geo G{m.H, m.BH, m.r, m.Ne, m.Nb, m.Nr};
   auto nbr32 = [&](int64_t el, int f) -> int32_t {
     int64_t h = m.HN[(size_t)(el + m.Ne * f)];
     if (h >= m.Ne || h < -m.Nb) return kOpenFace;  // INT64_MAX open face, or an invalid given HN

@@ -117,6 +117,13 @@ int build_neighbours(int dim, int64_t Ne, int64_t Nb, int64_t Nr, const int64_t 
 // bit 0 builds the FP64 records, bit 1 the FP32 records.  own: the mesh outlives the input's
 // arrays and copies them.
 int build_mesh(const vmc_input *in, int precision_mask, HostMesh &m, bool own);
+// Its parts, for a mesh whose neighbours and records are made on the device: sizes and arrays, the
+// boundary's areas and normals, the order of the faces, the elements' volumes.
+int take_geometry(const vmc_input *in, HostMesh &m, bool own);
+void measure_boundary(HostMesh &m);
+void list_boundary_faces(HostMesh &m);  // from HN, in any order
+void sort_faces(HostMesh &m);
+void measure_elements(HostMesh &m);
 
 // Job from the problem arrays of an input on mesh m (Init's light sources, BCLNormal
 // processing and wave numbers).  The job reads the input's optics arrays until keep().

@@ -891,7 +891,16 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   DeviceMesh dm;
   dm.device = o.device;
   const int mask = o.precision == VMC_FP64 ? 1 : 2;
-  s = build_mesh(in, mask, dm.host, false);
+  // (without a device the host's checks of the mesh still come first)
+  const bool on_device = builds_on_device(in->Ne) && select_device(o.device) == VMC_OK;
+  s = VMC_ERR_OUT_OF_MEMORY;
+  if (on_device) {
+    VMC_CK(cudaStreamCreateWithFlags(&call_stream.s, cudaStreamNonBlocking));
+    VMC_TRY(vmc::call_pool(o.device, &dm.pool));
+    dm.st = call_stream.s;
+    s = build_mesh_on_device(in, mask, dm, false, out->HN || o.precision == VMC_FP64);
+  }
+  if (s == VMC_ERR_OUT_OF_MEMORY) s = build_mesh(in, mask, dm.host, false);
   if (s) return s;
   HostJob hj;
   s = build_job(in, dm.host, hj);
@@ -904,12 +913,13 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   // every host-side check of ErrorChecks / Init has passed: now the device
   s = select_device(o.device);
   if (s) return s;
-  VMC_CK(cudaStreamCreateWithFlags(&call_stream.s, cudaStreamNonBlocking));
+  if (!on_device) {
+    VMC_CK(cudaStreamCreateWithFlags(&call_stream.s, cudaStreamNonBlocking));
+    VMC_TRY(vmc::call_pool(o.device, &dm.pool));
+    dm.st = call_stream.s;
+  }
   cudaStream_t stream = call_stream.s;
-  cudaMemPool_t call_pool = nullptr;
-  VMC_TRY(vmc::call_pool(o.device, &call_pool));
-  dm.pool = call_pool;
-  dm.st = stream;
+  const cudaMemPool_t call_pool = dm.pool;
   s = upload_mesh(dm, mask);
   if (s) return s;
   JobBuffers jb;
@@ -958,7 +968,10 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   LaunchResult lr;
   Raw<double> back;
   int ls = launch_jobs(o.device, spec, std::vector<JobDev>{d}, &o, stream, lr,
-                       [&] { touch_results(dm.host, jb, out, back); });
+                       [&] {
+                         touch_results(dm.host, jb, out, back);
+                         measure_elements(dm.host);
+                       });
   if (ls != VMC_OK && ls != VMC_ERR_CANCELLED && ls != VMC_ERR_TIMEOUT) return ls;
   st->photons_requested = in->Nphoton;
   st->photons_done = (int64_t)lr.done;
@@ -1003,7 +1016,16 @@ int vmc_mesh_create(const vmc_input *geometry, int32_t precision, int32_t device
   std::unique_ptr<vmc_mesh> m(new vmc_mesh);
   m->m.device = device;
   const int mask = precision == VMC_FP64 ? 1 : 2;
-  s = build_mesh(geometry, mask, m->m.host, true);
+  s = VMC_ERR_OUT_OF_MEMORY;
+  if (builds_on_device(geometry->Ne)) {
+    StreamGuard st;
+    VMC_CK(cudaStreamCreateWithFlags(&st.s, cudaStreamNonBlocking));
+    m->m.st = st.s;
+    s = build_mesh_on_device(geometry, mask, m->m, true, true);
+    m->m.st = nullptr;
+    if (s == VMC_OK) measure_elements(m->m.host);
+  }
+  if (s == VMC_ERR_OUT_OF_MEMORY) s = build_mesh(geometry, mask, m->m.host, true);
   if (s) return s;
   s = upload_mesh(m->m, mask);
   if (s) return s;
