@@ -77,3 +77,18 @@ def test_jobs_of_both_fp64_walks_share_a_batch(built, dim):
             a, b = getattr(r, k), getattr(ref, k)
             assert np.abs(a - b).sum() <= 1e-6 * np.abs(b).sum(), k
     mesh.close()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("g", [0.02, -0.9, 0.9995, -0.9995])
+def test_scattering_angles_at_the_ends_of_fixed_point(built, dim, g):
+    """|g| above 0.999 leaves the fixed-point angles for FP64 ones."""
+    p = problem(dim, "slivers", False, 0.0)
+    p.g[:] = g
+    gpu = V.run(p, precision=V.VMC_FP64)
+    ref = oracle.run(p, rng=oracle.RNG_PHILOX, nthreads=4)
+    assert gpu.stats["photons_done"] == p.Nphoton and gpu.stats["loss"] == ref.loss
+    assert gpu.stats["steps"] == ref.steps
+    for k in ("ER", "EBR"):
+        a, b = getattr(gpu, k), getattr(ref, k)
+        assert np.abs(a - b).sum() <= 1e-6 * np.abs(b).sum(), k

@@ -138,19 +138,22 @@ __device__ __forceinline__ float free_path_f(float u, float mus) {
 // Bound by the FP64 pipe, which starts one warp instruction in about 19 cycles of the SM; with
 // the reference's operation sequence taken literally a warp's step needed about 450 of them
 // (Moller-Trumbore face by face, the library's exp, log, sin, cos, sqrt and divisions).  Here
-// FP64 is spent where the state is: about 25 operations for the step and 45 for a scatter.
+// FP64 is spent where the state is: 25 operations for a step of which 1 belongs to the scatter.
 //   exit face  picked in FP32 from planes about vertex 0, when it is certain by margins above
 //              every FP32 rounding; else (2e-4 of the steps) by Moller-Trumbore, face by face as
 //              in the reference.  Its distance is one FP64 quotient n . (v - p) / n . d, with no
 //              more rounding than Moller-Trumbore's.
-//   samples    log, sine, cosine and the deposit's factor on the integer pipe (fixed64.hpp).
+//   samples    log, sine, cosine, the deposit's factor, the scattering angle and the turned
+//              direction on the integer pipe (fixed64.hpp); the last two by 48 FP64 operations of
+//              3D before (23 in 2D), with errors 3 to 100 times as large.
 //   quotients and roots from FP32 first values.
-// 1e5 photons on the phantom 313 -> 102 ms (571 before lanes were packed as well), 1e6 on the 2D
-// square 38.7 -> 9.0 ms, a 2304-tet frequency-domain box 19.5 -> 7.7 ms.  The square keeps the FP64
-// pipe 74 % busy; the phantom's run ends in walks of 12 000 steps, 4 us each.
+// 1e5 photons on the phantom 313 -> 102 -> 79 ms (571 before lanes were packed as well), 1e3 there
+// 46.8 -> 39.4, 20 000 in the 48k-tet cube 33.7 -> 27.4 (the middle figures with the scatter in
+// FP64).  The phantom's run ends in walks of 14 000 steps, with the issue slots 14 % and the FP64
+// pipe 14 % busy: the latency of some 1000 instructions a step.
 template <bool FD, class R>
 struct Walk3D64 {
-  static constexpr bool kBuffered = false;  // words left in a block are carried from step to step
+  static constexpr bool kBuffered = false;  // a block's words are drawn again rather than carried
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = true;
   static constexpr int kMinBlocks = 2;
@@ -211,41 +214,74 @@ struct Walk3D64 {
     return false;
   }
 
-  // What a scatter event draws: the polar cosine and sine, the azimuth's, the free path after it.
-  struct Event { double ct, st, cp, sp, path; };
+  // What a scatter event draws: the polar cosine and sine, the azimuth's (in units of 2^-60), the
+  // free path after it.
+  struct Event { int64_t ct, st, cp, sp; double path; };
 
   // ScatterPhoton, MC3D.hpp:1297-1315, from the words u, without the round trip through the
   // angle: the reference draws theta = acos(c) from the HG inverse CDF c and takes sin and cos
   // of it; here cos theta is c itself and sin theta = sqrt(1 - c^2) (|c| > 1 from rounding at
-  // the CDF's ends gives a NaN sine, as acos gives a NaN angle).  Drawn before the exit face is
-  // looked for, whether the step ends in a scatter or not: nearly every step of a warp has one,
-  // and the two chains of FP64 operations, each waiting some 75 cycles a link, overlap.
+  // the CDF's ends gives a NaN sine, as acos gives a NaN angle).
   __device__ __forceinline__ Event draw_event(uint3 u) const {
     Event e;
-    const double c0 = fma(word_d(u.x), 2.0 / 4294967295.0, -1.0);  // 2 xi - 1, the isotropic cosine
-    const double D = fma(g, c0, 1.0);                              // 1 - g (1 - 2 xi)
-    const double q = div_near(fma(-g, g, 1.0), D, f32_of(D));
-    double ct = fma(-q, q, fma(g, g, 1.0)) * ig;
-    ct = u.x == 0u ? -1.0 : u.x == 0xffffffffu ? 1.0 : ct;  // theta = (1 - xi) pi at xi in {0, 1}
-    ct = (__double_as_longlong(g) << 1) == 0 ? c0 : ct;
-    e.ct = ct;
-    const double s2 = fma(-ct, ct, 1.0);
-    const float s2f = f32_of(s2);
-    double y;
-    sqrt_near(s2, s2f, e.st, y);
-    e.st = s2f > 0.0f ? e.st : s2f == 0.0f ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
+    e.ct = hg_cosine(u.x, g, ig);
+    const Split60 c = split60(e.ct);
+    const int64_t s2 = kOne60 - mul60(c, c);
+    const Root60 s = sqrt60(s2);
+    e.st = s2 > 0 ? s.r >> s.k : 0;
+    if (s2 < 0) e.ct = kNoCosine;
     // the azimuth 2 pi u / (2^32 - 1): u 2^32 + u in 2^-64 turns, to one of them
-    sincos_turn(((uint64_t)u.y << 32) | u.y, e.sp, e.cp);
+    sincos_turn_fixed(((uint64_t)u.y << 32) | u.y, e.sp, e.cp);
+    e.sp >>= 2;
+    e.cp >>= 2;
     e.path = neg_log_open(u.z) * imus;
     return e;
   }
 
-  // the rotation of ScatterPhoton, MC3D.hpp:1316-1340
-  __device__ __forceinline__ void rotate(const Event &e) {
-    const double ct = e.ct, st = e.st, cp = e.cp, sp = e.sp;
-    const double dx = dir[0], dy = dir[1], dz = dir[2];
+  // the rotation of ScatterPhoton, MC3D.hpp:1316-1340; false: not for fixed point
+  __device__ __forceinline__ bool rotate(const Event &e) {
+    const uint32_t top = max(mag_of(dir[0]), max(mag_of(dir[1]), mag_of(dir[2])));
+    if (e.ct == kNoCosine || top > 0x3ff00000u) return false;
+    const int64_t z6 = fixed60_of(dir[2]);
+    const Split60 ct = split60(e.ct), st = split60(e.st), cp = split60(e.cp), sp = split60(e.sp), dz = split60(z6);
+    int64_t v[3];
+    if ((__double_as_longlong(dir[2]) & 0x7fffffffffffffffll) > __double_as_longlong(0.999)) {
+      v[0] = mul60(st, cp);
+      v[1] = mul60(st, sp);
+      v[2] = z6 > 0 ? e.ct : -e.ct;
+    } else {
+      const Split60 dx = split60(fixed60_of(dir[0])), dy = split60(fixed60_of(dir[1]));
+      const Root60 q = sqrt60(kOne60 - mul60(dz, dz));  // sqrt(1 - z^2), k <= 4
+      const Split60 isq = split60(q.y), zc = split60(mul60(dz, cp));
+      const Split60 ux = split60(mul60(dx, isq) << q.k), uy = split60(mul60(dy, isq) << q.k);
+      v[0] = dot60(st, split60(dot60(ux, zc, neg60(uy), sp)), dx, ct);
+      v[1] = dot60(st, split60(dot60(uy, zc, ux, sp)), dy, ct);
+      v[2] = dot60(dz, ct, split60(-mul60(st, cp)), split60(q.r >> q.k));
+    }
+    if (!unit60(v, 3)) return false;
+    dir[0] = double_of_60(v[0]); dir[1] = double_of_60(v[1]); dir[2] = double_of_60(v[2]);
+    curface = -1;
+    return true;
+  }
+
+  // Both in FP64, for what fixed point does not hold: |g| near 1 or nearly 0, a direction that is
+  // not a unit vector yet, a cosine beyond 1.
+  struct Dir { double x, y, z; };
+  __device__ __noinline__ static Dir scatter_d(uint32_t ux, uint32_t uy, double g, double ig, double dx, double dy, double dz) {
+    const double c0 = fma(word_d(ux), 2.0 / 4294967295.0, -1.0);  // 2 xi - 1, the isotropic cosine
+    const double D = fma(g, c0, 1.0);                              // 1 - g (1 - 2 xi)
+    const double q = div_near(fma(-g, g, 1.0), D, f32_of(D));
+    double ct = fma(-q, q, fma(g, g, 1.0)) * ig;
+    ct = ux == 0u ? -1.0 : ux == 0xffffffffu ? 1.0 : ct;  // theta = (1 - xi) pi at xi in {0, 1}
+    ct = (__double_as_longlong(g) << 1) == 0 ? c0 : ct;
+    const double t2 = fma(-ct, ct, 1.0);
+    const float t2f = f32_of(t2);
+    double st, y, sp, cp;
+    sqrt_near(t2, t2f, st, y);
+    st = t2f > 0.0f ? st : t2f == 0.0f ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
+    sincos_turn(((uint64_t)uy << 32) | uy, sp, cp);
     double nx, ny, nz;
-    if (fabsf(f32_of(dz)) > 0.9989f && fabs(dz) > 0.999) {
+    if (fabs(dz) > 0.999) {
       nx = st * cp;
       ny = st * sp;
       nz = dz > 0.0 ? ct : -ct;
@@ -259,8 +295,7 @@ struct Walk3D64 {
       nz = fma(-st * cp, sq, dz * ct);
     }
     const double s = unit_scale(fma(nx, nx, fma(ny, ny, nz * nz)));
-    dir[0] = nx * s; dir[1] = ny * s; dir[2] = nz * s;
-    curface = -1;
+    return Dir{nx * s, ny * s, nz * s};
   }
 
   // FresnelPhoton at a face with normal nor, of either orientation and any length
@@ -306,7 +341,7 @@ struct Walk3D64 {
   // 4e-6 |r|_1 |d|_1, and the ray starts clearly inside every other plane but the one it
   // entered by (which the reference does not test): then Moller-Trumbore finds u and v well
   // inside that face, and well outside the others or behind the photon.
-  __device__ __forceinline__ int exit_face(const JobDev &J, R &rng, double &dist, int4 &nbr, Event &ev) const {
+  __device__ __forceinline__ int exit_face(const JobDev &J, R &rng, double &dist, int4 &nbr) const {
     const TetRec *T = recs(J) + el;
     const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
     const double2 a1 = __ldg(reinterpret_cast<const double2 *>(T->v0) + 1);
@@ -340,7 +375,6 @@ struct Walk3D64 {
     const double nr = fma(m2, rz, fma(m1, ry, m0 * rx));
     const float dnf = f32_of(dn);
     dist = div_near((nf == 3 ? a1.y : 0.0) - nr, dn, dnf);
-    ev = draw_event(rng.peek3());
     if (sure && f32_safe(dnf)) return nf;
     const Exit e = which_face(verts(J) + el, pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], curface);
     dist = e.dist;
@@ -351,8 +385,7 @@ struct Walk3D64 {
     if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     double dist;
     int4 nb;
-    Event ev;
-    const int nf = exit_face(J, rng, dist, nb, ev);
+    const int nf = exit_face(J, rng, dist, nb);
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
@@ -387,7 +420,13 @@ struct Walk3D64 {
     bool on = true;
     if (ends) {
       if (positive(mus)) {
-        rotate(ev);
+        const Event ev = draw_event(rng.peek3());
+        if (!rotate(ev)) {
+          const uint3 u = rng.peek3();
+          const Dir d = scatter_d(u.x, u.y, g, ig, dir[0], dir[1], dir[2]);
+          dir[0] = d.x; dir[1] = d.y; dir[2] = d.z;
+          curface = -1;
+        }
         rng.take(3);
         prop = ev.path;
         n_scat++;
@@ -761,7 +800,7 @@ struct Walk3D32 {
   // per SM beat 24 (+7% on the 648k-tet phantom); 5 CTAs (48 registers) spill and lose
   static constexpr int kMinBlocks = 4;
   static constexpr bool kStaged = !FD;
-  static constexpr bool kBuffered = false;  // words left in a block are carried from step to step
+  static constexpr bool kBuffered = false;  // a block's words are drawn again rather than carried
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = true;
   using Tr = typename TraceFor<R>::type;
