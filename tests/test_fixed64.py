@@ -28,9 +28,9 @@ extern "C" void rcp(const uint64_t *d, uint64_t *y, long n) { for (long i = 0; i
 extern "C" void root(const int64_t *s, int64_t *r, int64_t *y, int32_t *k, long n) {
   for (long i = 0; i < n; i++) { const vmc::Root60 q = vmc::sqrt60(s[i]); r[i] = q.r; y[i] = q.y; k[i] = q.k; }
 }
-extern "C" void hg(const uint32_t *u, const double *g, const double *ig, int64_t *c, long n) { for (long i = 0; i < n; i++) c[i] = vmc::hg_cosine(u[i], g[i], ig[i]); }
-extern "C" void turn2(const uint32_t *u, const double *g, const double *kg, int64_t *c, int64_t *s, int32_t *ok, long n) {
-  for (long i = 0; i < n; i++) ok[i] = vmc::turn_2d(u[i], g[i], kg[i], c[i], s[i]);
+extern "C" void hg(const uint32_t *u, const double *g, int64_t *c, long n) { for (long i = 0; i < n; i++) c[i] = vmc::hg_cosine(u[i], g[i], vmc::hg_inverse(g[i])); }
+extern "C" void turn2(const uint32_t *u, const double *g, int64_t *c, int64_t *s, int32_t *ok, long n) {
+  for (long i = 0; i < n; i++) ok[i] = vmc::turn_2d(u[i], g[i], vmc::turn_ratio(g[i]), c[i], s[i]);
 }
 extern "C" void unit(int64_t *v, int32_t *ok, long n) { for (long i = 0; i < n; i++) ok[i] = vmc::unit60(v + 3 * i, 3); }
 """
@@ -153,21 +153,19 @@ def test_henyey_greenstein_cosine(lib):
     u = np.concatenate([np.arange(1, 50), 2 ** 32 - 2 - np.arange(50), [0, 2 ** 32 - 1], rng.integers(0, 2 ** 32, n)]).astype(np.uint32)
     g = rng.uniform(-0.999, 0.999, len(u))
     g[::5] = rng.choice([0.0, 0.8, 0.9, -0.5, 0.99, 0.01, 1e-6, 2.0 ** -30], len(g[::5]))
-    with np.errstate(divide="ignore"):
-        ig = 0.5 / g
-    c = call(lib.hg, u, g, ig, np.empty(len(u), np.int64))[-1]
+    c = call(lib.hg, u, g, np.empty(len(u), np.int64))[-1]
     gl, c0 = g.astype(np.longdouble), 2 * (u.astype(np.longdouble) / np.longdouble(2 ** 32 - 1)) - 1
     d = 1 + gl * c0
     q = (1 - gl * gl) / d
     with np.errstate(divide="ignore", invalid="ignore"):
-        want = np.where(gl == 0, c0, (1 + gl * gl - q * q) * ig.astype(np.longdouble))
-        # d is cut to 4 units of 2^-60, the other terms to 8; ig's own rounding belongs to the caller
-        bound = np.where(gl == 0, 4, np.abs(ig) * (2 * q * q * (4 / d + 8) + 8) + 4) / np.longdouble(ONE)
+        want = np.where(gl == 0, c0, (1 + gl * gl - q * q) / (2 * gl))
+        # d is cut to 4 units of 2^-60, the other terms to 8
+        bound = np.where(gl == 0, 4, np.abs(0.5 / g) * (2 * q * q * (4 / d + 8) + 8) + 4) / np.longdouble(ONE)
     inner = (u > 0) & (u < 2 ** 32 - 1)
     assert np.all(np.abs(c / np.longdouble(ONE) - want)[inner] <= bound[inner] + 2.0 ** -62)
     assert np.all(c[u == 0] == -ONE) and np.all(c[u == 2 ** 32 - 1] == ONE)
     edge = np.array([1.0, -1.0, 0.9995, 1e-10, np.nan, 2.0])
-    c = call(lib.hg, np.full(6, 12345, np.uint32), edge, 0.5 / edge, np.empty(6, np.int64))[-1]
+    c = call(lib.hg, np.full(6, 12345, np.uint32), edge, np.empty(6, np.int64))[-1]
     assert np.all(c == np.iinfo(np.int64).min)
 
 
@@ -177,25 +175,21 @@ def test_turn_in_the_plane(lib):
     u = np.concatenate([np.arange(50), 2 ** 32 - 1 - np.arange(50), 2 ** 31 + np.arange(-20, 20), rng.integers(0, 2 ** 32, n)]).astype(np.uint32)
     g = rng.uniform(-0.998, 0.998, len(u))
     g[::5] = rng.choice([0.0, 0.8, 0.9, -0.5, 0.99, 0.01, 1e-6, -0.998], len(g[::5]))
-    kg = (1 - np.abs(g)) / (1 + np.abs(g))
-    c, s, ok = call(lib.turn2, u, g, kg, np.empty(len(u), np.int64), np.empty(len(u), np.int64), np.empty(len(u), np.int32))[2:]
+    c, s, ok = call(lib.turn2, u, g, np.empty(len(u), np.int64), np.empty(len(u), np.int64), np.empty(len(u), np.int32))[1:]
     assert np.all(ok == 1)
     a = u.astype(np.longdouble) / np.longdouble(2 ** 32) * (4 * np.arctan(np.longdouble(1)))
-    k = kg.astype(np.longdouble)
+    k = (1 - np.abs(g.astype(np.longdouble))) / (1 + np.abs(g.astype(np.longdouble)))
     x, y = np.cos(a) * np.where(g < 0, k, 1), np.sin(a) * np.where(g < 0, 1, k)
     d = x * x + y * y
     # x and y are cut to 2 units of 2^-60 when the larger is brought to [1/2, 1), from units of 2^-62
-    # and k's 2^-64 of a number that is k / 2 at the least; each square to 6, times 1 / d <= 4, and the
+    # and k's own 5 of 2^-61; each square to 6, times 1 / d <= 4, and the
     # quotient's own 8
     bound = (4 * (6 + 6 + 4 / (4 * np.maximum(np.abs(x), np.abs(y))) * 4) + 8) / np.longdouble(ONE)
     iso = g == 0
     wc, ws = np.where(iso, np.cos(2 * a), (x * x - y * y) / d), np.where(iso, np.sin(2 * a), 2 * x * y / d)
     assert np.all(np.abs(c / np.longdouble(ONE) - wc) < bound) and np.all(np.abs(s / np.longdouble(ONE) - ws) < bound)
     edge = np.array([1.0, -1.0, 0.9999, 1e-300, 2.0, -2.0, np.nan])
-    with np.errstate(divide="ignore"):
-        ek = (1 - np.abs(edge)) / (1 + np.abs(edge))
-    ek[:2] = np.nan  # as the walk has it
-    ok = call(lib.turn2, np.full(7, 12345, np.uint32), edge, ek, np.empty(7, np.int64), np.empty(7, np.int64), np.empty(7, np.int32))[-1]
+    ok = call(lib.turn2, np.full(7, 12345, np.uint32), edge, np.empty(7, np.int64), np.empty(7, np.int64), np.empty(7, np.int32))[-1]
     assert not ok.any()
 
 

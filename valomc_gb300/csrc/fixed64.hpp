@@ -7,8 +7,8 @@
 // they are evaluated on the integer pipe, by Taylor series (and, for the logarithm, Tang's table of reciprocals,
 // ACM Trans. Math. Softw. 16, 1990) whose truncation lies below 2^-57, and rounded to double
 // once.  The first four's errors are at most 1.1 units in the last place of a result in [0.5, 1),
-// absolute; the Henyey-Greenstein cosine's is 9e-17 at g = 0.8 and 8e-16 at 0.99 (the same formula
-// in FP64: 2.6e-15 and 3.9e-14).  The CPU tests hold them to their bounds against wider arithmetic.
+// absolute; the Henyey-Greenstein cosine's is 7e-17 at g = 0.9 and 7e-16 at 0.99 (the same formula
+// in FP64: 4.5e-15 and 3.9e-14).  The CPU tests hold them to their bounds against wider arithmetic.
 // Host and device code (the host form is what the tests call).
 #pragma once
 #include <stdint.h>
@@ -209,11 +209,16 @@ VMC_HD inline Root60 sqrt60(int64_t s) {
 }
 
 // The Henyey-Greenstein cosine of the closed uniform's word u: with c = 2 xi - 1 and
-// q = (1 - g^2) / (1 + g c) it is (1 + g^2 - q^2) / (2 g), c when g = 0; ig = 1 / (2 g).
+// q = (1 - g^2) / (1 + g c) it is (1 + g^2 - q^2) / (2 g), c when g = 0.  inv = hg_inverse(g),
+// 1 / (2 |g|) brought to [1/2, 1] by a power of two: as a double its rounding would be every
+// event's, and walks added that up to more than all their other errors.
 // kNoCosine for |g| above 0.999 or below 2^-30, which these units do not hold to a double's last
 // place.
 constexpr int64_t kNoCosine = INT64_MIN;
-VMC_HD inline int64_t hg_cosine(uint32_t u, double g, double ig) {
+VMC_HD inline uint64_t hg_inverse(double g) {
+  return (rcp_fixed(((bits_of_double(g) & 0xfffffffffffffull) | 0x10000000000000ull) << 11) + 2) >> 2;
+}
+VMC_HD inline int64_t hg_cosine(uint32_t u, double g, uint64_t inv) {
   const int64_t c = (int64_t)((((uint64_t)u << 32) | u) ^ 0x8000000000000000ull) >> 3;
   if (u == 0u || u == 0xffffffffu) return u == 0u ? -kOne60 : kOne60;
   if ((bits_of_double(g) << 1) == 0) return c;
@@ -227,27 +232,28 @@ VMC_HD inline int64_t hg_cosine(uint32_t u, double g, double ig) {
   const uint64_t q = ((mulhi_u64(a, rcp_fixed(d << z) << 1)) << (z - 3)) >> 3;
   const Split60 qs = split60((int64_t)q);
   const int64_t m = 2 * kOne60 - (int64_t)(a >> 4) - mul60(qs, qs);
-  // ig = i 2^k, 1 <= i < 2, -1 <= k <= 29
-  const uint64_t ib = bits_of_double(ig);
-  const int k = (int)((ib >> 52) & 0x7ffu) - 1023;
-  const int64_t i = (int64_t)(((ib & 0xfffffffffffffull) | 0x10000000000000ull) << 8);
-  const int64_t ct = mul60(split60((m << (k + 1)) >> 1), split60(i));
-  return (int64_t)ib < 0 ? -ct : ct;
+  const int64_t ct = mul60(split60(m << (1022 - (int)(mag >> 20))), split60((int64_t)inv));
+  return (int64_t)bits_of_double(g) < 0 ? -ct : ct;
 }
 
 // Cosine and sine of the 2D scattering angle 2 atan(h), h = tan(pi xi) (1 - g) / (1 + g), xi =
-// u 2^-32, in units of 2^-60; kg = (1 - |g|) / (1 + |g|).  With x = cos(pi xi) and y = sin(pi xi),
-// the one that kg belongs to times it (x when g < 0), they are (x^2 - y^2) / (x^2 + y^2) and
-// 2 x y / (x^2 + y^2).  False for kg that rounds to 1 or lies below 2^-11.
-VMC_HD inline bool turn_2d(uint32_t u, double g, double kg, int64_t &c, int64_t &s) {
+// u 2^-32, in units of 2^-60; k = turn_ratio(g), (1 - |g|) / (1 + |g|) 2^64, or 0 for |g| above
+// 0.999 or below 2^-30.  With x = cos(pi xi) and y = sin(pi xi),
+// the one that k belongs to times it (x when g < 0), they are (x^2 - y^2) / (x^2 + y^2) and
+// 2 x y / (x^2 + y^2).  False when k = 0 and g is not.
+VMC_HD inline uint64_t turn_ratio(double g) {
+  const uint32_t mag = mag_of(g);
+  if (mag > 0x3feff7ceu || mag < 0x3e100000u) return 0;  // 0.999, 2^-30
+  const uint64_t ga = fixed_of_double(double_of_bits(bits_of_double(g) & 0x7fffffffffffffffull));
+  return mulhi_u64((uint64_t)0 - ga, rcp_fixed(0x8000000000000000ull + (ga >> 1)) << 2);
+}
+VMC_HD inline bool turn_2d(uint32_t u, double g, uint64_t k, int64_t &c, int64_t &s) {
   const bool iso = (bits_of_double(g) << 1) == 0;  // then the angle is 2 pi xi itself
   int64_t s0, c0;
   sincos_turn_fixed((uint64_t)u << (iso ? 32 : 31), s0, c0);
-  const uint32_t top = (uint32_t)(bits_of_double(kg) >> 32);
-  const uint64_t k6 = fixed_of_double(kg);
   uint64_t x = (uint64_t)(c0 < 0 ? -c0 : c0), y = (uint64_t)s0;
   const bool back = (int64_t)bits_of_double(g) < 0;
-  const uint64_t cut = mulhi_u64(back ? x : y, k6);
+  const uint64_t cut = mulhi_u64(back ? x : y, k);
   x = back ? cut : x;
   y = back ? y : cut;
   const int z = clz_u64(x > y ? x : y);
@@ -258,7 +264,7 @@ VMC_HD inline bool turn_2d(uint32_t u, double g, double kg, int64_t &c, int64_t 
   const int64_t cs = mul60(split60(a - b), inv) << (zd - 3), sn = mul60(split60(mul60(xs, ys)), inv) << (zd - 2);
   c = iso ? c0 >> 2 : cs;
   s = iso ? s0 >> 2 : c0 < 0 ? -sn : sn;
-  return iso || (top < 0x3ff00000u && top >= 0x3f400000u);
+  return iso || k != 0;
 }
 
 // v brought back to length 1 when it is there to 2^-30 already

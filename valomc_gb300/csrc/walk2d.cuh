@@ -40,7 +40,8 @@ struct Walk2D64 {
   using Tr = typename TraceFor<R>::type;
   double pos[2], dir[2];
   double w, prop, cph, sph;
-  double mua, mus, g, nidx, imus, kg;  // imus = 1 / mus, kg = (1 - g) / (1 + g)
+  double mua, mus, g, nidx, imus;  // imus = 1 / mus
+  uint64_t kg;                     // turn_ratio(g)
   double acc, accI;
   uint64_t turn;  // phase in 2^-64 turns
   int el, curface;
@@ -62,9 +63,9 @@ struct Walk2D64 {
     a = o0.x; s = o0.y; gg = o1.x; nn = o1.y;
   }
 
-  // (1 - |g|) / (1 + |g|); at |g| = 1 the reference's sqrt((g^2 + 1)^2 - 4 g^2) is 0 and its angle NaN
+  // (1 - g) / (1 + g); at |g| = 1 the reference's sqrt((g^2 + 1)^2 - 4 g^2) is 0 and its angle NaN
   __device__ __forceinline__ static double turn_factor(double g) {
-    return fabs(g) == 1.0 ? __longlong_as_double(0x7ff8000000000000ll) : fast_div(1.0 - fabs(g), 1.0 + fabs(g));
+    return fabs(g) == 1.0 ? __longlong_as_double(0x7ff8000000000000ll) : fast_div(1.0 - g, 1.0 + g);
   }
 
   __device__ void launch(const JobDev &J, R &rng, int64_t q) {
@@ -77,7 +78,7 @@ struct Walk2D64 {
     }
     optics(J, el, mua, mus, g, nidx);
     imus = fast_rcp(mus);
-    kg = turn_factor(g);
+    kg = turn_ratio(g);
     prop = neg_log_open(rng.next()) * imus;
     acc = accI = 0.0;
     nsteps = 0;
@@ -128,13 +129,13 @@ struct Walk2D64 {
   }
 
   // The turn in FP64, for what fixed point does not hold: |g| near 1 or nearly 0, a direction that
-  // is not a unit vector yet.  With (s0, c0) the sine and cosine of pi xi and ks = kg s0 the turn's
+  // is not a unit vector yet.  With (s0, c0) the sine and cosine of pi xi and ks = (1 - g) / (1 + g) s0 the turn's
   // cosine is (c0^2 - ks^2) / (c0^2 + ks^2) and its sine 2 ks c0 / (c0^2 + ks^2).
   struct Dir { double x, y; };
-  __device__ __noinline__ static Dir turn_d(uint32_t u, double g, double kg, double dx, double dy) {
+  __device__ __noinline__ static Dir turn_d(uint32_t u, double g, double dx, double dy) {
     double s0, c0;
     sincos_turn((uint64_t)u << 31, s0, c0);
-    const double ks = (g < 0.0 ? 1.0 / kg : kg) * s0;
+    const double ks = turn_factor(g) * s0;
     const double a = c0 * c0, b = ks * ks;
     const double den = a + b;
     const double y0 = f2d_int(__frcp_rn(f32_of(den)));
@@ -255,7 +256,7 @@ struct Walk2D64 {
       if (positive(mus)) {
         const Event ev = draw_event(rng.peek3());
         if (!rotate(ev)) {
-          const Dir d = turn_d(rng.peek3().x, g, kg, dir[0], dir[1]);
+          const Dir d = turn_d(rng.peek3().x, g, dir[0], dir[1]);
           dir[0] = d.x; dir[1] = d.y;
           curface = -1;
         }
@@ -348,7 +349,7 @@ struct Walk2D64 {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
     }
-    if (differ(g2, g)) kg = turn_factor(g2);
+    if (differ(g2, g)) kg = turn_ratio(g2);
     flush(J);
     curface = f2;
     el = nextel;

@@ -163,7 +163,8 @@ struct Walk3D64 {
   using Tr = typename TraceFor<R>::type;
   double pos[3], dir[3];
   double w, prop, cph, sph;
-  double mua, mus, g, nidx, imus, ig;  // imus = 1 / mus, ig = 1 / (2 g)
+  double mua, mus, g, nidx, imus;  // imus = 1 / mus
+  uint64_t ig;                     // hg_inverse(g)
   double acc, accI;
   uint64_t turn;  // phase in 2^-64 turns
   int el, curface;
@@ -195,7 +196,7 @@ struct Walk3D64 {
     }
     optics(J, el, mua, mus, g, nidx);
     imus = fast_rcp(mus);
-    ig = 0.5 * fast_rcp(g);
+    ig = hg_inverse(g);
     prop = neg_log_open(rng.next()) * imus;  // the outer loop's first draw, MC3D.hpp:1458
     acc = accI = 0.0;
     nsteps = 0;
@@ -267,11 +268,11 @@ struct Walk3D64 {
   // Both in FP64, for what fixed point does not hold: |g| near 1 or nearly 0, a direction that is
   // not a unit vector yet, a cosine beyond 1.
   struct Dir { double x, y, z; };
-  __device__ __noinline__ static Dir scatter_d(uint32_t ux, uint32_t uy, double g, double ig, double dx, double dy, double dz) {
+  __device__ __noinline__ static Dir scatter_d(uint32_t ux, uint32_t uy, double g, double dx, double dy, double dz) {
     const double c0 = fma(word_d(ux), 2.0 / 4294967295.0, -1.0);  // 2 xi - 1, the isotropic cosine
     const double D = fma(g, c0, 1.0);                              // 1 - g (1 - 2 xi)
     const double q = div_near(fma(-g, g, 1.0), D, f32_of(D));
-    double ct = fma(-q, q, fma(g, g, 1.0)) * ig;
+    double ct = fma(-q, q, fma(g, g, 1.0)) * (0.5 * fast_rcp(g));
     ct = ux == 0u ? -1.0 : ux == 0xffffffffu ? 1.0 : ct;  // theta = (1 - xi) pi at xi in {0, 1}
     ct = (__double_as_longlong(g) << 1) == 0 ? c0 : ct;
     const double t2 = fma(-ct, ct, 1.0);
@@ -423,7 +424,7 @@ struct Walk3D64 {
         const Event ev = draw_event(rng.peek3());
         if (!rotate(ev)) {
           const uint3 u = rng.peek3();
-          const Dir d = scatter_d(u.x, u.y, g, ig, dir[0], dir[1], dir[2]);
+          const Dir d = scatter_d(u.x, u.y, g, dir[0], dir[1], dir[2]);
           dir[0] = d.x; dir[1] = d.y; dir[2] = d.z;
           curface = -1;
         }
@@ -504,7 +505,7 @@ struct Walk3D64 {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
     }
-    if (differ(g2, g)) ig = 0.5 * fast_rcp(g2);
+    if (differ(g2, g)) ig = hg_inverse(g2);
     flush(J);
     curface = f2;
     el = nextel;
