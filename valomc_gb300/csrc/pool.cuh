@@ -39,7 +39,12 @@ __device__ __forceinline__ int find_job(const int64_t *begin, int njobs, int64_t
 // take ten times the mean, half of a 1e6-photon launch ran in warps that were mostly empty.
 // So the CTA's warps then meet every kPackEvery steps, and when the photons alive would fit
 // three quarters of the warps that hold them they are moved together through shared memory, a
-// few words of the state at a time.  A photon's arithmetic does not depend on the lane that
+// few words of the state at a time.  They stay in two warps while there are more than three, and
+// the last three get a warp each: two warps fill an SM's four schedulers with the FP64 forms' two
+// CTAs, and a warp of one photon takes one branch.  (Full warps to the end, two, four and eight
+// warps at the least: 9.6, 8.7, 8.8 and 10.1 ms at 1e4 photons on the phantom, 13.4, 13.4, 14.9
+// and 17.4 at 1e5, in FP64 78, 78, 84 and 96; at 1e3 there 38.7, and 33.0 with the last three
+// apart.)  A photon's arithmetic does not depend on the lane that
 // carries it.  With the photons of small launches dealt to all SMs alike (below): 35.9 ->
 // 29.6 ms for 1e6 photons on the phantom (32.1 without), 20.5 -> 13.4 at 1e5, 13-18 -> 9.6 at
 // 1e4; FP64 571 -> 313 ms at 1e5.  Meeting every 64 to 512 steps measured alike there; every 64
@@ -192,9 +197,9 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
             used += c > 0;
           }
           if (all == 0 && !pending) break;
-          const int want = (all + 31) >> 5;
+          const int want = all <= 3 ? all : max((all + 31) >> 5, 2);
           if constexpr (!R::kReplay) {
-            if (!pending && 4 * want <= 3 * used) {
+            if (!pending && (used < want || 4 * want <= 3 * used)) {
               const int each = (all + want - 1) / want;
               const int k = before + __popc(live & lt_mask);
               const int to = alive ? ((k / each + warp_turn(lp, warps)) % warps) * 32 + k % each : -1;
