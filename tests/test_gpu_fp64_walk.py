@@ -92,3 +92,21 @@ def test_scattering_angles_at_the_ends_of_fixed_point(built, dim, g):
     for k in ("ER", "EBR"):
         a, b = getattr(gpu, k), getattr(ref, k)
         assert np.abs(a - b).sum() <= 1e-6 * np.abs(b).sum(), k
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("source", ["c", "i"])
+@pytest.mark.parametrize("n_out", [1.35, 1.0, 1.36, 0.2, 6.0])
+def test_interfaces_and_launches(built, dim, source, n_out):
+    """The choice at an interface in FP32, where it is certain (index ratios of 1/4 to 4), and in
+    FP64 elsewhere; the launches' directions."""
+    p = problem(dim, "slivers", True, 0.0)
+    p.BCn[:] = n_out
+    p.BCType[p.BCType == ord("c")] = ord(source)
+    gpu = V.run(p, precision=V.VMC_FP64)
+    ref = oracle.run(p, rng=oracle.RNG_PHILOX, nthreads=4)
+    assert gpu.stats["photons_done"] == p.Nphoton and gpu.stats["loss"] == ref.loss
+    assert gpu.stats["steps"] == ref.steps
+    for k in ("ER", "EBR", "DEBR"):
+        a, b = getattr(gpu, k), getattr(ref, k)
+        assert np.abs(a - b).sum() <= 1e-6 * np.abs(b).sum(), k

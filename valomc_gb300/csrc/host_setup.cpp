@@ -599,6 +599,8 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
         S.n[0] = n[0]; S.n[1] = n[1];
         if (in->n_BCLNormal) { S.L[0] = L[ib]; S.L[1] = L[ib + Nb]; }
         S.phi0 = S.dirtype == 'n' ? atan2(n[1], n[0]) : atan2(S.L[1], S.L[0]);
+        S.cphi0 = cos(S.phi0);
+        S.sphi0 = sin(S.phi0);
         if (bt == 'g') {  // MC2D.hpp:1044
           S.sigma = in->GaussianSigma[ib];
           S.gauss_h = 0.5 - 0.5 * erf(kPi / S.sigma / 2.0 / sqrt(2.0));

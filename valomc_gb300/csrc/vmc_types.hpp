@@ -88,6 +88,7 @@ struct alignas(16) SourceRec {
   double e1[3], e2[3];         // cosinic frame (3D, both direction types)
   double L[3];                 // BCLNormal row after Init's normalisation / relative mapping
   double phi0;                 // 2D: atan2 of the mean direction (normal or BCLNormal)
+  double cphi0, sphi0;         // its cosine and sine
   double sigma;                // 2D Gaussian sigma
   double gauss_h;              // 2D: 0.5 - 0.5 erf(pi / sigma / 2 / sqrt 2)
   int32_t mother;              // LightSourcesMother

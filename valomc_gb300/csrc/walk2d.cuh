@@ -70,7 +70,7 @@ struct Walk2D64 {
 
   __device__ void launch(const JobDev &J, R &rng, int64_t q) {
     tr.begin(J, q);
-    create_photon_2d(J, rng, pos, dir, el, curface);
+    create_photon_2d<false>(J, rng, pos, dir, el, curface);
     w = 1.0;
     if (FD) {
       turn = J.turn0;
@@ -147,17 +147,34 @@ struct Walk2D64 {
     return Dir{fma(dx, c, -(dy * s)), fma(dy, c, dx * s)};
   }
 
-  __device__ __forceinline__ bool fresnel(R &rng, double n0, double n1, double nipnt, int nf, bool boundary) {
-    const double costhi = -(dir[0] * n0 + dir[1] * n1);
+  // FresnelPhoton at an edge with normal (n0, n1) of any length
+  __device__ __forceinline__ bool fresnel(R &rng, double n0, double n1, double nout, int nf, bool inside) {
+    const float f0 = f32_of(n0), f1 = f32_of(n1);
+    const Choice choice = fresnel_choice(rng, __fdividef(f32_of(nidx), f32_of(nout)), f0 * f32_of(dir[0]) + f1 * f32_of(dir[1]),
+                                         f0 * f0 + f1 * f1);
+    if (choice.what == Choice::kPass && !inside) return false;
+    const double nn = fma(n0, n0, n1 * n1), dn = fma(dir[0], n0, dir[1] * n1);
+    if (choice.what == Choice::kReflect) {
+      const double k = -2.0 * div_near(dn, nn, f32_of(nn));
+      dir[0] = fma(k, n0, dir[0]);
+      dir[1] = fma(k, n1, dir[1]);
+      curface = nf;
+      return true;
+    }
+    const double nipnt = fast_div(nidx, nout);
+    double len, inv;
+    fast_sqrt(nn, len, inv);
+    n0 *= inv; n1 *= inv;
+    const double costhi = -dn * inv;
     double costht = 0.0;
-    if (fresnel_reflects_d(rng, nipnt, costhi, costht)) {
+    if (fresnel_reflects_d(rng, choice, nipnt, costhi, costht)) {
       const double k = 2.0 * costhi;
       dir[0] = fma(k, n0, dir[0]);
       dir[1] = fma(k, n1, dir[1]);
       curface = nf;
       return true;
     }
-    if (boundary) return false;
+    if (!inside) return false;
     const double m = (costhi > 0.0) ? (nipnt * costhi - costht) : (nipnt * costhi + costht);
     dir[0] = fma(nipnt, dir[0], m * n0);
     dir[1] = fma(nipnt, dir[1], m * n1);
@@ -306,10 +323,7 @@ struct Walk2D64 {
     const bool light = inside && below(w, kWeight0);
     if (!inside || vacuum || jump || light) {
       const double *m = (recs(J) + el)->n[nf];
-      double n0 = __ldg(m), n1 = __ldg(m + 1);  // outward
-      double len, inv;
-      fast_sqrt(fma(n0, n0, n1 * n1), len, inv);
-      n0 *= inv; n1 *= inv;
+      const double n0 = __ldg(m), n1 = __ldg(m + 1);  // outward
       rng.reload();
       if (vacuum) prop = neg_log_open(rng.next()) / mus2;
       if (light) {
@@ -317,12 +331,13 @@ struct Walk2D64 {
           job_count(J, kJcRoulette); job_ledger(J, kLgRouletteKill, w);
           return die(J, kEvRoulette);
         }
-        job_ledger(J, kLgRouletteGain, w / kChance - w);
-        w /= kChance;
+        const double up = w / kChance;
+        job_ledger(J, kLgRouletteGain, up - w);
+        w = up;
       }
-      if (jump && fresnel(rng, n0, n1, fast_div(nidx, n2), nf, !inside)) return true;
+      if (jump && fresnel(rng, n0, n1, n2, nf, inside)) return true;
       if (!inside) {
-        const double idn = fast_rcp(dir[0] * n0 + dir[1] * n1);  // DEBR, MC2D.hpp:1410-1437
+        const double idn = fast_sqrt(fma(n0, n0, n1 * n1)) * fast_rcp(fma(dir[0], n0, dir[1] * n1));  // DEBR, MC2D.hpp:1410-1437
         flush(J);
         if (!FD) {
           add_d(J, J.EBR + ib, w);
@@ -394,7 +409,7 @@ struct Walk2D64L {
 
   __device__ void launch(const JobDev &J, R &rng, int64_t q) {
     tr.begin(J, q);
-    create_photon_2d(J, rng, pos, dir, el, curface);
+    create_photon_2d<true>(J, rng, pos, dir, el, curface);
     w = 1.0;
     phase = J.phase0;
     if (FD) sincos(phase, &sph, &cph);

@@ -44,13 +44,39 @@ __device__ __forceinline__ bool ray_tri(const double O[3], const double D[3], co
 // forms rs = (eta ci - ct) / (eta ci + ct), rp = (ci - eta ct) / (ci + eta ct) over one division:
 // the reference's R = (sin^2(thi - tht) / sin^2(thi + tht) + tan^2 / tan^2) / 2 to a few ulps,
 // without its seven angles and their functions.
+//
+// Where FP32 is certain of the choice it is made there, and the photon that leaves the body or is
+// reflected needs no root and no quotient in FP64: eta = n1 / n2 and ci = |cos| in FP32 have
+// errors of 3e-7, so 1 - ct^2 = eta^2 (1 - ci^2) one of 1e-6 (1 + eta^2), and R, from ct >= 0.1,
+// one of 1e-4 (1 + eta^2); twice the last and ten times the other are allowed for.  word: what
+// has been drawn, if anything.  With the launches' directions (create_photon_2d) 7.6 -> 5.8 ms
+// for 1e6 photons on the 2D square, which launch, and meet the boundary, every 30 steps.
+struct Choice {
+  enum What { kPass, kReflect, kUnsure } what;
+  bool drawn;
+  uint32_t word;
+};
 template <class R>
-__device__ __forceinline__ bool fresnel_reflects_d(R &rng, double nipnt, double costhi, double &costht) {
+__device__ __forceinline__ Choice fresnel_choice(R &rng, float eta, float dn, float nn) {
+  const float ci = fabsf(dn) * rsqrtf(nn), e2 = eta * eta, s2 = e2 * fmaf(-ci, ci, 1.0f), wide = 1.0f + e2;
+  if (!(eta > 0.25f && eta < 4.0f && nn > 1e-30f && nn < 1e30f && ci < 1.00001f)) return Choice{Choice::kUnsure, false, 0u};
+  if (s2 > 1.0f + 1e-5f * wide) return Choice{Choice::kReflect, false, 0u};
+  if (!(s2 < 0.99f)) return Choice{Choice::kUnsure, false, 0u};
+  const uint32_t w = rng.next();
+  const float ct = sqrtf(1.0f - s2);
+  const float rs = __fdividef(fmaf(eta, ci, -ct), fmaf(eta, ci, ct)), rp = __fdividef(fmaf(-eta, ct, ci), fmaf(eta, ct, ci));
+  const float m = (float)w * 2.3283064365386963e-10f - 0.5f * fmaf(rs, rs, rp * rp);
+  const bool near1 = ci > 0.999999f;  // above 1 the photon passes (below)
+  return Choice{m > 2e-4f * wide ? Choice::kPass : m < -2e-4f * wide && !near1 ? Choice::kReflect : Choice::kUnsure, true, w};
+}
+template <class R>
+__device__ __forceinline__ bool fresnel_reflects_d(R &rng, const Choice &choice, double nipnt, double costhi, double &costht) {
   const double s = 1.0 - nipnt * nipnt * (1.0 - costhi * costhi);
   if (s <= 0.0) return true;
   costht = fast_sqrt(s);
+  if (choice.what == Choice::kPass) return false;
   const double ci = fabs(costhi);
-  const double u = word_d(rng.next()) * (1.0 / 4294967295.0);  // unif_closed
+  const double u = word_d(choice.drawn ? choice.word : rng.next()) * (1.0 / 4294967295.0);  // unif_closed
   if (!(ci <= 1.0)) return false;  // acos is NaN there in the reference, and so is R
   const double a = fma(nipnt, ci, -costht), b = fma(nipnt, ci, costht);
   const double c = fma(-nipnt, costht, ci), d = fma(nipnt, costht, ci);
@@ -188,7 +214,7 @@ struct Walk3D64 {
 
   __device__ void launch(const JobDev &J, R &rng, int64_t q) {
     tr.begin(J, q);
-    create_photon_3d(J, rng, pos, dir, el, curface);
+    create_photon_3d<false>(J, rng, pos, dir, el, curface);
     w = 1.0;
     if (FD) {
       turn = J.turn0;
@@ -301,14 +327,27 @@ struct Walk3D64 {
 
   // FresnelPhoton at a face with normal nor, of either orientation and any length
   // (MC3D.hpp:1365-1447); true if reflected
-  __device__ __forceinline__ bool fresnel(R &rng, const double *nor, double nipnt, int nf) {
+  __device__ __forceinline__ bool fresnel(R &rng, const double *nor, double nout, int nf, bool inside) {
     double n0 = __ldg(nor), n1 = __ldg(nor + 1), n2 = __ldg(nor + 2);
+    const float f0 = f32_of(n0), f1 = f32_of(n1), f2 = f32_of(n2);
+    const Choice choice = fresnel_choice(rng, __fdividef(f32_of(nidx), f32_of(nout)),
+                                         f0 * f32_of(dir[0]) + f1 * f32_of(dir[1]) + f2 * f32_of(dir[2]),
+                                         f0 * f0 + f1 * f1 + f2 * f2);
+    if (choice.what == Choice::kPass && !inside) return false;
+    const double nn = fma(n0, n0, fma(n1, n1, n2 * n2)), dn = fma(dir[0], n0, fma(dir[1], n1, dir[2] * n2));
+    if (choice.what == Choice::kReflect) {
+      const double k = -2.0 * div_near(dn, nn, f32_of(nn));
+      dir[0] = fma(k, n0, dir[0]); dir[1] = fma(k, n1, dir[1]); dir[2] = fma(k, n2, dir[2]);
+      curface = nf;
+      return true;
+    }
+    const double nipnt = fast_div(nidx, nout);
     double len, inv;
-    fast_sqrt(fma(n0, n0, fma(n1, n1, n2 * n2)), len, inv);
+    fast_sqrt(nn, len, inv);
     n0 *= inv; n1 *= inv; n2 *= inv;
-    const double costhi = -(dir[0] * n0 + dir[1] * n1 + dir[2] * n2);
+    const double costhi = -dn * inv;
     double costht = 0.0;
-    if (fresnel_reflects_d(rng, nipnt, costhi, costht)) {
+    if (fresnel_reflects_d(rng, choice, nipnt, costhi, costht)) {
       const double k = 2.0 * costhi;
       dir[0] = fma(k, n0, dir[0]); dir[1] = fma(k, n1, dir[1]); dir[2] = fma(k, n2, dir[2]);
       curface = nf;
@@ -481,10 +520,11 @@ struct Walk3D64 {
           job_count(J, kJcRoulette); job_ledger(J, kLgRouletteKill, w);
           return die(J, kEvRoulette);
         }
-        job_ledger(J, kLgRouletteGain, w / kChance - w);
-        w /= kChance;
+        const double up = w / kChance;
+        job_ledger(J, kLgRouletteGain, up - w);
+        w = up;
       }
-      if (jump && fresnel(rng, nor, nidx / n2, nf)) return true;
+      if (jump && fresnel(rng, nor, n2, nf, inside)) return true;
     }
     if (!inside) {
       flush(J);
@@ -553,7 +593,7 @@ struct Walk3D64L {
 
   __device__ void launch(const JobDev &J, R &rng, int64_t q) {
     tr.begin(J, q);
-    create_photon_3d(J, rng, pos, dir, el, curface);
+    create_photon_3d<true>(J, rng, pos, dir, el, curface);
     w = 1.0;
     phase = J.phase0;
     if (FD) sincos(phase, &sph, &cph);

@@ -59,105 +59,6 @@ __device__ __forceinline__ void job_ledger(const JobDev &J, int which, double v)
   atomicAdd(J.ledger + (blockIdx.x & (kSlots - 1)) * kLgN + which, v);
 }
 
-// first source with xi < CDF (cpp/3d/MC3D.hpp:1068-1070), clamped to the last source
-// (cpp/2d/MC2D.hpp:969; in 3D the reference would read one past the end at xi == 1)
-__device__ __forceinline__ int pick_source(const JobDev &J, double xi) {
-  int lo = 0, hi = J.Ns;  // first index with cdf > xi in [lo, hi]
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (xi < __ldg(J.cdf + mid)) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo < J.Ns ? lo : J.Ns - 1;
-}
-
-// ---- 3D CreatePhoton (cpp/3d/MC3D.hpp:1060-1294) in double, from the face record ----
-template <class R>
-__device__ __forceinline__ void create_photon_3d(const JobDev &J, R &rng, double pos[3], double dir[3], int &curel, int &curface) {
-  double xi = unif_closed(rng);
-  const SourceRec &S = J.src[pick_source(J, xi)];
-  curel = S.mother;
-  curface = S.curface;
-  double r1 = unif_open(rng), r2 = unif_open(rng);
-  double sr = sqrt(r1);
-#pragma unroll
-  for (int c = 0; c < 3; c++) pos[c] = (1.0 - sr) * S.v0[c] + sr * (1.0 - r2) * S.v1[c] + sr * r2 * S.v2[c];
-  const double n0 = S.n[0], n1 = S.n[1], n2 = S.n[2];
-  dir[0] = n0; dir[1] = n1; dir[2] = n2;  // 'l', and the combinations the reference leaves undefined
-  const char bt = S.type, dt = S.dirtype;
-  if (dt != 'n' && (bt == 'l' || bt == 'L')) {
-    dir[0] = S.L[0]; dir[1] = S.L[1]; dir[2] = S.L[2];
-  } else if (dt != 'n' && bt == 'p') {
-    pos[0] = S.L[0]; pos[1] = S.L[1]; pos[2] = S.L[2];
-  } else if ((dt == 'n' && bt == 'i') || (dt != 'n' && (bt == 'i' || bt == 'I'))) {
-    // rejection on the sphere, Mathworld sphere point picking (MC3D.hpp:1124-1141)
-    double rr0 = n0, rr1 = n1, rr2 = n2;
-    for (int it = 0; it < kMaxRejections; it++) {
-      double th = 2.0 * kPi * unif_halfup(rng);
-      double u = 2.0 * unif_closed(rng) - 1.0;
-      double st, ct;
-      sincos(th, &st, &ct);
-      double sq = sqrt(1.0 - u * u);
-      rr0 = sq * ct; rr1 = sq * st; rr2 = u;
-      if (n0 * rr0 + n1 * rr1 + n2 * rr2 > 0.0 || rng.exhausted()) break;
-    }
-    dir[0] = rr0; dir[1] = rr1; dir[2] = rr2;
-  } else if (bt == 'c' || bt == 'C') {
-    // cosinic: phi = asin(2U - 1), theta = 2 pi U, mapped onto the face frame (MC3D.hpp:1142-1191)
-    double phi = asin(2.0 * unif_open(rng) - 1.0);
-    double th = 2.0 * kPi * unif_closed(rng);
-    double sp, cp, st, ct;
-    sincos(phi, &sp, &cp);
-    sincos(th, &st, &ct);
-    double f0 = cp, f1 = ct * sp, f2 = st * sp;
-#pragma unroll
-    for (int c = 0; c < 3; c++) dir[c] = f0 * S.n[c] + f1 * S.e1[c] + f2 * S.e2[c];
-  }
-}
-
-// ---- 2D CreatePhoton (cpp/2d/MC2D.hpp:958-1132) ----
-template <class R>
-__device__ double gauss_angle(R &rng, double sigma, double h) {
-  double xi = unif_open(rng);
-  double a = -kPi / 2, b = kPi / 2, phi = 0.0;
-  const double isq2 = sqrt(2.0);
-  for (int it = 0; it < 16; it++) {
-    phi = (a + b) / 2.0;
-    double cdf = (0.5 + 0.5 * erf(phi / sigma / isq2) - h) / (1 - 2.0 * h);
-    if (cdf - xi < 0.0) a = phi;
-    else b = phi;
-  }
-  return phi;
-}
-
-template <class R>
-__device__ __forceinline__ void create_photon_2d(const JobDev &J, R &rng, double pos[2], double dir[2], int &curel, int &curface) {
-  double xi = unif_closed(rng);
-  const SourceRec &S = J.src[pick_source(J, xi)];
-  curel = S.mother;
-  curface = S.curface;
-  double wv = unif_open(rng);
-  pos[0] = S.v0[0] + wv * (S.v1[0] - S.v0[0]);
-  pos[1] = S.v0[1] + wv * (S.v1[1] - S.v0[1]);
-  const double n0 = S.n[0], n1 = S.n[1];
-  dir[0] = n0; dir[1] = n1;
-  const char bt = S.type, dt = S.dirtype;
-  if (bt == 'l') {
-    if (dt != 'n') { dir[0] = S.L[0]; dir[1] = S.L[1]; }
-  } else if (bt == 'i') {
-    double phi = kPi * (unif_open(rng) - 0.5);
-    sincos(S.phi0 + phi, &dir[1], &dir[0]);
-  } else if (bt == 'c' || bt == 'g') {
-    // direction type 'n': one draw; otherwise redraw until the direction points inward
-    // (MC2D.hpp:1085-1124)
-    for (int it = 0; it < kMaxRejections; it++) {
-      double phi = (bt == 'c') ? asin(2.0 * unif_open(rng) - 1.0) : gauss_angle(rng, S.sigma, S.gauss_h);
-      sincos(S.phi0 + phi, &dir[1], &dir[0]);
-      if (dt == 'n' || n0 * dir[0] + n1 * dir[1] > 0.0 || rng.exhausted()) break;
-    }
-  }
-}
-
 // A reduction into a global FP64 accumulator.  The accumulators are plain device buffers,
 // so the address is converted to the global window once and the add is issued as a
 // fire-and-forget global reduction (no generic-address resolution, no returned value).
@@ -430,6 +331,146 @@ __device__ __forceinline__ double word_d(uint32_t w) { return __hiloint2double(0
 // unif_closed(rng) <= p, by that mapping (word / (2^32 - 1))
 template <class R> __device__ __forceinline__ bool closed_at_most(R &rng, double p) {
   return word_d(rng.next()) * (1.0 / 4294967295.0) <= p;
+}
+
+// first source with xi < CDF (cpp/3d/MC3D.hpp:1068-1070), clamped to the last source
+// (cpp/2d/MC2D.hpp:969; in 3D the reference would read one past the end at xi == 1)
+__device__ __forceinline__ int pick_source(const JobDev &J, double xi) {
+  int lo = 0, hi = J.Ns;  // first index with cdf > xi in [lo, hi]
+  while (lo < hi) {
+    int mid = (lo + hi) >> 1;
+    // xi < cdf by their bits, on the integer pipe: xi >= 0
+    if (__double_as_longlong(xi) < __double_as_longlong(__ldg(J.cdf + mid))) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo < J.Ns ? lo : J.Ns - 1;
+}
+
+// 2 U - 1 of the open uniform's word, and the cosine of the angle whose sine that is
+__device__ __forceinline__ void open_sine(uint32_t w, double &s, double &c) {
+  s = fma(word_d(w) + 0.5, 0x1p-31, -1.0);
+  c = fast_sqrt(fma(-s, s, 1.0));
+}
+
+// ---- 3D CreatePhoton (cpp/3d/MC3D.hpp:1060-1294) in double, from the face record ----
+// kLiteral: with the reference's functions in its order; else, as in the rest of the plain walks,
+// sines and cosines on the integer pipe and sin(asin(s)) = s: a launch in the plane took some 150
+// operations of the FP64 pipe, now 35.
+template <bool kLiteral, class R>
+__device__ __forceinline__ void create_photon_3d(const JobDev &J, R &rng, double pos[3], double dir[3], int &curel, int &curface) {
+  double xi = unif_closed(rng);
+  const SourceRec &S = J.src[pick_source(J, xi)];
+  curel = S.mother;
+  curface = S.curface;
+  double r1 = unif_open(rng), r2 = unif_open(rng);
+  double sr = kLiteral ? sqrt(r1) : fast_sqrt(r1);
+#pragma unroll
+  for (int c = 0; c < 3; c++) pos[c] = (1.0 - sr) * S.v0[c] + sr * (1.0 - r2) * S.v1[c] + sr * r2 * S.v2[c];
+  const double n0 = S.n[0], n1 = S.n[1], n2 = S.n[2];
+  dir[0] = n0; dir[1] = n1; dir[2] = n2;  // 'l', and the combinations the reference leaves undefined
+  const char bt = S.type, dt = S.dirtype;
+  if (dt != 'n' && (bt == 'l' || bt == 'L')) {
+    dir[0] = S.L[0]; dir[1] = S.L[1]; dir[2] = S.L[2];
+  } else if (dt != 'n' && bt == 'p') {
+    pos[0] = S.L[0]; pos[1] = S.L[1]; pos[2] = S.L[2];
+  } else if ((dt == 'n' && bt == 'i') || (dt != 'n' && (bt == 'i' || bt == 'I'))) {
+    // rejection on the sphere, Mathworld sphere point picking (MC3D.hpp:1124-1141)
+    double rr0 = n0, rr1 = n1, rr2 = n2;
+    for (int it = 0; it < kMaxRejections; it++) {
+      double u, st, ct, sq;
+      if constexpr (kLiteral) {
+        double th = 2.0 * kPi * unif_halfup(rng);
+        u = 2.0 * unif_closed(rng) - 1.0;
+        sincos(th, &st, &ct);
+        sq = sqrt(1.0 - u * u);
+      } else {
+        sincos_turn((uint64_t)rng.next() << 32, st, ct);
+        u = fma(word_d(rng.next()), 2.0 / 4294967295.0, -1.0);
+        sq = fast_sqrt(fma(-u, u, 1.0));
+      }
+      rr0 = sq * ct; rr1 = sq * st; rr2 = u;
+      if (n0 * rr0 + n1 * rr1 + n2 * rr2 > 0.0 || rng.exhausted()) break;
+    }
+    dir[0] = rr0; dir[1] = rr1; dir[2] = rr2;
+  } else if (bt == 'c' || bt == 'C') {
+    // cosinic: phi = asin(2U - 1), theta = 2 pi U, mapped onto the face frame (MC3D.hpp:1142-1191)
+    double sp, cp, st, ct;
+    if constexpr (kLiteral) {
+      double phi = asin(2.0 * unif_open(rng) - 1.0);
+      double th = 2.0 * kPi * unif_closed(rng);
+      sincos(phi, &sp, &cp);
+      sincos(th, &st, &ct);
+    } else {
+      open_sine(rng.next(), sp, cp);
+      const uint32_t w = rng.next();
+      sincos_turn(((uint64_t)w << 32) | w, st, ct);
+    }
+    double f0 = cp, f1 = ct * sp, f2 = st * sp;
+#pragma unroll
+    for (int c = 0; c < 3; c++) dir[c] = f0 * S.n[c] + f1 * S.e1[c] + f2 * S.e2[c];
+  }
+}
+
+// ---- 2D CreatePhoton (cpp/2d/MC2D.hpp:958-1132) ----
+template <class R>
+__device__ double gauss_angle(R &rng, double sigma, double h) {
+  double xi = unif_open(rng);
+  double a = -kPi / 2, b = kPi / 2, phi = 0.0;
+  const double isq2 = sqrt(2.0);
+  for (int it = 0; it < 16; it++) {
+    phi = (a + b) / 2.0;
+    double cdf = (0.5 + 0.5 * erf(phi / sigma / isq2) - h) / (1 - 2.0 * h);
+    if (cdf - xi < 0.0) a = phi;
+    else b = phi;
+  }
+  return phi;
+}
+
+// the mean direction turned by an angle
+__device__ __forceinline__ void turned(const SourceRec &S, double sn, double cs, double dir[2]) {
+  dir[0] = fma(S.cphi0, cs, -(S.sphi0 * sn));
+  dir[1] = fma(S.sphi0, cs, S.cphi0 * sn);
+}
+
+template <bool kLiteral, class R>
+__device__ __forceinline__ void create_photon_2d(const JobDev &J, R &rng, double pos[2], double dir[2], int &curel, int &curface) {
+  double xi = unif_closed(rng);
+  const SourceRec &S = J.src[pick_source(J, xi)];
+  curel = S.mother;
+  curface = S.curface;
+  double wv = unif_open(rng);
+  pos[0] = S.v0[0] + wv * (S.v1[0] - S.v0[0]);
+  pos[1] = S.v0[1] + wv * (S.v1[1] - S.v0[1]);
+  const double n0 = S.n[0], n1 = S.n[1];
+  dir[0] = n0; dir[1] = n1;
+  const char bt = S.type, dt = S.dirtype;
+  if (bt == 'l') {
+    if (dt != 'n') { dir[0] = S.L[0]; dir[1] = S.L[1]; }
+  } else if (bt == 'i') {
+    if constexpr (kLiteral) {
+      double phi = kPi * (unif_open(rng) - 0.5);
+      sincos(S.phi0 + phi, &dir[1], &dir[0]);
+    } else {  // (U - 1/2) / 2 of a turn
+      double sp, cp;
+      const uint64_t u = ((uint64_t)rng.next() << 32) + 0x80000000u;
+      sincos_turn((uint64_t)((int64_t)(u ^ 0x8000000000000000ull) >> 1), sp, cp);
+      turned(S, sp, cp, dir);
+    }
+  } else if (bt == 'c' || bt == 'g') {
+    // direction type 'n': one draw; otherwise redraw until the direction points inward
+    // (MC2D.hpp:1085-1124)
+    for (int it = 0; it < kMaxRejections; it++) {
+      if (kLiteral || bt == 'g') {
+        double phi = (bt == 'c') ? asin(2.0 * unif_open(rng) - 1.0) : gauss_angle(rng, S.sigma, S.gauss_h);
+        sincos(S.phi0 + phi, &dir[1], &dir[0]);
+      } else {
+        double sp, cp;
+        open_sine(rng.next(), sp, cp);
+        turned(S, sp, cp, dir);
+      }
+      if (dt == 'n' || n0 * dir[0] + n1 * dir[1] > 0.0 || rng.exhausted()) break;
+    }
+  }
 }
 
 // 1 - exp(-mua ds) of an absorbing step (mua > 0)
