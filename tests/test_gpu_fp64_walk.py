@@ -110,3 +110,17 @@ def test_interfaces_and_launches(built, dim, source, n_out):
     for k in ("ER", "EBR", "DEBR"):
         a, b = getattr(gpu, k), getattr(ref, k)
         assert np.abs(a - b).sum() <= 1e-6 * np.abs(b).sum(), k
+
+
+@pytest.mark.parametrize("sigma", [0.02, 0.2, 1.0, 5.0, 100.0])
+def test_gaussian_launch_angles(built, sigma):
+    """The bisection's halvings are decided by the inverse error function where it is certain."""
+    p = problem(2, "slivers", False, 0.0)
+    p.BCType[p.BCType == ord("c")] = ord("g")
+    p.GaussianSigma = np.full(p.Nb, sigma)
+    gpu = V.run(p, precision=V.VMC_FP64)
+    ref = oracle.run(p, rng=oracle.RNG_PHILOX, nthreads=4)
+    assert (gpu.stats["steps"], gpu.stats["loss"]) == (ref.steps, ref.loss)
+    for k in ("ER", "EBR", "DEBR"):
+        a, b = getattr(gpu, k), getattr(ref, k)
+        assert np.abs(a - b).sum() <= 1e-6 * np.abs(b).sum(), k

@@ -288,6 +288,7 @@ JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, const 
   d.k_scale = j.k_scale;
   d.k_scale_f = (float)j.k_scale;
   d.phase0 = j.phase0;
+  d.phase_f = fmodf((float)j.phase0, 6.28318530717958647692f);
   d.k_turn = j.k_turn;
   d.turn0 = j.turn0;
   d.seed = j.seed;

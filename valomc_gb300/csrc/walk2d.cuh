@@ -676,7 +676,7 @@ struct Walk2D32 {
       outward = ln.x * dx + ln.y * dy > 0.0f;
     }
     w = 1.0f;
-    phase = fmodf(d2f_int(J.phase0), kTwoPiF);
+    phase = J.phase_f;
     float4 o = optics(J, el);
     mua = o.x; mus = o.y; g = o.z; nidx = o.w;
     prop = free_path_f(unif_open_f(rng), mus);
@@ -779,7 +779,6 @@ struct Walk2D32 {
     const Tri32 *T = reinterpret_cast<const Tri32 *>(J.geom) + el;
     const float4 *L4 = reinterpret_cast<const float4 *>(T->ln);
     const float4 l0 = __ldg(L4 + 0), l1 = __ldg(L4 + 1), l2 = __ldg(L4 + 2);
-    const int4 nb = __ldg(reinterpret_cast<const int4 *>(T->nbr));
     // selects over all three edges, no branch per edge; num / nd compared by cross
     // products, one reciprocal for the winning edge (bnd = 0: none yet)
     float bnum = 1.0f, bnd = 0.0f;
@@ -840,7 +839,7 @@ struct Walk2D32 {
       return res;
     }
     const float nx = lsel(l0, l1, l2, nf, 0), ny = lsel(l0, l1, l2, nf, 1);
-    const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nb.z;
+    const int nextel = __ldg(T->nbr + nf);
     const int ib = -1 - nextel;  // the boundary edge when nextel < 0
     const bool inside = nextel >= 0;
     if (nextel >= J.Ne) {

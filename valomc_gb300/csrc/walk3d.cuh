@@ -905,7 +905,7 @@ struct Walk3D32 {
       outward = pl.x * dx + pl.y * dy + pl.z * dz > 0.0f;
     }
     w = 1.0f;
-    phase = fmodf(d2f_int(J.phase0), kTwoPiF);
+    phase = J.phase_f;
     float4 o = optics(J, el);
     mua = o.x; mus = o.y; g = o.z; nidx = o.w;
     prop = free_path_f(unif_open_f(rng), mus);

@@ -199,15 +199,35 @@ __device__ __forceinline__ void create_photon_3d_f(const JobDev &J, R &rng, floa
   }
 }
 
+// The Gaussian launch angle: 16 bisections of its CDF.  Each needed an erf and two quotients; now
+// FP32's inverse x, with t = x / (sigma sqrt 2) = erfinv((2 xi - 1)(1 - 2 h)), decides the
+// halvings whose middle is further from it than the CDF's rounding (3e-7 of 0.5 + 0.5 erf) and
+// the inverse's own can move the root, and only the others, one launch in ten, are looked up: the
+// same angle, to the last bit.  333k photons on the uneven frequency-domain mesh 2.56 ->
+// 2.41 ms.
+struct GaussRoot {
+  float x, err;
+  __device__ __forceinline__ GaussRoot(float xi, float sigma, float h) {
+    const float t = erfinvf((2.0f * xi - 1.0f) * (1.0f - 2.0f * h));
+    x = 1.41421356f * sigma * t;
+    err = 4e-6f * fabsf(sigma) * __expf(t * t) + 2e-6f * fabsf(x) + 1e-7f;
+  }
+  __device__ __forceinline__ bool sure(float phi) const { return fabsf(phi - x) > err; }  // not for NaN, inf
+};
 template <class R>
 __device__ __forceinline__ float gauss_angle_f(R &rng, float sigma, float h) {
   const float xi = unif_open_f(rng);
+  const GaussRoot root(xi, sigma, h);
   float a = -0.5f * (float)kPi, b = 0.5f * (float)kPi, phi = 0.0f;
 #pragma unroll 1
   for (int it = 0; it < 16; it++) {
     phi = 0.5f * (a + b);
-    const float cdf = (0.5f + 0.5f * erff(phi / sigma * 0.70710678118654752f) - h) / (1.0f - 2.0f * h);
-    if (cdf - xi < 0.0f) a = phi;
+    bool low = phi < root.x;
+    if (!root.sure(phi)) {
+      const float cdf = (0.5f + 0.5f * erff(phi / sigma * 0.70710678118654752f) - h) / (1.0f - 2.0f * h);
+      low = cdf - xi < 0.0f;
+    }
+    if (low) a = phi;
     else b = phi;
   }
   return phi;
@@ -415,12 +435,19 @@ __device__ __forceinline__ void create_photon_3d(const JobDev &J, R &rng, double
 template <class R>
 __device__ double gauss_angle(R &rng, double sigma, double h) {
   double xi = unif_open(rng);
+  const GaussRoot root((float)xi, (float)sigma, (float)h);
   double a = -kPi / 2, b = kPi / 2, phi = 0.0;
   const double isq2 = sqrt(2.0);
+#pragma unroll 1
   for (int it = 0; it < 16; it++) {
-    phi = (a + b) / 2.0;
-    double cdf = (0.5 + 0.5 * erf(phi / sigma / isq2) - h) / (1 - 2.0 * h);
-    if (cdf - xi < 0.0) a = phi;
+    phi = (a + b) * 0.5;
+    const float f = f32_of(phi);
+    bool low = f < root.x;
+    if (!root.sure(f)) {
+      double cdf = (0.5 + 0.5 * erf(phi / sigma / isq2) - h) / (1 - 2.0 * h);
+      low = cdf - xi < 0.0;
+    }
+    if (low) a = phi;
     else b = phi;
   }
   return phi;
