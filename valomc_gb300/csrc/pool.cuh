@@ -6,10 +6,11 @@
 // chunk of the global photon counter (one atomic per chunk), once refill_min lanes are
 // idle or on every 8th iteration, so a warp never runs half-empty for long while photons
 // remain.  A one-job launch on a small mesh stages the job's accumulators in shared memory
-// (LaunchParams::dense) and adds them to the job's arrays when the CTA ends.  A photon index selects its job (batched launches),
-// its Philox stream (key = job seed, counter = photon index) or its tape segment, and the
-// walk advances one element step per loop iteration.  Each loop iteration polls nothing
-// but registers; the host cancel flag is read every 1024 iterations.
+// (LaunchParams::dense) and adds them to the job's arrays when the CTA ends.  A photon index
+// selects its job (batched launches), its Philox stream (key = job seed, counter = photon
+// index) or its tape segment, and the walk advances one element step per loop iteration.
+// Each loop iteration polls nothing but registers; the host cancel flag is read every 1024
+// iterations.
 #pragma once
 #include "walk2d.cuh"
 
@@ -255,7 +256,19 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
       }
     }
     if (!W::kPack && chunk_left < 0 && !__any_sync(kFull, alive)) break;
-    if (alive) {
+    const bool was = alive;
+    // Events (W::kDefer): what a step ends in besides a scatter and a common crossing, the
+    // boundary, an interface, roulette, takes as many instructions as several steps, and with a few
+    // of 32 lanes at it a warp paid for it in nearly every step.  Lanes with an event wait until
+    // they are a quarter of the warp's live ones.  1e6 photons on the 2D square, which meet one
+    // every ten steps, 0.855 -> 0.705 ms (an eighth: 0.76, a third: 0.72), in FP64 5.8 -> 5.1;
+    // uneven 2D mesh 2.35 -> 2.31 and 4.3 -> 3.9; a small tetrahedral box in FP64 7.0 -> 6.3.  The
+    // FP32 tetrahedral walk, with one in a hundred steps, loses more by the waiting (1e7 photons on
+    // the phantom 187 -> 220 ms, at a sixteenth 199) and does without; so would a mesh whose
+    // index of refraction changes at every face (0.59 -> 0.65 ms; 0.70 before these forms).
+    bool waits = false;
+    if constexpr (W::kDefer) waits = s.pending();
+    if (alive && !waits) {
       if constexpr (W::kCap32) {
         alive = s.step(*J, rng, cap, n_scat);
       } else {
@@ -263,11 +276,18 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
         n_scat += r == kScattered;
         alive = r <= kAliveMax;
       }
-      if (!alive) {
-        n_done++;
-        n_steps += (uint32_t)s.nsteps;
-        job_count_add(*J, kJcSteps, (unsigned long long)s.nsteps);
+    }
+    if constexpr (W::kDefer) {
+      const bool event = alive && s.pending();
+      const unsigned events = __ballot_sync(kFull, event);
+      if (events && 4 * __popc(events) >= __popc(__ballot_sync(kFull, alive))) {
+        if (event) alive = s.event(*J, rng, cap, n_scat);
       }
+    }
+    if (was && !alive) {
+      n_done++;
+      n_steps += (uint32_t)s.nsteps;
+      job_count_add(*J, kJcSteps, (unsigned long long)s.nsteps);
     }
   }
   if constexpr (W::kStaged) {

@@ -33,6 +33,8 @@ struct Walk2D64 {
   static constexpr bool kBuffered = false;
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = true;
+  static constexpr bool kDefer = true;
+  __device__ __forceinline__ bool pending() const { return pend != 0; }
   static constexpr int kMinBlocks = 2;
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
@@ -46,12 +48,13 @@ struct Walk2D64 {
   uint64_t turn;  // phase in 2^-64 turns
   int el, curface;
   int32_t nsteps;
+  int pend;  // event to come: 1 + the face crossed, 0 none
   Tr tr;
 
   // moves the photon's state between lanes (Packer)
   template <class F> __device__ __forceinline__ void move(const F &f) {
-    if constexpr (FD) f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, imus, kg, acc, turn, cph, sph, accI, el, curface, nsteps);
-    else f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, imus, kg, acc, el, curface, nsteps);
+    if constexpr (FD) f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, imus, kg, acc, turn, cph, sph, accI, el, curface, nsteps, pend);
+    else f(pos[0], pos[1], dir[0], dir[1], w, prop, mua, mus, g, nidx, imus, kg, acc, el, curface, nsteps, pend);
   }
 
   __device__ __forceinline__ static const TriRec *recs(const JobDev &J) { return reinterpret_cast<const TriRec *>(J.geom); }
@@ -82,6 +85,7 @@ struct Walk2D64 {
     prop = neg_log_open(rng.next()) * imus;
     acc = accI = 0.0;
     nsteps = 0;
+    pend = 0;
   }
 
   __device__ __forceinline__ void flush(const JobDev &J) {
@@ -268,7 +272,6 @@ struct Walk2D64 {
       cph = cn; sph = sn;
       w *= att;
     }
-    bool on = true;
     if (ends) {
       if (positive(mus)) {
         const Event ev = draw_event(rng.peek3());
@@ -287,8 +290,45 @@ struct Walk2D64 {
     } else {
       prop -= dist;
       const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nb.z;
-      on = cross(J, rng, nf, nextel);
+      if (!cross_on(J, nextel)) {
+        pend = 1 + nf;
+        return true;
+      }
     }
+    if (nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
+      job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
+      return die(J, kEvCapped);
+    }
+    return true;
+  }
+
+  // The common crossing: into an element that scatters, no index jump, weight above the roulette
+  // threshold.
+  __device__ __forceinline__ bool cross_on(const JobDev &J, int nextel) {
+    if ((unsigned)nextel >= (unsigned)J.Ne) return false;
+    double mua2, mus2, g2, n2;
+    optics(J, nextel, mua2, mus2, g2, n2);
+    if (!positive(mus) || differ(nidx, n2) || below(w, kWeight0)) return false;
+    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((recs(J) + nextel)->nbr));
+    const int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : -1;
+    if (f2 < 0) return false;
+    if (differ(mus2, mus)) {
+      prop *= mus / mus2;  // x (mus / mus) == x
+      imus = fast_rcp(mus2);
+    }
+    if (differ(g2, g)) kg = turn_ratio(g2);
+    flush(J);
+    curface = f2;
+    el = nextel;
+    mua = mua2; mus = mus2; g = g2; nidx = n2;
+    return true;
+  }
+
+  // What else lies behind face pend - 1, for several lanes of a warp together.
+  __device__ __forceinline__ bool event(const JobDev &J, R &rng, int32_t cap, uint32_t &) {
+    const int nf = pend - 1;
+    pend = 0;
+    const bool on = cross(J, rng, nf, __ldg((recs(J) + el)->nbr + nf));
     if (on && nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
       job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
       return die(J, kEvCapped);
@@ -379,6 +419,7 @@ struct Walk2D64L {
   static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = false;
+  static constexpr bool kDefer = false;
   static constexpr int kMinBlocks = 2;
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
@@ -638,6 +679,8 @@ struct Walk2D32 {
   static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
   static constexpr bool kPack = false;  // its walks are short: packing gains nothing and costs the loop 2 %
   static constexpr bool kCap32 = false;
+  static constexpr bool kDefer = true;
+  __device__ __forceinline__ bool pending() const { return pend != 0; }
   static constexpr int kMinBlocks = 4;
   static constexpr bool kStaged = false;
   Stage stage;
@@ -648,6 +691,7 @@ struct Walk2D32 {
   float acc, accI;
   int el;
   int32_t nsteps;
+  int pend;  // event to come: 1 + the edge crossed, 4 for the end of the free path, 0 none
   bool outward;  // launched out through its own entry edge
   Tr tr;
 
@@ -682,6 +726,7 @@ struct Walk2D32 {
     prop = free_path_f(unif_open_f(rng), mus);
     acc = accI = 0.0f;
     nsteps = 0;
+    pend = 0;
   }
 
   __device__ __forceinline__ void flush(const JobDev &J) {
@@ -759,11 +804,6 @@ struct Walk2D32 {
     return false;
   }
 
-  __device__ __forceinline__ static float lsel(const float4 &a, const float4 &b, const float4 &c, int f, int k) {
-    const float4 &q = f == 0 ? a : f == 1 ? b : c;
-    return k == 0 ? q.x : k == 1 ? q.y : q.z;
-  }
-
   __device__ int step(const JobDev &J, R &rng, int64_t max_steps) {
     if (rng.exhausted()) { job_count(J, kJcTapeEnd); die(J, kEvTapeEnd); return kDiedEarly; }
     if (nsteps >= max_steps) {
@@ -838,31 +878,45 @@ struct Walk2D32 {
       prop = free_path_f(unif_open_f(rng), mus);
       return res;
     }
-    const float nx = lsel(l0, l1, l2, nf, 0), ny = lsel(l0, l1, l2, nf, 1);
+    // the common crossing (scattering medium, weight above the roulette threshold, no index jump)
+    const int nextel = __ldg(T->nbr + nf);
+    if ((unsigned)nextel < (unsigned)J.Ne && mus > 0.0f && w >= (float)kWeight0) {
+      const float4 o2 = optics(J, nextel);
+      if (nidx == o2.w) {
+        if (o2.y != mus) prop *= mus / o2.y;
+        flush(J);
+        el = nextel;
+        mua = o2.x; mus = o2.y; g = o2.z;
+        return kAlive;
+      }
+    }
+    pend = 1 + nf;
+    return kAlive;
+  }
+
+  // What is left of a step that ends in neither: run for several lanes of a warp together.
+  __device__ __forceinline__ bool event(const JobDev &J, R &rng, int32_t, uint32_t &) {
+    const int nf = pend - 1;
+    pend = 0;
+    const Tri32 *T = reinterpret_cast<const Tri32 *>(J.geom) + el;
+    const float2 line = __ldg(reinterpret_cast<const float2 *>(T->ln[nf]));
+    const float nx = line.x, ny = line.y;
     const int nextel = __ldg(T->nbr + nf);
     const int ib = -1 - nextel;  // the boundary edge when nextel < 0
     const bool inside = nextel >= 0;
     if (nextel >= J.Ne) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
-      return die(J, kEvLost);
+      die(J, kEvLost);
+      return false;
     }
     float4 o2 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (inside) {
       o2 = optics(J, nextel);
-      // the common crossing (scattering medium, weight above the roulette threshold, no index
-      // jump) tested at once
-      if (mus > 0.0f && w >= (float)kWeight0 && nidx == o2.w) {
-        if (o2.y != mus) prop *= mus / o2.y;
-        flush(J);
-        el = nextel;
-        mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;
-        return kAlive;
-      }
     } else {
       if (is_mirror(__ldg(J.bctype + ib))) {
         const float dn = fmaf(dy, ny, __fmul_rn(dx, nx));
         dx -= 2.0f * dn * nx; dy -= 2.0f * dn * ny;
-        return kAlive;
+        return true;
       }
       o2.w = d2f_int(__ldg(J.bcn + ib));
     }
@@ -870,8 +924,11 @@ struct Walk2D32 {
     // Philox block per draw, and the kernel waits for instructions as it is
     const bool vacuum = inside && mus <= 0.0f && o2.y > 0.0f;
     if (vacuum) prop = free_path_f(unif_open_f(rng), o2.y);
-    if (inside && roulette(J, rng)) return die(J, kEvRoulette);
-    if ((inside ? nidx != o2.w : o2.w > 0.0f) && fresnel(rng, nx, ny, nidx / o2.w, !inside)) return kAlive;
+    if (inside && roulette(J, rng)) {
+      die(J, kEvRoulette);
+      return false;
+    }
+    if ((inside ? nidx != o2.w : o2.w > 0.0f) && fresnel(rng, nx, ny, nidx / o2.w, !inside)) return true;
     if (!inside) {
       const float dn = fmaf(dy, ny, __fmul_rn(dx, nx));
       flush(J);
@@ -888,13 +945,13 @@ struct Walk2D32 {
       }
       tr.put(-1 - (int64_t)ib);
       tr.end();
-      return kDied;
+      return false;
     }
     if (!vacuum && o2.y != mus) prop *= mus / o2.y;
     flush(J);
     el = nextel;
     mua = o2.x; mus = o2.y; g = o2.z; nidx = o2.w;
-    return kAlive;
+    return true;
   }
 };
 

@@ -182,6 +182,8 @@ struct Walk3D64 {
   static constexpr bool kBuffered = false;  // a block's words are drawn again rather than carried
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = true;
+  static constexpr bool kDefer = true;
+  __device__ __forceinline__ bool pending() const { return pend != 0; }
   static constexpr int kMinBlocks = 2;
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
@@ -195,12 +197,13 @@ struct Walk3D64 {
   uint64_t turn;  // phase in 2^-64 turns
   int el, curface;
   int32_t nsteps;
+  int pend;  // event to come: 1 + the face crossed, 0 none
   Tr tr;
 
   // moves the photon's state between lanes (Packer)
   template <class F> __device__ __forceinline__ void move(const F &f) {
-    if constexpr (FD) f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, imus, ig, acc, turn, cph, sph, accI, el, curface, nsteps);
-    else f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, imus, ig, acc, el, curface, nsteps);
+    if constexpr (FD) f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, imus, ig, acc, turn, cph, sph, accI, el, curface, nsteps, pend);
+    else f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, imus, ig, acc, el, curface, nsteps, pend);
   }
 
   __device__ __forceinline__ static const TetRec *recs(const JobDev &J) { return reinterpret_cast<const TetRec *>(J.geom); }
@@ -226,6 +229,7 @@ struct Walk3D64 {
     prop = neg_log_open(rng.next()) * imus;  // the outer loop's first draw, MC3D.hpp:1458
     acc = accI = 0.0;
     nsteps = 0;
+    pend = 0;
   }
 
   __device__ __forceinline__ void flush(const JobDev &J) {
@@ -457,7 +461,6 @@ struct Walk3D64 {
       cph = cn; sph = sn;
       w *= att;
     }
-    bool on = true;
     if (ends) {
       if (positive(mus)) {
         const Event ev = draw_event(rng.peek3());
@@ -477,8 +480,45 @@ struct Walk3D64 {
     } else {
       prop -= dist;
       const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nf == 2 ? nb.z : nb.w;
-      on = cross(J, rng, nf, nextel);
+      if (!cross_on(J, nextel)) {
+        pend = 1 + nf;
+        return true;
+      }
     }
+    if (nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
+      job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
+      return die(J, kEvCapped);
+    }
+    return true;
+  }
+
+  // The common crossing: into an element that scatters, no index jump, weight above the roulette
+  // threshold.
+  __device__ __forceinline__ bool cross_on(const JobDev &J, int nextel) {
+    if ((unsigned)nextel >= (unsigned)J.Ne) return false;
+    double mua2, mus2, g2, n2;
+    optics(J, nextel, mua2, mus2, g2, n2);
+    if (!positive(mus) || differ(nidx, n2) || below(w, kWeight0)) return false;
+    const int4 nb2 = __ldg(reinterpret_cast<const int4 *>((recs(J) + nextel)->nbr));
+    const int f2 = nb2.x == el ? 0 : nb2.y == el ? 1 : nb2.z == el ? 2 : nb2.w == el ? 3 : -1;
+    if (f2 < 0) return false;
+    if (differ(mus2, mus)) {
+      prop *= mus / mus2;  // x (mus / mus) == x
+      imus = fast_rcp(mus2);
+    }
+    if (differ(g2, g)) ig = hg_inverse(g2);
+    flush(J);
+    curface = f2;
+    el = nextel;
+    mua = mua2; mus = mus2; g = g2; nidx = n2;
+    return true;
+  }
+
+  // What else lies behind face pend - 1, for several lanes of a warp together.
+  __device__ __forceinline__ bool event(const JobDev &J, R &rng, int32_t cap, uint32_t &) {
+    const int nf = pend - 1;
+    pend = 0;
+    const bool on = cross(J, rng, nf, __ldg((recs(J) + el)->nbr + nf));
     if (on && nsteps >= cap && !rng.exhausted()) {  // a tape that ends here is reported as that
       job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
       return die(J, kEvCapped);
@@ -563,6 +603,7 @@ struct Walk3D64L {
   static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = false;
+  static constexpr bool kDefer = false;
   static constexpr int kMinBlocks = 2;  // ~125 registers: 2 CTAs of 256 per SM
   static constexpr bool kStaged = false;
   static constexpr bool kLaunchLoss = false;
@@ -844,6 +885,7 @@ struct Walk3D32 {
   static constexpr bool kBuffered = false;  // a block's words are drawn again rather than carried
   static constexpr bool kPack = true;
   static constexpr bool kCap32 = true;
+  static constexpr bool kDefer = false;
   using Tr = typename TraceFor<R>::type;
   float px, py, pz, dx, dy, dz;
   float w, prop, phase;
