@@ -477,6 +477,15 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
   // optics rows; a job whose elements all share one row keeps a single row
   j.homogeneous = Ne > 0 && uniform(in->mua, Ne) && uniform(in->mus, Ne) && uniform(in->g, Ne) && uniform(in->n, Ne);
   j.mua = in->mua; j.mus = in->mus; j.g = in->g; j.n = in->n;
+  {  // from up to 64 elements across the mesh
+    double a = 0, s = 0;
+    for (int64_t k = 0, i = 0; k < 64 && i < Ne; k++, i = Ne / 64 * k + std::min<int64_t>(k, Ne % 64)) {
+      a += fabs(j.mua[i]);
+      s += fabs(j.mus[i]);
+    }
+    const double w = s / a;
+    j.walk = w >= 0 ? (float)std::min(w, 1e30) : 0.0f;
+  }
   j.bctype.assign(reinterpret_cast<const uint8_t *>(in->BCType), reinterpret_cast<const uint8_t *>(in->BCType) + Nb);
   j.bcn.assign(in->BCn, in->BCn + Nb);
   // BCLightDirectionType defaults to 'n' (MC3D.hpp:646-654), BCLNormal is normalised

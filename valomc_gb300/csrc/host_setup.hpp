@@ -92,6 +92,7 @@ struct HostJob {
   uint64_t turn0 = 0;           // phase0 in 2^-64 turns
   int64_t Nphoton = 0;
   uint64_t seed = 0;
+  float walk = 0;               // about how long its walks are: scatterings per absorption length
 };
 
 // Whether the scattering coefficient or the index changes across more than an eighth of the mesh's

@@ -208,6 +208,7 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   d.k_scale_f = (float)hj.k_scale;
   d.phase0 = hj.phase0;
   d.phase_f = fmodf((float)hj.phase0, 6.28318530717958647692f);
+  d.walk = hj.walk;
   d.k_turn = hj.k_turn;
   d.turn0 = hj.turn0;
   d.seed = hj.seed;

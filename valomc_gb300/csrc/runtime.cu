@@ -289,6 +289,7 @@ JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, const 
   d.k_scale_f = (float)j.k_scale;
   d.phase0 = j.phase0;
   d.phase_f = fmodf((float)j.phase0, 6.28318530717958647692f);
+  d.walk = j.walk;
   d.k_turn = j.k_turn;
   d.turn0 = j.turn0;
   d.seed = j.seed;
@@ -453,6 +454,11 @@ int plan_launch(int device, const LaunchSpec &spec, const std::vector<JobDev> &j
   if (!p.fn) { set_error("no kernel for this configuration"); return VMC_ERR_INVALID_ARGUMENT; }
   reset_carveout(p.fn);
   p.jobs = jobs_in;
+  // The jobs with the longest walks first: photons are handed out in this order, and a launch ends
+  // when the last of them has been walked.  Ten cubes of different optics 52.5 -> 47.6, 41.4 ->
+  // 41.4, 44.0 -> 43.7 and 75.0 -> 71.0 ms (the longest last: 52.8, 47.4, 50.0, 82.2), twenty
+  // served requests 72.8 -> 69.5, 62.3 -> 53.6, 55.0 -> 53.6, 64.8 -> 57.9.
+  std::stable_sort(p.jobs.begin(), p.jobs.end(), [](const JobDev &a, const JobDev &b) { return a.walk > b.walk; });
   p.begin.assign(p.jobs.size() + 1, 0);
   for (size_t i = 0; i < p.jobs.size(); i++) {
     p.jobs[i].pbegin = p.begin[i];

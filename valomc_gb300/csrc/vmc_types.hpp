@@ -147,6 +147,7 @@ struct JobDev {
   int32_t dense;               // > 0: the launch stages the 2 Ne + 4 Nb accumulators per CTA in shared memory
   double phase0;
   float phase_f;               // the same modulo 2 pi in FP32, for the tracking form
+  float walk;                  // HostJob::walk
   double k_turn;               // k_scale / (2 pi), and phase0 in 2^-64 turns: the plain form's phase
   uint64_t turn0;
   uint64_t seed;
