@@ -196,14 +196,16 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   d.Ns = (int32_t)ns;
   d.Ne = (int32_t)Ne;
   d.Nb = (int32_t)Nb;
-  d.cdf = reinterpret_cast<const double *>(base + kOffCdf);
-  d.src = reinterpret_cast<const SourceRec *>(base + kOffSrc);
-  d.cdf_f = reinterpret_cast<const float *>(base + kOffCdfF);
-  d.src_f = reinterpret_cast<const SourceRecF *>(base + kOffSrcF);
+  if (o.precision == VMC_FP64) {
+    d.cdf = reinterpret_cast<const double *>(base + kOffCdf);
+    d.src = reinterpret_cast<const SourceRec *>(base + kOffSrc);
+  } else {
+    d.cdf_f = reinterpret_cast<const float *>(base + kOffCdfF);
+    d.src_f = reinterpret_cast<const SourceRecF *>(base + kOffSrcF);
+  }
   d.bctype = dev->bctype;
   d.bcn = dev->bcn;
   d.bnorm = m->d_bnorm;
-  d.omega = hj.omega;
   d.k_scale = hj.k_scale;
   d.k_scale_f = (float)hj.k_scale;
   d.phase0 = hj.phase0;

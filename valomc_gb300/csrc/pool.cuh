@@ -266,9 +266,12 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
     // FP32 tetrahedral walk, with one in a hundred steps, loses more by the waiting (1e7 photons on
     // the phantom 187 -> 220 ms, at a sixteenth 199) and does without; so would a mesh whose
     // index of refraction changes at every face (0.59 -> 0.65 ms; 0.70 before these forms).
-    bool waits = false;
-    if constexpr (W::kDefer) waits = s.pending();
-    if (alive && !waits) {
+    const auto ended = [&] {
+      n_done++;
+      n_steps += (uint32_t)s.nsteps;
+      job_count_add(*J, kJcSteps, (unsigned long long)s.nsteps);
+    };
+    const auto step = [&] {
       if constexpr (W::kCap32) {
         alive = s.step(*J, rng, cap, n_scat);
       } else {
@@ -276,18 +279,19 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
         n_scat += r == kScattered;
         alive = r <= kAliveMax;
       }
-    }
+    };
     if constexpr (W::kDefer) {
+      const bool was = alive;
+      if (alive && !s.pending()) step();
       const bool event = alive && s.pending();
       const unsigned events = __ballot_sync(kFull, event);
       if (events && 4 * __popc(events) >= __popc(__ballot_sync(kFull, alive))) {
         if (event) alive = s.event(*J, rng, cap, n_scat);
       }
-    }
-    if (was && !alive) {
-      n_done++;
-      n_steps += (uint32_t)s.nsteps;
-      job_count_add(*J, kJcSteps, (unsigned long long)s.nsteps);
+      if (was && !alive) ended();
+    } else if (alive) {
+      step();
+      if (!alive) ended();
     }
   }
   if constexpr (W::kStaged) {

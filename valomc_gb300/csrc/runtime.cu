@@ -277,14 +277,16 @@ JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, const 
   d.Ns = (int32_t)j.src.size();
   d.Ne = (int32_t)Ne;
   d.Nb = (int32_t)Nb;
-  d.cdf = b.d_cdf;
-  d.src = b.d_src;
-  d.cdf_f = b.d_cdf_f;
-  d.src_f = b.d_src_f;
+  if (precision == VMC_FP64) {
+    d.cdf = b.d_cdf;
+    d.src = b.d_src;
+  } else {
+    d.cdf_f = b.d_cdf_f;
+    d.src_f = b.d_src_f;
+  }
   d.bctype = b.d_bctype;
   d.bcn = b.d_bcn;
   d.bnorm = m.d_bnorm;
-  d.omega = j.omega;
   d.k_scale = j.k_scale;
   d.k_scale_f = (float)j.k_scale;
   d.phase0 = j.phase0;

@@ -125,8 +125,11 @@ constexpr int kSlots = 64;
 constexpr int kDefaultRefill = 4;
 // largest accumulator set (2 Ne + 4 Nb doubles) a launch stages whole in each CTA's shared memory
 constexpr int64_t kDenseStageBytes = 32 * 1024;
-// largest job table a multi-job launch copies into each CTA's shared memory
-constexpr int kSmemJobs = 64;
+// Largest job table a multi-job launch copies into each CTA's shared memory.  The walk keeps a
+// job's hot fields in registers, and what the tables of four CTAs take the L1 loses: two jobs on
+// the phantom 36.9 ms with the table and 37.4 without, ten cubes 41.25 and 41.26, 64 cubes of up to
+// 3 million tetrahedra (table 17 KB, L1 128 KB of an SM's 228) 310 and 303.
+constexpr int kSmemJobs = 16;
 
 struct JobDev {
   const void *geom;            // Tet64 / Tet32 / Tri64 / Tri32 [Ne]
@@ -134,14 +137,17 @@ struct JobDev {
   int32_t opt_mask;            // -1: per element, 0: one homogeneous row
   int32_t Ns;                  // emitting faces
   int32_t Ne, Nb;
-  const double *cdf;           // [Ns]
-  const SourceRec *src;        // [Ns]
-  const float *cdf_f;          // [Ns] FP32 copies for the tracking form
-  const SourceRecF *src_f;     // [Ns]
+  union {                      // [Ns], FP32 copies for the tracking form
+    const double *cdf;
+    const float *cdf_f;
+  };
+  union {
+    const SourceRec *src;
+    const SourceRecF *src_f;
+  };
   const uint8_t *bctype;       // [Nb]
   const double *bcn;           // [Nb]
   const double *bnorm;         // [Nb x 4] Normal(ib) for MirrorPhoton (FP64 forms)
-  double omega;                // 2 pi f
   double k_scale;              // omega / c0: k = k_scale * n  (cpp/3d/MC3D.hpp:662)
   float k_scale_f;             // the same in FP32, for the tracking form
   int32_t dense;               // > 0: the launch stages the 2 Ne + 4 Nb accumulators per CTA in shared memory
@@ -163,6 +169,7 @@ struct JobDev {
   unsigned long long *jc;      // [kSlots x kJcN]
   double *ledger;              // [kSlots x kLgN]
 };
+static_assert(sizeof(JobDev) <= 272, "the job tables take their room from the L1");
 static_assert(sizeof(JobDev) % sizeof(uint64_t) == 0, "JobDev is copied as 8-byte words");
 
 // Launch-wide control block in device memory.
