@@ -68,7 +68,9 @@ enum vmc_status {
 
 /* arithmetic form of the photon walk */
 enum vmc_precision {
-  VMC_FP64 = 0, /* plain form: the reference's FP64 arithmetic and Moller-Trumbore face test */
+  VMC_FP64 = 0, /* plain form: FP64 state, the exit faces of the reference's Moller-Trumbore test
+                   and its draws; the reference's operations one by one where a mesh's optics
+                   change at most faces */
   VMC_FP32 = 1  /* tracking form: FP32 position/direction/weight, barycentric (plane)
                    exit test robust to rounding, FP64 accumulators */
 };
