@@ -335,3 +335,23 @@ def test_photons_dealt_and_moved_between_lanes_walk_alike(built, name, precision
     if p.f == 0.0 or precision == V.VMC_FP64:  # the FP32 one-job form rounds the phase differently
         np.testing.assert_allclose(both[0].EBR, parts[0].EBR, rtol=1e-9, atol=1e-9)
     mesh.close()
+
+
+@pytest.mark.parametrize("block", [32, 64, 96])
+@pytest.mark.parametrize("name,precision,n", [("phantom3d", V.VMC_FP32, 20000), ("phantom3d_fd", V.VMC_FP32, 6001),
+                                              ("phantom3d", V.VMC_FP64, 5000), ("mixed2d_fd", V.VMC_FP64, 5003)])
+def test_blocks_of_few_warps_lose_no_photon(built, name, precision, n, block):
+    """CTAs of one to three warps pack their last photons without dropping one: the walks of the
+    default block, in steps, scatters and sums."""
+    p = cases()[name][0].copy(Nphoton=n, seed=31)
+    want = V.run(p, precision=precision, normalize=False)
+    one = V.run(p, precision=precision, normalize=False, block_size=block)
+    assert one.stats["photons_done"] == want.stats["photons_done"] == n
+    assert one.stats["steps"] == want.stats["steps"] and one.stats["scatters"] == want.stats["scatters"]
+    for k in ("ER", "EI", "EBR", "EBI"):
+        np.testing.assert_allclose(getattr(one, k), getattr(want, k), rtol=1e-9, atol=1e-9)
+    mesh = V.Mesh(p, precision=precision)
+    _, st = V.run_batch([mesh, mesh], [p.copy(Nphoton=n // 3), p.copy(Nphoton=n - n // 3)], precision=precision,
+                        block_size=block)
+    assert st["photons_done"] == n
+    mesh.close()

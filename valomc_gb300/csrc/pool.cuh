@@ -198,12 +198,11 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
             used += c > 0;
           }
           if (all == 0 && !pending) break;
-          const int want = all <= 3 ? all : max((all + 31) >> 5, 2);
+          const int want = pack_warps(all, warps);
           if constexpr (!R::kReplay) {
             if (!pending && (used < want || 4 * want <= 3 * used)) {
-              const int each = (all + want - 1) / want;
               const int k = before + __popc(live & lt_mask);
-              const int to = alive ? ((k / each + warp_turn(lp, warps)) % warps) * 32 + k % each : -1;
+              const int to = alive ? pack_thread(k, all, want, warp_turn(lp, warps), warps) : -1;
               auto slot = rng.take_slot();  // the lanes' stream slots are the buffer
               const Packer<decltype(slot)> pack(rng.slots(), to);
               s.move(pack);

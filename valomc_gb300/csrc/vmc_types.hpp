@@ -192,6 +192,20 @@ VMC_HD inline int32_t fill_of(int64_t total, int sms) {
   return (int32_t)(n < 1 ? 1 : n > 32 ? 32 : n);
 }
 
+// The warps of a CTA that its `all` live photons are moved to when lanes are packed: full ones, but
+// two while there are more than three photons, and one each for the last three, as far as the CTA
+// has so many warps.
+VMC_HD inline int pack_warps(int all, int warps) {
+  const int want = all <= 3 ? all : all <= 64 ? 2 : (all + 31) >> 5;
+  return want < warps ? want : warps;
+}
+// the thread that the k-th of them is moved to; `want` = pack_warps(all, warps), and the first of
+// those warps is warp `turn`
+VMC_HD inline int pack_thread(int k, int all, int want, int turn, int warps) {
+  const int each = (all + want - 1) / want;
+  return ((k / each + turn) % warps) * 32 + k % each;
+}
+
 struct LaunchParams {
   const JobDev *jobs;
   const int64_t *job_begin;   // [njobs + 1] prefix of photon counts
