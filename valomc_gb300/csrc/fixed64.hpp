@@ -296,10 +296,11 @@ VMC_HD inline double one_minus_exp_over_x(double x) {
   return e == 0 ? 1.0 : double_of_fixed((uint64_t)0 - e, 0);
 }
 
-struct LogEntry {
+struct alignas(16) LogEntry {  // read by one 16-byte load
   uint64_t log_r;  // log(r / 256) 2^63
   uint64_t r;      // 256 / (the interval's middle), rounded: 256 at the end, where log is 0
 };
+static_assert(alignof(LogEntry) == 16 && sizeof(LogEntry) == 16, "LogEntry is loaded as 16 bytes");
 #ifdef __CUDACC__
 __device__
 #endif
