@@ -174,38 +174,50 @@ inline float near_rcp(float x) { return 1.0f / x; }
 inline float near_rsqrt(float x) { return 1.0f / sqrtf(x); }
 #endif
 
-// 1 / (d 2^-64) in units of 2^-61, d >= 2^63: an FP32 quotient y0 and what 1 - d y0 = e leaves of
-// it, y0 (1 + e + e^2), |e| < 2^-22
-VMC_HD inline uint64_t rcp_fixed(uint64_t d) {
-  const int32_t y0 = (int32_t)(near_rcp((float)(uint32_t)(d >> 32)) * 2305843009213693952.0f);  // 2^-29
+// 1 / (d 2^-64) in units of 2^-61, d >= 2^63: an FP32 quotient y of d's upper half and what
+// 1 - d y = e leaves of it, y (1 + e + e^2).  |e| < 2^-21 by the conversion of the upper half
+// (2^-24) and the quotient's documented error of an ulp; the shift leaves room for 2^-21.
+VMC_HD inline uint64_t rcp_refined(uint64_t d, float y) {
+  const int32_t y0 = (int32_t)(y * 2305843009213693952.0f);  // 2^-29
   const uint64_t p = (d >> 32) * (uint32_t)y0 + (((uint64_t)(uint32_t)d * (uint32_t)y0) >> 32);
   const int64_t e = (int64_t)(0x2000000000000000ull - p);  // 2^-61
-  const int32_t e5 = (int32_t)(e >> 8);                    // 2^-53
-  const int64_t t = e + (wide(e5, e5) >> 45);
+  const int32_t e5 = (int32_t)(e >> 9);                    // 2^-52
+  const int64_t t = e + (wide(e5, e5) >> 43);
   return ((uint64_t)y0 << 32) + (uint64_t)((wide(y0, (int32_t)(t >> 15)) >> 14) + (wide(y0, (int32_t)(t & 0x7fff)) >> 29));
 }
+VMC_HD inline float rcp_first(uint64_t d) { return near_rcp((float)(uint32_t)(d >> 32)); }
+VMC_HD inline uint64_t rcp_fixed(uint64_t d) { return rcp_refined(d, rcp_first(d)); }
 
-// sqrt(s) 2^-k and 2^k / sqrt(s), s > 0, both in [1/2, 2]: h = s y0 from an FP32 y0, then with
-// e = 1 - h y0 both times 1 + e / 2 + 3 e^2 / 8, |e| < 2^-21
+// sqrt(s) 2^-k and 2^k / sqrt(s), s > 0, both in [1/2, 2]: h = t y from t = s 4^k, brought to
+// [1/4, 1] or less than a unit above, and an FP32 y = 1 / sqrt(t); then with e = 1 - h y both
+// times 1 + e / 2 + 3 e^2 / 8.  Two ulps of the root's documented error, t's conversion and the
+// cut of y to 2^-29 make |e| < 5.5e-7; the shift leaves room for 2^-20.
 struct Root60 {
   int64_t r, y;
   int k;
 };
-VMC_HD inline Root60 sqrt60(int64_t s) {
-  const int k = (clz_u64((uint64_t)s | 1u) - (s >> 60 ? 3 : 4)) >> 1;  // s = 1 is 2^60: none
-  const int64_t t = s << (2 * k);  // [1/4, 1] or less than a unit above
-  const int32_t y0 = (int32_t)(near_rsqrt((float)(uint32_t)(t >> 29) * 4.656612873077393e-10f) * 536870912.0f);  // 2^-29
+VMC_HD inline int root_shift(int64_t s) {
+  return (clz_u64((uint64_t)s | 1u) - (s >> 60 ? 3 : 4)) >> 1;  // s = 1 is 2^60: none
+}
+VMC_HD inline float root_first(int64_t t) { return near_rsqrt((float)(uint32_t)(t >> 29) * 4.656612873077393e-10f); }
+VMC_HD inline Root60 root_refined(int64_t t, int k, float y) {
+  const int32_t y0 = (int32_t)(y * 536870912.0f);  // 2^-29
   const Split60 ts = split60(t);
   const int64_t h = (wide(ts.h, y0) << 1) + (wide(ts.l, y0) >> 29);
   const Split60 hs = split60(h);
   const int64_t e = kOne60 - ((wide(hs.h, y0) << 1) + (wide(hs.l, y0) >> 29));
-  const int32_t e5 = (int32_t)(e >> 8);  // 2^-52
-  const int64_t u = (e >> 1) + ((3 * (wide(e5, e5) >> 44)) >> 3);
+  const int32_t e5 = (int32_t)(e >> 9);  // 2^-51
+  const int64_t u = (e >> 1) + ((3 * (wide(e5, e5) >> 42)) >> 3);
   Root60 q;
   q.r = h + mul60(hs, split60(u));
   q.y = ((int64_t)y0 << 31) + (wide(y0, (int32_t)(u >> 15)) >> 14) + (wide(y0, (int32_t)(u & 0x7fff)) >> 29);
   q.k = k;
   return q;
+}
+VMC_HD inline Root60 sqrt60(int64_t s) {
+  const int k = root_shift(s);
+  const int64_t t = s << (2 * k);
+  return root_refined(t, k, root_first(t));
 }
 
 // The Henyey-Greenstein cosine of the closed uniform's word u: with c = 2 xi - 1 and
