@@ -355,3 +355,32 @@ def test_blocks_of_few_warps_lose_no_photon(built, name, precision, n, block):
                         block_size=block)
     assert st["photons_done"] == n
     mesh.close()
+
+
+@pytest.mark.parametrize("mua", [1e-38, 2e-38, 1e-37])  # subnormal in FP32, and with depths that are
+@pytest.mark.parametrize("f", [0.0, 1e-27])
+def test_deposits_of_the_smallest_absorption(built, mua, f):
+    """Absorption next to none, in FP32's smallest numbers, gives the fluence of none: the walks are
+    the same, and a visit to an element loses its deposit only where that is below 1.18e-38."""
+    r, H, BH = mg.box_mesh_3d(3, 3, 3)
+    r = 20.0 * r
+    ne, nb = len(H), len(BH)
+    types = np.full(nb, ord("a"), np.uint8)
+    types[np.all(r[BH][:, :, 2] == r[:, 2].min(), axis=1)] = ord("c")
+    p = mg.Problem(dim=3, H=H, BH=BH, r=r, mua=np.zeros(ne), mus=np.full(ne, 2.0), g=np.zeros(ne), n=np.full(ne, 1.0),
+                   BCType=types, BCn=np.full(nb, 1.0), Nphoton=2000, seed=5)
+    none = V.run(p, normalize=False)
+    out = V.run(p.copy(mua=np.full(ne, mua), f=f), normalize=False)
+    assert out.stats["steps"] == none.stats["steps"]
+    path = none.ER.sum()  # of all photons, weight 1
+    if f == 0.0:
+        got, least = out.ER / mua, mua
+    else:  # MonteCarlo's normalisation, without volume and number
+        k = 2 * np.pi * f / 2.99792458e11
+        got, least = (out.EI * k + out.ER * mua) / (k * k + mua * mua), min(k, mua)
+    visits = none.stats["steps"] - none.stats["scatters"] + p.Nphoton
+    lost = 1.18e-38 / least * visits
+    assert lost < 0.75 * path
+    # FP32 sums of up to some hundred steps a visit: 1e-4
+    assert path * (1 - 1e-4) - lost < got.sum() < path * (1 + 1e-4)
+    assert np.all(got <= none.ER * (1 + 1e-4) + 1e-300)

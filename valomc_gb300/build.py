@@ -23,8 +23,8 @@ CU_UNITS = ["kern3d32.cu", "kern3d64.cu", "kern2d32.cu", "kern2d64.cu", "kern3d6
             "tools.cu", "server.cu", "noalloc.cu", "geometry.cu"]
 # The tetrahedral tracking kernel flushes FP32 subnormals: its reciprocals, roots, logarithms and
 # exponentials then need no scaling around them (5 % fewer instructions a step; 202.2 -> 197.2 ms
-# for 1e7 photons on the 648k-tet phantom).  A walk meets none: lengths are clamped at 0 and the
-# conversion to the FP64 accumulators has always dropped subnormal deposits.
+# for 1e7 photons on the 648k-tet phantom).  The deposits, which an absorption coefficient near
+# 1e-38 makes subnormal, are computed by operations that keep them (walk3d.cuh, keep_mul).
 FLAGS = {"kern3d32.cu": ["-ftz=true"]}
 CPP_UNITS = ["host_setup.cpp"]
 APPS = {"MC3D": "app/mc3d_main.cpp", "MC2D": "app/mc2d_main.cpp", "vmc_textdump": "app/textdump.cpp"}
