@@ -384,3 +384,17 @@ def test_deposits_of_the_smallest_absorption(built, mua, f):
     # FP32 sums of up to some hundred steps a visit: 1e-4
     assert path * (1 - 1e-4) - lost < got.sum() < path * (1 + 1e-4)
     assert np.all(got <= none.ER * (1 + 1e-4) + 1e-300)
+
+
+@pytest.mark.parametrize("precision", [V.VMC_FP32, V.VMC_FP64])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_photons_without_a_position_are_lost_at_once(built, precision, bad):
+    """Pencil beams, into the body from all sides, from points that are no numbers: no face is ever
+    found, as in the reference."""
+    p = cases()["jitter3d"][0].copy(Nphoton=500)
+    p = p.copy(BCType=np.full(p.Nb, ord("p"), np.uint8), BCLightDirectionType=np.full(p.Nb, ord("p"), np.uint8),
+               BCLNormal=np.full((p.Nb, 3), bad))
+    out = V.run(p, precision=precision, normalize=False, max_steps=2000)
+    assert out.stats["loss"] == p.Nphoton and out.stats["steps"] == 0 and out.stats["capped"] == 0
+    assert np.all(out.ER == 0) and np.all(out.EBR == 0)
+    assert out.stats["ledger"]["lost"] == p.Nphoton

@@ -1134,7 +1134,7 @@ struct Walk3D32 {
       for (int f = 0; f < 4; f++) {
         const float nd = pl[f].x * dx + pl[f].y * dy + pl[f].z * dz;
         const float num = pl[f].w - (pl[f].x * px + pl[f].y * py + pl[f].z * pz);
-        const bool better = f == 0 ? nd > 0.0f : nd > 0.0f && num * bnd < bnum * nd;
+        const bool better = nd > 0.0f && num * bnd < bnum * nd;  // false where num is no number
         bnum = better ? num : bnum;
         bnd = better ? nd : bnd;
         nf = better ? f : nf;
