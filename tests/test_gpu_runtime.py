@@ -398,3 +398,18 @@ def test_photons_without_a_position_are_lost_at_once(built, precision, bad):
     assert out.stats["loss"] == p.Nphoton and out.stats["steps"] == 0 and out.stats["capped"] == 0
     assert np.all(out.ER == 0) and np.all(out.EBR == 0)
     assert out.stats["ledger"]["lost"] == p.Nphoton
+
+
+@pytest.mark.parametrize("precision", [V.VMC_FP32, V.VMC_FP64])
+def test_trace_of_a_photon_that_finds_no_face(built, precision):
+    """A replayed photon without a direction is lost before it has walked an element: the trace
+    holds that event and no element, as the reference's."""
+    p = cases()["jitter3d"][0].copy(Nphoton=6)
+    p = p.copy(BCType=np.full(p.Nb, ord("l"), np.uint8), BCLightDirectionType=np.full(p.Nb, ord("a"), np.uint8),
+               BCLNormal=np.zeros((p.Nb, 3)))
+    tape = np.random.default_rng(3).integers(0, 2 ** 32, 6 * 50, dtype=np.uint64).astype(np.uint32)
+    off = np.arange(7, dtype=np.int64) * 50
+    out = V.run(p, precision=precision, tape=tape, tape_off=off, trace_photons=6, trace_stride=100)
+    assert out.stats["loss"] == 6 and out.stats["steps"] == 0
+    lost = -2 ** 63 + 2
+    assert [list(t) for t in out.traces] == [[lost]] * 6

@@ -1157,7 +1157,7 @@ struct Walk3D32 {
     }
     if (prop > dist && (unsigned)nextel < (unsigned)ne(J)) o2 = optics(J, nextel);
     px += dx * ds; py += dy * ds; pz += dz * ds;
-    tr.put(el);
+    if (found) tr.put(el);
     const float x = keep_mul(mua, ds);
     if (!FD) {
       const float dep = keep_mul(w, one_minus_exp_neg_keep(x));
