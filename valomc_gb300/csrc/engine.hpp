@@ -58,6 +58,8 @@ cudaError_t make_plane_records(int dim, void *geom, int64_t Ne, cudaStream_t st)
 // Memory of calls and launches: a pool of this library's per device, so that a call's buffers
 // are not mapped and unmapped each time.  It keeps at most kPoolKeep bytes between calls (what is
 // freed beyond that goes back at the next synchronisation), and all of it when an allocation fails.
+// It belongs to the device's current context (the device is selected): another one after
+// cudaDeviceReset.
 constexpr uint64_t kPoolKeep = 256ull << 20;
 int call_pool(int device, cudaMemPool_t *pool);
 // cudaMallocFromPoolAsync; gives the kept memory back and tries again when there is none

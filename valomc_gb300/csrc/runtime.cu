@@ -3,6 +3,7 @@
 // normalisation, resident meshes, batched launches, autotuning and the roofline
 // micro-benchmarks.  No CPU fallback: without an sm_103 device every call fails with
 // VMC_ERR_NO_DEVICE.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -88,12 +89,40 @@ static int dalloc(T **p, size_t count, int64_t &bytes) {
   return VMC_OK;
 }
 
+// The current context's id, unique for the life of the process (a context made after
+// cudaDeviceReset has another one, at the same address); 0 when the driver does not tell.
+static unsigned long long context_id() {
+  using GetId = CUresult (*)(CUcontext, unsigned long long *);
+  static const GetId get = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<GetId>(f);
+  }();
+  unsigned long long id = 0;
+  return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 int call_pool(int device, cudaMemPool_t *pool) {
+  struct Kept {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long context = 0;
+  };
   static std::mutex mu;
-  static cudaMemPool_t pools[128] = {nullptr};
+  static Kept kept[128];
   if (device < 0 || device >= 128) return VMC_ERR_INVALID_ARGUMENT;
+  const unsigned long long context = context_id();
+  if (!context) {  // nothing can be kept: the device's default pool
+    VMC_CK(cudaDeviceGetDefaultMemPool(pool, device));
+    return VMC_OK;
+  }
   std::lock_guard<std::mutex> lk(mu);
-  if (!pools[device]) {
+  Kept &k = kept[device];
+  if (k.context != context) {  // the first call, or the first after cudaDeviceReset, which took the old pool
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -103,9 +132,9 @@ int call_pool(int device, cudaMemPool_t *pool) {
     VMC_CK(cudaMemPoolCreate(&p, &props));
     uint64_t keep = kPoolKeep;
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    pools[device] = p;
+    k = Kept{p, context};
   }
-  *pool = pools[device];
+  *pool = k.pool;
   return VMC_OK;
 }
 
