@@ -6,6 +6,9 @@ import sys
 
 import pytest
 
+import valomc_gb300 as V
+from valomc_gb300 import meshgen as mg
+
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 AFTER_RESET = r"""
@@ -37,3 +40,16 @@ def test_calls_after_a_device_reset(built):
     env = dict(os.environ, PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tests"), os.path.join(ROOT, "oracle")]))
     r = subprocess.run([sys.executable, "-c", AFTER_RESET, runtimes[0]], capture_output=True, text=True, timeout=300, env=env)
     assert r.returncode == 0 and r.stdout.strip().endswith("done"), r.stdout + r.stderr
+
+
+def test_a_server_counts_the_memory_of_finished_calls_as_free(built):
+    """vmc_server_create limits its budget to the free memory: not less what calls before it have
+    left in their pool."""
+    torch = pytest.importorskip("torch")
+    p = mg.config_3d_phantom(nphoton=10, seed=1)
+    V.run(p)  # 648k tetrahedra: 52 MB of records and more
+    before = torch.cuda.mem_get_info()[0]
+    with_calls_memory = V.Server(memory_budget=1 << 30)
+    after = torch.cuda.mem_get_info()[0]
+    with_calls_memory.close()
+    assert after - before > 32 << 20

@@ -401,7 +401,10 @@ int vmc_server_create(const vmc_server_config *cfg, vmc_server **out) {
     // admission cannot promise more device memory than the device has free: the budget is
     // clamped to the free bytes at creation, less a margin for the launch tables and the
     // stream-ordered pool's own granularity
+    // (what the pool of finished calls keeps is free memory: it is given back first)
     size_t free_b = 0, total_b = 0;
+    cudaMemPool_t kept = nullptr;
+    if (call_pool(cfg->device, &kept) == VMC_OK) cudaMemPoolTrimTo(kept, 0);
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
       const int64_t margin = 256ll << 20;
       const int64_t usable = std::max<int64_t>(0, (int64_t)free_b - margin);
