@@ -4,6 +4,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 import valomc_gb300 as V
@@ -53,3 +54,38 @@ def test_a_server_counts_the_memory_of_finished_calls_as_free(built):
     after = torch.cuda.mem_get_info()[0]
     with_calls_memory.close()
     assert after - before > 32 << 20
+
+
+# 1.11 GB with planes, in a memory where that leaves less than half; 1.00 GB where it does not fit
+@pytest.mark.parametrize("layers,left", [(90, 2200 << 20), (81, 500 << 20)])
+def test_fp64_mesh_without_room_for_plane_records(built, layers, left):
+    """An FP64 mesh whose vertex records and job fit the device's memory runs, though its plane
+    records (three times as much again) would not fit or would leave no room: by the walk that
+    needs none of them."""
+    torch = pytest.importorskip("torch")
+    r, H, BH = mg.box_mesh_3d(80, 80, layers)
+    ne, nb = len(H), len(BH)
+    types = np.full(nb, ord("a"), np.uint8)
+    types[np.all(r[BH][:, :, 2] == 0, axis=1)] = ord("c")
+    p = mg.Problem(dim=3, H=H, BH=BH, r=r, mua=np.full(ne, 0.05), mus=np.full(ne, 1.0), g=np.full(ne, 0.8),
+                   n=np.full(ne, 1.4), BCType=types, BCn=np.full(nb, 1.0), Nphoton=300, seed=3)
+    mesh = V.Mesh(p, precision=V.VMC_FP64)
+    assert mesh.device_bytes >= 320 * ne
+    want, _ = V.run_batch([mesh], [p], precision=V.VMC_FP64, normalize=False)
+    mesh.close()
+    V.Server(memory_budget=1 << 30).close()  # gives back what the calls' pool keeps
+    free = torch.cuda.mem_get_info()[0]
+    held = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+    try:
+        mesh = V.Mesh(p, precision=V.VMC_FP64)
+        assert 112 * ne <= mesh.device_bytes < 200 * ne
+        got, st = V.run_batch([mesh, mesh], [p, p.copy(seed=4)], precision=V.VMC_FP64, normalize=False)
+        mesh.close()
+        assert st["photons_done"] == 2 * p.Nphoton
+        one = V.run(p, precision=V.VMC_FP64, normalize=False)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    for x in (got[0], one):
+        np.testing.assert_allclose(x.ER, want[0].ER, rtol=1e-8, atol=1e-9)
+        np.testing.assert_allclose(x.EBR, want[0].EBR, rtol=1e-8, atol=1e-9)

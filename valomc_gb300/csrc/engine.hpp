@@ -38,8 +38,20 @@ struct DeviceMesh {
   cudaMemPool_t pool = nullptr;
   cudaStream_t st = nullptr;
   ~DeviceMesh();
-  const void *geom(int precision) const { return d_geom[precision]; }
+  // FP64: the plane records are made (then d_geom holds them, and the vertex records behind them)
+  bool planes = true;
+  // what a walk reads: the plain FP64 one the plane records, the literal one the vertex records
+  const void *geom(int precision, bool literal) const;
+  // device bytes of an element's records
+  size_t record_bytes(int precision) const;
 };
+// Whether an FP64 mesh gets plane records beside the vertex records (320 bytes a tetrahedron, 112
+// without, 192 and 64 a triangle): only where such a mesh and the arrays of a job on it (48 bytes
+// an element) leave half of the device's free memory.  One that does not, or for which there is no
+// memory when it is made, is the size it was before there were planes, and its jobs take the
+// literal walk, which needs none.  Up to kPlanesAlways bytes the memory is not asked for.
+constexpr size_t kPlanesAlways = 1ull << 30;
+bool planes_fit(int dim, int64_t Ne);
 int upload_mesh(DeviceMesh &m, int precision_mask);
 // The same from the input's arrays with neighbours and records made on the device (m.device is
 // current, m.st and m.pool are set).  keep_HN: the host gets HN too.  Out of memory leaves nothing
@@ -52,7 +64,7 @@ int build_mesh_on_device(const vmc_input *in, int precision_mask, DeviceMesh &m,
 // Above 2^26 elements the scratch of 90 bytes an element could be what a mesh that fits by itself
 // lacks.
 inline bool builds_on_device(int64_t Ne) { return Ne >= 1000 && Ne <= (int64_t)1 << 26; }
-// TetRec / TriRec [Ne] at `geom` from the Tet64 / Tri64 [Ne] behind them
+// TetRec / TriRec [Ne] at `geom` from the Tet64 / Tri64 [Ne] behind them (planes)
 cudaError_t make_plane_records(int dim, void *geom, int64_t Ne, cudaStream_t st);
 
 // Memory of calls and launches: a pool of this library's per device, so that a call's buffers
@@ -95,13 +107,15 @@ struct JobBuffers {
 // bytes of device state a job on mesh m needs (admission control)
 int64_t job_footprint(const HostJob &j, const HostMesh &m);
 int upload_job(const HostJob &j, const DeviceMesh &m, int precision, JobBuffers &b, cudaStream_t st);
-JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, const JobBuffers &b);
+JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, bool literal, const JobBuffers &b);
+// Whether a job runs the literal FP64 walk (rough_optics, or a mesh without plane records).
+bool runs_literal(const vmc_input *in, const DeviceMesh &m, int precision);
 int zero_job(JobBuffers &b, cudaStream_t st);
 
 struct LaunchSpec {
   int dim = 3, precision = VMC_FP32;
   bool fd = false, tape = false;
-  bool literal = false; // FP64: the reference's operation sequence (rough_optics)
+  bool literal = false; // FP64: the reference's operation sequence (runs_literal)
   bool graph = false;  // launch through a (reused) CUDA graph
   int stage_slots = 0; // shared-memory staging slots per CTA (0: off)
   int block = 0, blocks_per_sm = 0, chunk = 0;

@@ -353,17 +353,15 @@ int build(const vmc_input *in, int mask, DeviceMesh &m, bool keep_HN, Temp &t) {
   // the records
   for (int prec = 0; prec < 2; prec++) {
     if (!(mask & (1 << prec))) continue;
-    const size_t size = prec == VMC_FP64 ? (D == 3 ? sizeof(TetRec) + sizeof(Tet64) : sizeof(TriRec) + sizeof(Tri64))
-                                         : (D == 3 ? sizeof(Tet32) : sizeof(Tri32));
+    const size_t size = m.record_bytes(prec);
     void *p = nullptr;
     if (m.pool) VMC_CK(pool_alloc(&p, size * (size_t)Ne, m.pool, m.st));
     else VMC_CK(cudaMalloc(&p, size * (size_t)Ne));
     m.d_geom[prec] = p;
     m.bytes += (int64_t)(size * (size_t)Ne);
     if (prec == VMC_FP64) {
-      unsigned char *vert = static_cast<unsigned char *>(p) + (D == 3 ? sizeof(TetRec) : sizeof(TriRec)) * (size_t)Ne;
-      vertex_records<<<blocks(Ne), 256, 0, st>>>(g, D, vert);
-      VMC_CK(make_plane_records(D, p, Ne, st));
+      vertex_records<<<blocks(Ne), 256, 0, st>>>(g, D, const_cast<void *>(m.geom(VMC_FP64, true)));
+      if (m.planes) VMC_CK(make_plane_records(D, p, Ne, st));
     } else if (D == 3) {
       tet32_records<<<blocks(Ne * 4), 256, 0, st>>>(g, static_cast<Tet32 *>(p));
     } else {
@@ -413,6 +411,7 @@ int build_mesh_on_device(const vmc_input *in, int precision_mask, DeviceMesh &m,
   m.dim = in->dim;
   cudaMemPool_t pool = nullptr;
   if ((s = call_pool(m.device, &pool))) return s;
+  m.planes = planes_fit(m.dim, m.host.Ne);
   Temp t{pool, m.st, {}};
   const int64_t before = m.bytes;
   s = build(in, precision_mask, m, keep_HN, t);

@@ -190,7 +190,8 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   JobDev d;
   memset(&d, 0, sizeof(d));
   double *acc = dev->acc;
-  d.geom = m->geom(o.precision);
+  const bool literal = runs_literal(&in, *m, o.precision);
+  d.geom = m->geom(o.precision, literal);
   d.optics = dev->optics;
   d.opt_mask = hj.homogeneous ? 0 : -1;
   d.Ns = (int32_t)ns;
@@ -235,7 +236,7 @@ extern "C" int vmc_run_noalloc(vmc_mesh *mesh, const vmc_input *job, const vmc_o
   spec.dim = m->host.dim;
   spec.precision = o.precision;
   spec.fd = hj.omega > 0.0;
-  spec.literal = o.precision == VMC_FP64 && rough_optics(&in, m->host);
+  spec.literal = literal;
   spec.tape = false;
   const void *fn = select_kernel(spec);
   int sms = 0;

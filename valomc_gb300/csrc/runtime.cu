@@ -186,20 +186,53 @@ DeviceMesh::~DeviceMesh() {
     }
 }
 
+size_t DeviceMesh::record_bytes(int precision) const {
+  if (precision != VMC_FP64) return dim == 3 ? sizeof(Tet32) : sizeof(Tri32);
+  const size_t vert = dim == 3 ? sizeof(Tet64) : sizeof(Tri64);
+  return planes ? vert + (dim == 3 ? sizeof(TetRec) : sizeof(TriRec)) : vert;
+}
+
+const void *DeviceMesh::geom(int precision, bool literal) const {
+  const unsigned char *d = static_cast<const unsigned char *>(d_geom[precision]);
+  if (precision != VMC_FP64 || !literal || !planes || !d) return d;
+  return d + (size_t)host.Ne * (dim == 3 ? sizeof(TetRec) : sizeof(TriRec));
+}
+
+bool planes_fit(int dim, int64_t Ne) {
+  const size_t full = (size_t)Ne * (dim == 3 ? sizeof(TetRec) + sizeof(Tet64) : sizeof(TriRec) + sizeof(Tri64));
+  if (full <= kPlanesAlways) return true;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return 2 * (full + 48 * (size_t)Ne) <= free_b;
+}
+
+bool runs_literal(const vmc_input *in, const DeviceMesh &m, int precision) {
+  return precision == VMC_FP64 && (!m.planes || rough_optics(in, m.host));
+}
+
 int upload_mesh(DeviceMesh &m, int precision_mask) {
   HostMesh &h = m.host;
   m.dim = h.dim;
   cudaStream_t st = m.st;
   if ((precision_mask & 1) && !m.d_geom[VMC_FP64]) {
     // the face-plane records, made on the device from the vertex records uploaded behind them
-    const size_t ne = (size_t)h.Ne, rec = h.dim == 3 ? sizeof(TetRec) : sizeof(TriRec);
-    const size_t vert = h.dim == 3 ? sizeof(Tet64) : sizeof(Tri64);
+    const size_t ne = (size_t)h.Ne, vert = h.dim == 3 ? sizeof(Tet64) : sizeof(Tri64);
     const void *src = h.dim == 3 ? static_cast<const void *>(h.tet64.data()) : h.tri64.data();
-    unsigned char *d;
-    VMC_TRY(dalloc(&d, ne * (rec + vert), m.bytes, m.pool, st));
+    unsigned char *d = nullptr;
+    m.planes = planes_fit(h.dim, h.Ne);
+    int s = dalloc(&d, ne * m.record_bytes(VMC_FP64), m.bytes, m.pool, st);
+    if (s == VMC_ERR_OUT_OF_MEMORY && m.planes) {
+      m.planes = false;
+      s = dalloc(&d, ne * m.record_bytes(VMC_FP64), m.bytes, m.pool, st);
+    }
+    if (s) return s;
     m.d_geom[VMC_FP64] = d;
-    VMC_TRY(h2d(d + ne * rec, static_cast<const unsigned char *>(src), ne * vert, st));
-    VMC_CK(make_plane_records(h.dim, d, (int64_t)ne, st));
+    const size_t behind = ne * (m.record_bytes(VMC_FP64) - vert);
+    VMC_TRY(h2d(d + behind, static_cast<const unsigned char *>(src), ne * vert, st));
+    if (m.planes) VMC_CK(make_plane_records(h.dim, d, (int64_t)ne, st));
   }
   if ((precision_mask & 2) && !m.d_geom[VMC_FP32]) {
     if (h.dim == 3) {
@@ -296,11 +329,11 @@ int zero_job(JobBuffers &b, cudaStream_t st) {
   return VMC_OK;
 }
 
-JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, const JobBuffers &b) {
+JobDev describe_job(const HostJob &j, const DeviceMesh &m, int precision, bool literal, const JobBuffers &b) {
   JobDev d;
   memset(&d, 0, sizeof(d));
   const int64_t Ne = m.host.Ne, Nb = m.host.Nb;
-  d.geom = m.geom(precision);
+  d.geom = m.geom(precision, literal);
   d.optics = b.d_optics;
   d.opt_mask = j.homogeneous ? 0 : -1;
   d.Ns = (int32_t)j.src.size();
@@ -965,7 +998,8 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   jb.free_stream = stream;
   s = upload_job(hj, dm, o.precision, jb, stream);
   if (s) return s;
-  JobDev d = describe_job(hj, dm, o.precision, jb);
+  const bool literal = runs_literal(in, dm, o.precision);
+  JobDev d = describe_job(hj, dm, o.precision, literal, jb);
   d.pcount = nph;
   d.poffset = o.photon_offset;
   d.stream = o.stream_id;
@@ -994,7 +1028,7 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   spec.dim = in->dim;
   spec.precision = o.precision;
   spec.fd = hj.omega > 0.0;
-  spec.literal = o.precision == VMC_FP64 && rough_optics(in, dm.host);
+  spec.literal = literal;
   spec.tape = o.rng == VMC_RNG_TAPE;
   spec.block = o.block_size;
   spec.blocks_per_sm = o.blocks_per_sm;
@@ -1128,7 +1162,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
     sp.dim = meshes[i]->m.host.dim;
     sp.precision = o.precision;
     sp.fd = hj[(size_t)i].omega > 0.0;
-    sp.literal = o.precision == VMC_FP64 && rough_optics(&jobs[i], meshes[i]->m.host);
+    sp.literal = runs_literal(&jobs[i], meshes[i]->m, o.precision);
     sp.block = o.block_size;
     sp.blocks_per_sm = o.blocks_per_sm;
     sp.chunk = o.fetch_chunk;
@@ -1153,7 +1187,7 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
       jb[(size_t)i]->free_stream = stream;
       s = upload_job(hj[(size_t)i], meshes[i]->m, o.precision, *jb[(size_t)i], stream);
       if (s) return s;
-      JobDev d = describe_job(hj[(size_t)i], meshes[i]->m, o.precision, *jb[(size_t)i]);
+      JobDev d = describe_job(hj[(size_t)i], meshes[i]->m, o.precision, g.spec.literal, *jb[(size_t)i]);
       d.pcount = std::max<int64_t>(0, jobs[i].Nphoton);  // a negative count runs none
       d.poffset = o.photon_offset;
       d.stream = o.stream_id;

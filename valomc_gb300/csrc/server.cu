@@ -256,7 +256,7 @@ void vmc_server::loop() {
       std::vector<int64_t> quota;
       for (Request *r : c.rs) {
         DeviceMesh *m = mesh_impl(meshes[(size_t)r->mesh_id]);
-        JobDev d = describe_job(r->job, *m, cfg.precision, *r->buf);
+        JobDev d = describe_job(r->job, *m, cfg.precision, c.literal, *r->buf);
         int64_t qn = r->slice;
         d.pcount = qn;
         d.poffset = r->issued;
@@ -464,7 +464,7 @@ int vmc_server_submit(vmc_server *s, int32_t mesh_id, const vmc_input *job, int6
   if (st) return st;
   r->job.keep();  // the caller's arrays may go before the request is admitted
   r->job.seed = in.seed_given ? in.seed : clock_seed();
-  r->literal = s->cfg.precision == VMC_FP64 && rough_optics(&in, m->host);
+  r->literal = runs_literal(&in, *m, s->cfg.precision);
   r->mesh_id = mesh_id;
   r->nphoton = in.Nphoton;
   r->footprint = job_footprint(r->job, m->host);

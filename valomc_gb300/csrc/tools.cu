@@ -161,9 +161,13 @@ int vmc_autotune(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs, 
     jb[(size_t)i].reset(new JobBuffers);
     s = upload_job(hj[(size_t)i], *m, prec, *jb[(size_t)i], 0);
     if (s) return s;
-    descs.push_back(describe_job(hj[(size_t)i], *m, prec, *jb[(size_t)i]));
     total += jobs[i].Nphoton;
   }
+  // the trials are one launch each: of the first job's walk, or of the one that needs no planes
+  bool literal = runs_literal(&jobs[0], *mesh_impl(meshes[0]), prec);
+  for (int i = 0; i < njobs; i++) literal = literal || (prec == VMC_FP64 && !mesh_impl(meshes[i])->planes);
+  for (int i = 0; i < njobs; i++)
+    descs.push_back(describe_job(hj[(size_t)i], *mesh_impl(meshes[i]), prec, literal, *jb[(size_t)i]));
   if (total <= 0) return VMC_ERR_INVALID_ARGUMENT;
   // a first short run calibrates the photon rate so each trial lasts about budget / trials
   const int blocks[] = {128, 256, 64};
@@ -172,7 +176,7 @@ int vmc_autotune(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs, 
   const int nshape = 3 * 3 * 2 + 4;
   LaunchSpec base;
   base.dim = dim; base.precision = prec; base.fd = fd; base.max_steps = opt->max_steps;
-  base.literal = prec == VMC_FP64 && rough_optics(&jobs[0], mesh_impl(meshes[0])->host);
+  base.literal = literal;
   auto run = [&](const LaunchSpec &sp, double frac, double &rate) -> int {
     std::vector<JobDev> d = descs;
     int64_t n = 0;

@@ -132,7 +132,7 @@ constexpr int64_t kDenseStageBytes = 32 * 1024;
 constexpr int kSmemJobs = 16;
 
 struct JobDev {
-  const void *geom;            // Tet64 / Tet32 / Tri64 / Tri32 [Ne]
+  const void *geom;            // [Ne] TetRec, then Tet64 (literal walk: Tet64 alone) / Tet32; the same of triangles
   const void *optics;          // double4 or float4 rows
   int32_t opt_mask;            // -1: per element, 0: one homogeneous row
   int32_t Ns;                  // emitting faces

@@ -660,9 +660,7 @@ struct Walk3D64L {
     else f(pos[0], pos[1], pos[2], dir[0], dir[1], dir[2], w, prop, mua, mus, g, nidx, acc, el, curface, nsteps);
   }
 
-  __device__ __forceinline__ static const Tet64 *tets(const JobDev &J) {
-    return reinterpret_cast<const Tet64 *>(reinterpret_cast<const TetRec *>(J.geom) + J.Ne);
-  }
+  __device__ __forceinline__ static const Tet64 *tets(const JobDev &J) { return reinterpret_cast<const Tet64 *>(J.geom); }
   __device__ __forceinline__ void optics(const JobDev &J, int e, double &a, double &s, double &gg, double &nn) const {
     const double2 *o = reinterpret_cast<const double2 *>(J.optics) + 2 * (int64_t)(e & J.opt_mask);
     const double2 o0 = __ldg(o), o1 = __ldg(o + 1);
