@@ -1078,6 +1078,8 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
 int vmc_mesh_create(const vmc_input *geometry, int32_t precision, int32_t device, vmc_mesh **out) {
   if (!geometry || !out || (precision != VMC_FP64 && precision != VMC_FP32)) return VMC_ERR_INVALID_ARGUMENT;
   *out = nullptr;
+  if (geometry->dim != 2 && geometry->dim != 3) return VMC_ERR_INVALID_ARGUMENT;
+  if (geometry->Ne < 0 || geometry->Nb < 0 || geometry->Nr < 0) return VMC_ERR_INVALID_ARGUMENT;
   if ((geometry->Ne && !geometry->H) || (geometry->Nb && !geometry->BH) || (geometry->Nr && !geometry->r))
     return VMC_ERR_INVALID_ARGUMENT;
   const int64_t nh = geometry->Ne * (geometry->dim + 1), nb = geometry->Nb * geometry->dim;
