@@ -438,6 +438,32 @@ void HostJob::keep() {
   mua = own.data(); mus = mua + c; g = mua + 2 * c; n = mua + 3 * c;
 }
 
+ResultSpans::ResultSpans(const vmc_output *outs, const HostMesh *const *meshes, int n) {
+  spans_.reserve(7 * (size_t)n);
+  for (int i = 0; i < n; i++) {
+    const vmc_output &o = outs[i];
+    const HostMesh &m = *meshes[i];
+    auto add = [&](const void *p, int64_t count) {
+      const uintptr_t b = reinterpret_cast<uintptr_t>(p);
+      if (p && count > 0) spans_.push_back(Span{b, b + 8 * (uintptr_t)count});
+    };
+    add(o.ER, m.Ne); add(o.EI, m.Ne);
+    add(o.EBR, m.Nb); add(o.EBI, m.Nb); add(o.DEBR, m.Nb); add(o.DEBI, m.Nb);
+    add(o.HN, m.Ne * (m.dim + 1));
+  }
+  std::sort(spans_.begin(), spans_.end(), [](const Span &a, const Span &b) { return a.begin < b.begin; });
+  for (size_t i = 1; i < spans_.size(); i++) spans_[i].end = std::max(spans_[i].end, spans_[i - 1].end);
+}
+
+bool ResultSpans::meets(const HostJob &j) const {
+  for (const double *x : {j.mua, j.mus, j.g, j.n}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(x), e = b + 8 * (uintptr_t)j.rows();
+    auto it = std::lower_bound(spans_.begin(), spans_.end(), e, [](const Span &s, uintptr_t at) { return s.begin < at; });
+    if (it != spans_.begin() && (it - 1)->end > b) return true;  // the largest end of those that begin before e
+  }
+  return false;
+}
+
 template <class T>
 static void rows_of(const HostJob &j, T *out) {
   const int64_t c = (int64_t)j.rows();

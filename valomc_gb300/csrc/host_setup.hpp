@@ -95,6 +95,19 @@ struct HostJob {
   float walk = 0;               // about how long its walks are: scatterings per absorption length
 };
 
+// Memory that a call writes its results to.  A job reads its optics from the caller's arrays until
+// the results are normalised: where a caller has results written over those arrays, the job keeps
+// its own copy (HostJob::keep).
+class ResultSpans {
+ public:
+  ResultSpans(const vmc_output *outs, const HostMesh *const *meshes, int n);
+  bool meets(const HostJob &j) const;  // an array of j's optics overlaps one of the results
+
+ private:
+  struct Span { uintptr_t begin, end; };
+  std::vector<Span> spans_;  // by their begin, each end the largest so far
+};
+
 // Whether the scattering coefficient or the index changes across more than an eighth of the mesh's
 // interior faces: such jobs run the literal FP64 walk.  A photon's remaining path is multiplied
 // by mus / mus2 at each of these faces, so rounding differences are too: on the 648k-tet phantom

@@ -976,6 +976,8 @@ int vmc_run(const vmc_input *in, const vmc_options *opt_in, vmc_output *out, vmc
   HostJob hj;
   s = build_job(in, dm.host, hj);
   if (s) return s;
+  const HostMesh *const one = &dm.host;
+  if (ResultSpans(out, &one, 1).meets(hj)) hj.keep();
   hj.seed = in->seed_given ? in->seed : clock_seed();
   // photons simulated: a negative count runs none, as MonteCarlo's loop does, and is still
   // the divisor of the normalisation (the reference's -0.0 results)
@@ -1149,6 +1151,13 @@ int vmc_run_batch(vmc_mesh *const *meshes, const vmc_input *jobs, int32_t njobs,
     s = build_job(&in, mm->m.host, hj[(size_t)i]);
     if (s) return s;
     hj[(size_t)i].seed = in.seed_given ? in.seed : clock_seed() + (uint64_t)i;
+  }
+  {
+    std::vector<const HostMesh *> hosts;
+    for (int i = 0; i < njobs; i++) hosts.push_back(&meshes[i]->m.host);
+    const ResultSpans results(outs, hosts.data(), njobs);
+    for (HostJob &j : hj)
+      if (results.meets(j)) j.keep();
   }
   s = select_device(o.device);
   if (s) return s;
