@@ -494,7 +494,7 @@ int build_job(const vmc_input *in, const HostMesh &m, HostJob &j) {
   j.phase0 = ph0;
   {  // the same in turns, for the plain form's fixed-point phase
     const long double two_pi = 6.283185307179586476925286766559005768L;
-    j.k_turn = (double)((long double)j.k_scale / two_pi);
+    j.k_turn = in->f / kC0;  // one rounding: every step's phase has it
     long double t = (long double)ph0 / two_pi;
     t -= floorl(t);
     j.turn0 = t >= 0 && t < 1 ? (uint64_t)ldexpl(t, 64) : 0;

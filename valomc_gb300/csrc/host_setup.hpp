@@ -88,7 +88,7 @@ struct HostJob {
   std::vector<SourceRecF> src_f;  // FP32 copies for the tracking form
   std::vector<float> cdf_f;
   double f = 0, omega = 0, k_scale = 0, phase0 = 0;
-  double k_turn = 0;            // k_scale / (2 pi)
+  double k_turn = 0;            // f / c0, turns a millimetre in vacuum
   uint64_t turn0 = 0;           // phase0 in 2^-64 turns
   int64_t Nphoton = 0;
   uint64_t seed = 0;

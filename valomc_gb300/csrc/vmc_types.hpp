@@ -154,7 +154,7 @@ struct JobDev {
   double phase0;
   float phase_f;               // the same modulo 2 pi in FP32, for the tracking form
   float walk;                  // HostJob::walk
-  double k_turn;               // k_scale / (2 pi), and phase0 in 2^-64 turns: the plain form's phase
+  double k_turn;               // f / c0, and phase0 in 2^-64 turns: the plain form's phase
   uint64_t turn0;
   uint64_t seed;
   uint32_t stream;
