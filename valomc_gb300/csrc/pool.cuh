@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
           }
           if (all == 0 && !pending) break;
           const int want = pack_warps(all, warps);
-          if constexpr (!R::kReplay) {
+          if constexpr (W::kPack && !R::kReplay) {
             if (!pending && (used < want || 4 * want <= 3 * used)) {
               const int k = before + __popc(live & lt_mask);
               const int to = alive ? pack_thread(k, all, want, warp_turn(lp, warps), warps) : -1;
@@ -255,7 +255,6 @@ __global__ void __launch_bounds__(256, W::kMinBlocks) pool_kernel(const __grid_c
       }
     }
     if (!W::kPack && chunk_left < 0 && !__any_sync(kFull, alive)) break;
-    const bool was = alive;
     // Events (W::kDefer): what a step ends in besides a scatter and a common crossing, the
     // boundary, an interface, roulette, takes as many instructions as several steps, and with a few
     // of 32 lanes at it a warp paid for it in nearly every step.  Lanes with an event wait until

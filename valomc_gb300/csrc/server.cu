@@ -93,7 +93,7 @@ struct vmc_server {
 
 namespace {
 // One of the two launch pipelines of the serving loop: a stream, an arena per launch class
-// (dimension x CW/FD) and the requests whose slices ride in its current epoch.
+// (dimension x CW/FD x FP64 walk) and the requests whose slices ride in its current epoch.
 struct Lane {
   cudaStream_t st = nullptr;
   std::vector<std::unique_ptr<LaunchArena>> arenas;

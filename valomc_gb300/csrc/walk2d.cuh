@@ -198,7 +198,7 @@ struct Walk2D64 {
   }
 
   // the exit edge and the distance to it, as in the tetrahedral walk
-  __device__ __forceinline__ int exit_face(const JobDev &J, R &rng, double &dist, int4 &nbr) const {
+  __device__ __forceinline__ int exit_face(const JobDev &J, double &dist, int4 &nbr) const {
     const TriRec *T = recs(J) + el;
     const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
     const double offd = __ldg(&T->off);
@@ -241,7 +241,7 @@ struct Walk2D64 {
     if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     double dist;
     int4 nb;
-    const int nf = exit_face(J, rng, dist, nb);
+    const int nf = exit_face(J, dist, nb);
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
@@ -546,11 +546,10 @@ struct Walk2D64L {
   }
 
   __device__ int step(const JobDev &J, R &rng, int64_t max_steps) {
-    if (rng.exhausted()) { job_count(J, kJcTapeEnd); die(J, kEvTapeEnd); return kDiedEarly; }
+    if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     if (nsteps >= max_steps) {
       job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
-      die(J, kEvCapped);
-      return kDiedEarly;
+      return die(J, kEvCapped);
     }
     const Tri64 *T = tris(J) + el;
     double V[3][2];
@@ -570,8 +569,7 @@ struct Walk2D64L {
     else if (curface != 2 && ray_seg(pos, dir, V[2], V[0], dist) && dist > 0.0) nf = 2;
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
-      die(J, kEvLost);
-      return kDiedEarly;
+      return die(J, kEvLost);
     }
     const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nb.z;
     nsteps++;
@@ -674,7 +672,6 @@ struct Walk2D64L {
 
 template <bool FD, class R>
 struct Walk2D32 {
-  static constexpr bool kBuffered = true;  // words left in a block are carried from step to step
   static constexpr bool kPack = false;  // its walks are short: packing gains nothing and costs the loop 2 %
   static constexpr bool kCap32 = false;
   static constexpr bool kDefer = true;
@@ -689,15 +686,9 @@ struct Walk2D32 {
   float acc, accI;
   int el;
   int32_t nsteps;
-  int pend;  // event to come: 1 + the edge crossed, 4 for the end of the free path, 0 none
+  int pend;  // event to come: 1 + the edge crossed, 0 none
   bool outward;  // launched out through its own entry edge
   Tr tr;
-
-  // moves the photon's state between lanes (Packer)
-  template <class F> __device__ __forceinline__ void move(const F &f) {
-    if constexpr (FD) f(px, py, dx, dy, w, prop, mua, mus, g, nidx, acc, phase, accI, el, nsteps);
-    else f(px, py, dx, dy, w, prop, mua, mus, g, nidx, acc, el, nsteps);
-  }
 
   __device__ __forceinline__ float4 optics(const JobDev &J, int e) const {
     return __ldg(reinterpret_cast<const float4 *>(J.optics) + (e & J.opt_mask));
@@ -803,16 +794,14 @@ struct Walk2D32 {
   }
 
   __device__ int step(const JobDev &J, R &rng, int64_t max_steps) {
-    if (rng.exhausted()) { job_count(J, kJcTapeEnd); die(J, kEvTapeEnd); return kDiedEarly; }
+    if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     if (nsteps >= max_steps) {
       job_count(J, kJcCapped); job_ledger(J, kLgLost, f2d_int(w));
-      die(J, kEvCapped);
-      return kDiedEarly;
+      return die(J, kEvCapped);
     }
     if (R::kReplay && outward) {  // with Philox streams this is settled at launch
       job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
-      die(J, kEvLost);
-      return kDiedEarly;
+      return die(J, kEvLost);
     }
     const Tri32 *T = reinterpret_cast<const Tri32 *>(J.geom) + el;
     const float4 *L4 = reinterpret_cast<const float4 *>(T->ln);
@@ -836,8 +825,7 @@ struct Walk2D32 {
     const float best = __fdividef(bnum, bnd);
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, f2d_int(w));
-      die(J, kEvLost);
-      return kDiedEarly;
+      return die(J, kEvLost);
     }
     nsteps++;
     const float dist = fmaxf(best, 0.0f);

@@ -18,7 +18,7 @@
 
 namespace vmc {
 
-enum StepResult { kAlive = 0, kScattered = 1, kAliveMax = kScattered, kDied = 2, kDiedEarly = 3 };
+enum StepResult { kAlive = 0, kScattered = 1, kAliveMax = kScattered, kDied = 2 };
 
 // Moller-Trumbore (RayTriangleIntersects, cpp/3d/MC3D.hpp:1825-1869)
 __device__ __forceinline__ bool ray_tri(const double O[3], const double D[3], const double *V0, const double *V1,
@@ -422,7 +422,7 @@ struct Walk3D64 {
   // 4e-6 |r|_1 |d|_1, and the ray starts clearly inside every other plane but the one it
   // entered by (which the reference does not test): then Moller-Trumbore finds u and v well
   // inside that face, and well outside the others or behind the photon.
-  __device__ __forceinline__ int exit_face(const JobDev &J, R &rng, double &dist, int4 &nbr) const {
+  __device__ __forceinline__ int exit_face(const JobDev &J, double &dist, int4 &nbr) const {
     const TetRec *T = recs(J) + el;
     const double2 a0 = __ldg(reinterpret_cast<const double2 *>(T->v0));
     const double2 a1 = __ldg(reinterpret_cast<const double2 *>(T->v0) + 1);
@@ -466,7 +466,7 @@ struct Walk3D64 {
     if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     double dist;
     int4 nb;
-    const int nf = exit_face(J, rng, dist, nb);
+    const int nf = exit_face(J, dist, nb);
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
       return die(J, kEvLost);
@@ -752,11 +752,10 @@ struct Walk3D64L {
   }
 
   __device__ int step(const JobDev &J, R &rng, int64_t max_steps) {
-    if (rng.exhausted()) { job_count(J, kJcTapeEnd); die(J, kEvTapeEnd); return kDiedEarly; }
+    if (rng.exhausted()) { job_count(J, kJcTapeEnd); return die(J, kEvTapeEnd); }
     if (nsteps >= max_steps) {
       job_count(J, kJcCapped); job_ledger(J, kLgLost, w);
-      die(J, kEvCapped);
-      return kDiedEarly;
+      return die(J, kEvCapped);
     }
     const Tet64 *T = tets(J) + el;
     double V[4][3];
@@ -779,8 +778,7 @@ struct Walk3D64L {
     else if (curface != 3 && ray_tri(pos, dir, V[1], V[2], V[3], dist) && dist > 0.0) nf = 3;
     if (nf < 0) {
       job_count(J, kJcLoss); job_ledger(J, kLgLost, w);
-      die(J, kEvLost);
-      return kDiedEarly;
+      return die(J, kEvLost);
     }
     const int nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nf == 2 ? nb.z : nb.w;
     nsteps++;
