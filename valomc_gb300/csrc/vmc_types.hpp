@@ -127,8 +127,9 @@ constexpr int kDefaultRefill = 4;
 constexpr int64_t kDenseStageBytes = 32 * 1024;
 // Largest job table a multi-job launch copies into each CTA's shared memory.  The walk keeps a
 // job's hot fields in registers, and what the tables of four CTAs take the L1 loses: two jobs on
-// the phantom 36.9 ms with the table and 37.4 without, ten cubes 41.25 and 41.26, 64 cubes of up to
-// 3 million tetrahedra (table 17 KB, L1 128 KB of an SM's 228) 310 and 303.
+// the phantom 36.9 ms with the table and 37.4 without, two cubes 8.9 and 8.9, ten 41.65 and 41.4, 16
+// 81.7 and 81.1; above the line 17 cubes 78.6 and 78.1, 32 142.4 and 141.4, 64 497 and 487, 64 of up
+// to 3 million tetrahedra (table 17 KB, L1 128 KB of an SM's 228) 310 and 303.
 constexpr int kSmemJobs = 16;
 
 struct JobDev {

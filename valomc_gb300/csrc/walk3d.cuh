@@ -209,8 +209,8 @@ __device__ __forceinline__ float free_path_f(float u, float mus) {
 //              direction on the integer pipe (fixed64.hpp); the last two by 48 FP64 operations of
 //              3D before (23 in 2D), with errors 3 to 100 times as large.
 //   quotients and roots from FP32 first values.
-// 1e5 photons on the phantom 313 -> 102 -> 79 ms (571 before lanes were packed as well), 1e3 there
-// 46.8 -> 39.4, 20 000 in the 48k-tet cube 33.7 -> 27.4 (the middle figures with the scatter in
+// 1e5 photons on the phantom 313 -> 102 -> 72 ms (571 before lanes were packed as well), 1e3 there
+// 46.8 -> 31.7, 20 000 in the 48k-tet cube 33.7 -> 25.9 (102, 46.8 and 33.7 with the scatter in
 // FP64).  The phantom's run ends in walks of 14 000 steps, with the issue slots 20 % and the FP64
 // pipe 19 % busy: the latency of some 1000 instructions a step.  Against 80-bit arithmetic the
 // elements' median error in the cube is 5e-14; with the library's functions it was 2.6e-13.
@@ -1112,8 +1112,8 @@ struct Walk3D32 {
     const float4 p0 = __ldg(P4 + 0), p1 = __ldg(P4 + 1), p2 = __ldg(P4 + 2), p3 = __ldg(P4 + 3);
     // The neighbours: a launch of one job loads the one it crosses to when it crosses, a quarter of
     // the steps.  The gathers keep the L1 73 % busy, each 16-byte load of a warp taking 16 cycles
-    // of it: 1e7 photons on the phantom 197.5 -> 189.5 ms, frequency domain at 1e6 33.9 -> 32.7,
-    // the 48k-tet cube 6.74 -> 6.54.  Launches of several jobs, whose records come from the L2 more
+    // of it: 1e7 photons on the phantom 197.3 -> 187.3 ms, frequency domain at 1e6 33.9 -> 32.0,
+    // the 48k-tet cube 6.74 -> 6.51.  Launches of several jobs, whose records come from the L2 more
     // often, load all four with the planes (ten cubes 41.5 ms, 42.3 the other way).
     int4 nb = make_int4(0, 0, 0, 0);
     if constexpr (!R::kOneJob) nb = __ldg(reinterpret_cast<const int4 *>(T->nbr));
