@@ -413,3 +413,22 @@ def test_trace_of_a_photon_that_finds_no_face(built, precision):
     assert out.stats["loss"] == 6 and out.stats["steps"] == 0
     lost = -2 ** 63 + 2
     assert [list(t) for t in out.traces] == [[lost]] * 6
+
+
+@pytest.mark.parametrize("mus", [2e-38, 5e-38, 1e-37, 1e-20])
+def test_path_left_on_entering_a_scattering_element(built, mus):
+    """A layer that scatters next to nothing before one that does: the path left there is the path of
+    a vacuum, whose draw is independent, so that sums over layers agree within their noise."""
+    r, H, BH = mg.box_mesh_3d(4, 4, 6)
+    ne, nb, n = len(H), len(BH), 1000000
+    z = r[H].mean(axis=1)[:, 2]
+    types = np.full(nb, ord("a"), np.uint8)
+    types[np.all(r[BH][:, :, 2] == 0, axis=1)] = ord("l")
+    base = mg.Problem(dim=3, H=H, BH=BH, r=r, mua=np.full(ne, 0.2), mus=np.where(z < 2, mus, 2.0), g=np.zeros(ne),
+                      n=np.full(ne, 1.0), BCType=types, BCn=np.full(nb, 1.0), Nphoton=n, seed=5)
+    tiny = V.run(base, normalize=False)
+    none = V.run(base.copy(mus=np.where(z < 2, 0.0, 2.0), seed=6), normalize=False)
+    for k in range(6):
+        a, b = (x.ER[(z >= k) & (z < k + 1)].sum() for x in (tiny, none))
+        assert abs(a - b) < 6 * np.sqrt(2 * n / 4)  # a photon leaves between 0 and 1 there
+    assert abs(tiny.stats["scatters"] / none.stats["scatters"] - 1) < 0.02

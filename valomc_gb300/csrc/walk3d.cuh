@@ -171,6 +171,12 @@ __device__ __forceinline__ float keep_fma(float a, float b, float c) {
   asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
+// (a path left of 1e37 mm in an element that hardly scatters, times 1e-38 on entering one that does)
+__device__ __forceinline__ float keep_div(float a, float b) {
+  float r;
+  asm("div.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 __device__ __forceinline__ bool keep_positive(float x) { return __float_as_uint(x) - 1u < 0x7f800000u; }  // x > 0
 __device__ __forceinline__ float one_minus_exp_neg_keep(float x) {
   const float s = keep_mul(x, 1.0f + x * (-0.5f + x * (1.0f / 6.0f + x * (-1.0f / 24.0f + x * (1.0f / 120.0f)))));
@@ -1190,7 +1196,7 @@ struct Walk3D32 {
     // the common crossing: interior, scattering medium, weight above the roulette threshold,
     // no index jump
     if (going && prop > 0.0f && (unsigned)nextel < (unsigned)ne(J) && mus > 0.0f && w >= (float)kWeight0 && nidx == o2.w) {
-      if (o2.y != mus) prop *= mus / o2.y;
+      if (o2.y != mus) prop = keep_mul(prop, keep_div(mus, o2.y));
       flush(J);
       el = nextel;
       mua = o2.x; mus = o2.y; g = o2.z;
@@ -1274,7 +1280,7 @@ struct Walk3D32 {
       if (nidx != o2.w) {
         if (fresnel(rng, nx, ny, nz, nidx / o2.w)) return true;
       }
-      if (o2.y != mus) prop *= mus / o2.y;
+      if (o2.y != mus) prop = keep_mul(prop, keep_div(mus, o2.y));
     }
     flush(J);
     el = nextel;
