@@ -432,3 +432,24 @@ def test_path_left_on_entering_a_scattering_element(built, mus):
         a, b = (x.ER[(z >= k) & (z < k + 1)].sum() for x in (tiny, none))
         assert abs(a - b) < 6 * np.sqrt(2 * n / 4)  # a photon leaves between 0 and 1 there
     assert abs(tiny.stats["scatters"] / none.stats["scatters"] - 1) < 0.02
+
+
+def test_a_path_that_is_no_number(built):
+    """Elements without a scattering coefficient (NaN): what becomes of the photons there is the same
+    in a launch of one job and in one of several, and none leaves through a boundary element that
+    it has not come to."""
+    r, H, BH = mg.box_mesh_3d(4, 4, 6)
+    ne, nb = len(H), len(BH)
+    z = r[H].mean(axis=1)[:, 2]
+    zb = r[BH].mean(axis=1)[:, 2]
+    types = np.full(nb, ord("a"), np.uint8)
+    types[zb == 6] = ord("l")
+    p = mg.Problem(dim=3, H=H, BH=BH, r=r, mua=np.full(ne, 0.2), mus=np.where((z > 2) & (z < 4), np.nan, 2.0), g=np.zeros(ne),
+                   n=np.full(ne, 1.0), BCType=types, BCn=np.full(nb, 1.0), Nphoton=5000, seed=5)
+    one = V.run(p, normalize=False, max_steps=300)
+    mesh = V.Mesh(p)
+    two, _ = V.run_batch([mesh, mesh], [p, p.copy(Nphoton=0)], normalize=False, max_steps=300)
+    mesh.close()
+    assert zb[0] < 1 and one.EBR[0] == 0
+    np.testing.assert_allclose(one.EBR, two[0].EBR, rtol=1e-9, atol=1e-9)
+    np.testing.assert_allclose(np.nan_to_num(one.ER), np.nan_to_num(two[0].ER), rtol=1e-9, atol=1e-9)

@@ -1153,7 +1153,7 @@ struct Walk3D32 {
     int nextel = -1;
     float4 o2 = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (R::kOneJob) {
-      if (prop > dist) nextel = __ldg(T->nbr + (nf & 3));
+      if (!(prop <= dist)) nextel = __ldg(T->nbr + (nf & 3));  // also of a path that is no number
     } else {
       nextel = nf == 0 ? nb.x : nf == 1 ? nb.y : nf == 2 ? nb.z : nb.w;
     }
