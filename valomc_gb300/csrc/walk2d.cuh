@@ -358,7 +358,7 @@ struct Walk2D64 {
       }
       n2 = __ldg(J.bcn + ib);
     }
-    const bool vacuum = inside && !positive(mus) && positive(mus2);
+    const bool vacuum = inside && at_most_zero(mus) && positive(mus2);
     const bool jump = inside ? differ(nidx, n2) : positive(n2);
     const bool light = inside && below(w, kWeight0);
     if (!inside || vacuum || jump || light) {

@@ -286,9 +286,13 @@ __device__ __forceinline__ float f32_of(double x) {
 __device__ __forceinline__ bool positive(double x) {  // x > 0
   return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
 }
-__device__ __forceinline__ bool differ(double a, double b) {  // a != b (a, b no NaN)
+__device__ __forceinline__ bool at_most_zero(double x) {  // x <= 0
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return b - 1ull >= 0x7fffffffffffffffull && (b << 1) <= 0xffe0000000000000ull;
+}
+__device__ __forceinline__ bool differ(double a, double b) {  // a != b
   const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
-  return x != y && ((x | y) << 1) != 0ull;
+  return x != y ? ((x | y) << 1) != 0ull : (x << 1) > 0xffe0000000000000ull;
 }
 __device__ __forceinline__ bool below(double x, double limit) {  // x < limit, for x >= 0 and limit > 0
   return __double_as_longlong(x) < __double_as_longlong(limit);
