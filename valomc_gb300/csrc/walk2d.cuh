@@ -80,6 +80,7 @@ struct Walk2D64 {
       sincos_turn(turn, sph, cph);
     }
     optics(J, el, mua, mus, g, nidx);
+    nidx = index_at_launch(nidx);
     imus = fast_rcp(mus);
     kg = turn_ratio(g);
     prop = neg_log_open(rng.next()) * imus;

@@ -267,6 +267,7 @@ struct Walk3D64 {
       sincos_turn(turn, sph, cph);
     }
     optics(J, el, mua, mus, g, nidx);
+    nidx = index_at_launch(nidx);
     imus = fast_rcp(mus);
     ig = hg_inverse(g);
     prop = neg_log_open(rng.next()) * imus;  // the outer loop's first draw, MC3D.hpp:1458

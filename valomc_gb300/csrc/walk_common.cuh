@@ -290,9 +290,17 @@ __device__ __forceinline__ bool at_most_zero(double x) {  // x <= 0
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   return b - 1ull >= 0x7fffffffffffffffull && (b << 1) <= 0xffe0000000000000ull;
 }
-__device__ __forceinline__ bool differ(double a, double b) {  // a != b
+__device__ __forceinline__ bool differ(double a, double b) {  // a != b, but a NaN and its copy do not differ
   const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
-  return x != y ? ((x | y) << 1) != 0ull : (x << 1) > 0xffe0000000000000ull;
+  return x != y && ((x | y) << 1) != 0ull;
+}
+// The index of the element that a photon starts in: an undefined one in bits that differ from any
+// other's, so that its first crossing is an interface, as a comparison of doubles has it.  (Entered
+// elements need none: the interface before them loses the photon.)  In the comparison itself the
+// test took 2 to 3 % of a step.
+__device__ __forceinline__ double index_at_launch(double n) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(n);
+  return (b << 1) > 0xffe0000000000000ull ? __longlong_as_double((long long)(b ^ 0x0000a5c3d2e1f0b7ull)) : n;
 }
 __device__ __forceinline__ bool below(double x, double limit) {  // x < limit, for x >= 0 and limit > 0
   return __double_as_longlong(x) < __double_as_longlong(limit);
