@@ -75,7 +75,10 @@ def test_fp64_mesh_without_room_for_plane_records(built, layers, left):
     mesh.close()
     V.Server(memory_budget=1 << 30).close()  # gives back what the calls' pool keeps
     free = torch.cuda.mem_get_info()[0]
-    held = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+    try:
+        held = torch.empty(free - left, dtype=torch.uint8, device="cuda")
+    except RuntimeError:
+        pytest.skip("the device's free memory cannot be held in one piece")
     try:
         mesh = V.Mesh(p, precision=V.VMC_FP64)
         assert 112 * ne <= mesh.device_bytes < 200 * ne
